@@ -39,15 +39,16 @@ enum {
     NTTB_ERR_BUDGET = 6       /* serving admission refused: HBM budget exceeded */
 };
 
-/* Inner-DFT engines.  AUTO picks the fastest one that serves the request:
- * the INT8 tensor-core kernel at N = 2^16 from 8 (polynomial, limb) units
- * on; the batch queue's tensor tiles at N = 2^17 .. 2^20 once a call holds
- * 2^20 residues; the CUDA-core engine otherwise.  The tiles engine keeps up
+/* Inner-DFT engines.  AUTO picks one that serves the request: out of place the
+ * CUDA-core engine; in place the INT8 tensor-core kernel at N = 2^16 from 8
+ * (polynomial, limb) units on, the batch queue's tensor tiles at N = 2^17 ..
+ * 2^20 once a call holds 2^20 residues, the CUDA-core engine otherwise (it
+ * stages its first pass in the plan's workspace).  The tiles engine keeps up
  * to eight prepared queues per plan (one per source, destination, count,
  * direction), each with its own workspace ring of up to 16 x N words. */
 enum {
     NTTB_ENGINE_AUTO = 0,
-    NTTB_ENGINE_SCALAR = 1, /* CUDA-core radix-2 in shared memory */
+    NTTB_ENGINE_SCALAR = 1, /* CUDA-core radix-2 stages in registers and shared memory */
     NTTB_ENGINE_DMMA = 2,   /* FP64 mma.sync m8n8k4 radix-8 contractions (the plain drop-in form) */
     NTTB_ENGINE_INT8 = 3,   /* tcgen05 kind::i8, byte-plane radix-64 contractions, INT32 in TMEM */
     NTTB_ENGINE_TILES = 4   /* the batch queue's tcgen05 tensor tiles (two-pass four-step, 2^13 .. 2^20) */
@@ -207,8 +208,7 @@ NTTB_API int nttb_rns_stream_host(nttb_rns_plan* plan, const uint32_t* h_src, ui
  * the allocator because cudaMalloc can synchronize the device, a fixed
  * up-front memory budget).  The first pass is staged in a static device
  * buffer of NTTB_NOALLOC_SCRATCH_BYTES that every GPU loading the library
- * holds until exit.  Shapes that run in two passes (n > 8192, or n >= 4096
- * with fewer than 8 (polynomial, limb) units) stage n_polys * n_limbs * n * 4
+ * holds until exit.  Shapes that run in two passes (n > 8192) stage n_polys * n_limbs * n * 4
  * bytes there, and batches needing more are rejected with
  * NTTB_ERR_INVALID_ARG; one-pass shapes stage nothing and are not limited.
  * The plan's device must be the current device (else NTTB_ERR_INVALID_ARG).
@@ -237,11 +237,9 @@ NTTB_API int nttb_wide_transform(const nttb_wide_plan* plan, uint64_t* d_dst, co
 /* The same with the engine named: NTTB_ENGINE_INT8 runs the tcgen05 kind::i8
  * byte-plane engine (eight byte planes of each uint64 word, DFT-32 x DFT-32
  * per pass of the four-step 1024 x 1024; served for n = 2^20, cyclic plans;
- * NTTB_ERR_UNSUPPORTED otherwise), NTTB_ENGINE_SCALAR the CUDA-core
- * Montgomery-64 engine, NTTB_ENGINE_AUTO (what nttb_wide_transform uses) the
- * INT8 engine where it serves the plan and the batch has fewer than 8
- * (polynomial, limb) units (it has the shorter latency; the CUDA-core engine
- * the higher throughput on larger batches).  Pointers 16-byte aligned; src may
+ * NTTB_ERR_UNSUPPORTED otherwise), NTTB_ENGINE_SCALAR the CUDA-core engine,
+ * NTTB_ENGINE_AUTO (what nttb_wide_transform uses) the CUDA-core engine too: it
+ * has the shorter latency and the higher throughput at every size.  Pointers 16-byte aligned; src may
  * equal dst.  Replaces the reference's run_forward_ct_tcu<K> for primes near
  * 2^60 (include/ntt_arbitrary.cuh:2599-2646, its limb products on FP64 MMA). */
 NTTB_API int nttb_wide_transform_engine(const nttb_wide_plan* plan, uint64_t* d_dst, const uint64_t* d_src,

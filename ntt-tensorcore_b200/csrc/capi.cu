@@ -299,20 +299,16 @@ int nttb_phase_profile(uint64_t* out16, int* enabled, int clear) {
     return cuda_status("phase_profile");
 }
 
-// A wide (64-bit modulus) transform: AUTO takes the INT8 engine where it
-// serves the plan (n = 2^20, cyclic) for fewer than 8 (polynomial, limb)
-// units, the CUDA-core Montgomery-64 engine otherwise.  Both spend about the
-// same number of integer multiplies per residue (the 64-bit REDCs and twiddle
-// products of the byte-plane epilogues match the radix-2 butterflies'); the
-// INT8 engine's two passes have the shorter latency (one 2^20 polynomial:
-// 82 against 95 us forward + inverse), the CUDA-core engine the higher
-// throughput from 16 units on (1.01 against 1.07 ms for 16).
+// A wide (64-bit modulus) transform: AUTO takes the CUDA-core engine, whose
+// register-radix passes (radix.cuh) beat the INT8 byte-plane engine from one
+// 2^20 polynomial on (23 against 39 us forward, three of them 66 against 103).
+// The drop-in's uint64 words (`dropin`) keep the byte-plane engine below
+// kWideTcMaxUnits polynomials: it is the engine that entry point names for them.
 constexpr uint64_t kWideTcMaxUnits = 8;
 static int wide_transform(Plan64& p, const void* src, void* dst, uint32_t n_polys, bool inverse, int engine,
-                          cudaStream_t s) {
-    if (engine == NTTB_ENGINE_AUTO)
-        engine = wide_tc_serves(p) && (uint64_t)n_polys * p.n_limbs < kWideTcMaxUnits ? NTTB_ENGINE_INT8
-                                                                                       : NTTB_ENGINE_SCALAR;
+                          bool dropin, cudaStream_t s) {
+    if (engine == NTTB_ENGINE_AUTO && dropin && wide_tc_serves(p) && n_polys < kWideTcMaxUnits)
+        engine = NTTB_ENGINE_INT8;
     if (engine == NTTB_ENGINE_INT8) return wide_tc_transform64(p, src, dst, n_polys, inverse, s);
     if (engine == NTTB_ENGINE_TILES) return 1;  // the batch queue's tiles take moduli < 2^31
     return scalar_transform64(p, src, dst, n_polys, inverse, s);  // the 31-bit engines do not serve 64-bit moduli
@@ -493,7 +489,7 @@ int nttb_u64_transform(const nttb_plan* P, uint64_t* d, uint64_t batch, int inve
     cudaStream_t s = (cudaStream_t)stream;
     int rc;
     if (P->wide) {
-        rc = wide_transform(const_cast<Plan64&>(P->p64), d, d, (uint32_t)batch, inverse != 0, engine, s);
+        rc = wide_transform(const_cast<Plan64&>(P->p64), d, d, (uint32_t)batch, inverse != 0, engine, true, s);
     } else {
         rc = run_transform32(const_cast<Plan32&>(P->p32), d, d, true, (uint32_t)batch, inverse != 0, engine, s);
     }
@@ -635,7 +631,7 @@ int nttb_rns_forward_inverse(const nttb_rns_plan* P, uint32_t* d, uint32_t n_pol
     if (((uintptr_t)d) & 15) return fail(NTTB_ERR_INVALID_ARG, "rns_forward_inverse: pointer must be 16-byte aligned");
     Plan32& p = const_cast<Plan32&>(P->p);
     cudaStream_t s = (cudaStream_t)stream;
-    int eng = engine == NTTB_ENGINE_AUTO ? auto_engine32(p, false, (uint64_t)n_polys * p.n_limbs) : engine;
+    int eng = engine == NTTB_ENGINE_AUTO ? auto_engine32(p, false, (uint64_t)n_polys * p.n_limbs, true) : engine;
     int rc;
     if (eng == NTTB_ENGINE_INT8) {
         rc = int8_forward_inverse32(p, d, n_polys, s);
@@ -654,7 +650,7 @@ int nttb_rns_stream_host(nttb_rns_plan* P, const uint32_t* h_src, uint32_t* h_ds
     Plan32& p = P->p;
     cudaStream_t s = (cudaStream_t)stream;
     const size_t bw = (size_t)n_polys * p.n_limbs * p.n;
-    const int eng = engine == NTTB_ENGINE_AUTO ? auto_engine32(p, false, (uint64_t)n_polys * p.n_limbs) : engine;
+    const int eng = engine == NTTB_ENGINE_AUTO ? auto_engine32(p, false, (uint64_t)n_polys * p.n_limbs, true) : engine;
     nttb::HostStream*& H = P->hs;
     if (!H || H->words < bw) {  // (re)build the buffers, streams and events
         nttb::host_stream_free(H);
@@ -779,7 +775,7 @@ int nttb_wide_transform_engine(const nttb_wide_plan* P, uint64_t* dst, const uin
     if ((((uintptr_t)dst) | ((uintptr_t)src)) & 15) return fail(NTTB_ERR_INVALID_ARG, "wide_transform: pointers must be 16-byte aligned");
     if (n_polys == 0) return NTTB_OK;
     const int rc = wide_transform(const_cast<Plan64&>(P->p), src, dst, n_polys, inverse != 0, engine,
-                                  (cudaStream_t)stream);
+                                  false, (cudaStream_t)stream);
     return engine_status(rc, "wide_transform");
 }
 

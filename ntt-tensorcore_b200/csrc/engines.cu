@@ -17,21 +17,21 @@ static int env_engine() {
     return NTTB_ENGINE_AUTO;
 }
 
-// The INT8 cluster kernel gives each (polynomial, limb) unit four SMs; AUTO
-// takes it from kInt8MinUnits units on, below which the CUDA-core engine,
-// which spreads one polynomial over the whole GPU, is faster (uint64 words at
-// 2^16: 13 - 17 us for 1 - 4 polynomials against 21 us; 25 against 21 us for 8).
+// Out of place, the CUDA-core engine's register-radix passes (radix.cuh) are
+// the fastest at every size (us, forward, this engine / the other): 8 x 2^16
+// 6.9 / 16.6 (INT8), 24 x 2^16 9.7 / 17.4 (INT8), 192 x 2^16 57 / 95 (INT8),
+// 33 x 2^17 22.8 / 62 (tiles), 1 x 2^20 10 / 25 (tiles).  In place they stage
+// their first pass in the plan's workspace, which ties the plan's calls to one
+// stream; the sizes and counts below keep an engine that does not:
+// the INT8 cluster kernel at 2^16 from kInt8MinUnits (polynomial, limb) units
+// on, and the batch queue's tensor tiles at 2^17 .. 2^20 once a call holds
+// 2^20 residues (each prepared queue has a ring of its own).
 constexpr uint64_t kInt8MinUnits = 8;
-// The batch queue's tensor tiles take sizes 2^17 .. 2^20 once a call holds
-// 2^20 residues: single forward transforms of BabyBear words, CUDA events
-// over 200 calls, tiles / CUDA-core engine in us: 1 x 2^20 26.4 / 33.8,
-// 4 x 2^18 23.6 / 32.7, 4 x 2^20 51.2 / 81.9; below that the CUDA-core
-// engine, which spreads a call over the whole GPU with less set-up, is as
-// fast or faster (4 x 2^17 22.5 / 22.6, 1 x 2^19 24.4 / 22.5).
 constexpr uint32_t kTilesMinLog = 17;
 constexpr uint64_t kTilesMinResidues = 1ull << 20;
 
-int auto_engine32(const Plan32& p, bool src_u64, uint64_t units) {
+int auto_engine32(const Plan32& p, bool src_u64, uint64_t units, bool in_place) {
+    if (!in_place && scalar_serves(p, units)) return NTTB_ENGINE_SCALAR;
     if (int8_serves(p, src_u64) && units >= kInt8MinUnits) return NTTB_ENGINE_INT8;
     if (tiles_serve(p) && p.log_n >= kTilesMinLog && (units << p.log_n) >= kTilesMinResidues) return NTTB_ENGINE_TILES;
     return NTTB_ENGINE_SCALAR;
@@ -40,7 +40,7 @@ int auto_engine32(const Plan32& p, bool src_u64, uint64_t units) {
 int run_transform32(Plan32& p, const void* src, void* dst, bool src_u64, uint32_t n_polys, bool inverse,
                     int engine, cudaStream_t s) {
     if (engine == NTTB_ENGINE_AUTO) engine = env_engine();
-    if (engine == NTTB_ENGINE_AUTO) engine = auto_engine32(p, src_u64, (uint64_t)n_polys * p.n_limbs);
+    if (engine == NTTB_ENGINE_AUTO) engine = auto_engine32(p, src_u64, (uint64_t)n_polys * p.n_limbs, src == dst);
     switch (engine) {
         case NTTB_ENGINE_SCALAR:
             return scalar_transform32(p, src, dst, src_u64, n_polys, inverse, s);

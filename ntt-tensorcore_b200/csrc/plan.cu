@@ -80,21 +80,27 @@ static void fill_powers(E* dst, uint64_t base, uint64_t start, uint64_t n, uint6
     }
 }
 
-// Shoup pairs of the roots of each length L = 2^l <= n, level by level:
-// pairs 2^(l-1) - 1 + k = (root_L^k, floor(root_L^k * 2^bits / q)), k < L/2,
-// root_L = root_n^(n/L); n - 1 pairs in all.
-template <class E>
-static void fill_shoup_levels(E* dst, uint64_t root_n, uint32_t log_n, uint64_t q) {
-    for (uint32_t l = 1; l <= log_n; l++) {
-        const uint64_t step = h_powmod(root_n, 1ull << (log_n - l), q);
-        E* lvl = dst + 2 * ((1ull << (l - 1)) - 1);
-        uint64_t x = 1 % q;
-        for (uint64_t k = 0; k < (1ull << (l - 1)); k++) {
-            lvl[2 * k] = (E)x;
-            if constexpr (sizeof(E) == 4) lvl[2 * k + 1] = (E)((x << 32) / q);
-            else lvl[2 * k + 1] = (E)(((unsigned __int128)x << 64) / q);
-            x = h_mulmod(x, step, q);
+// Shoup pairs from Montgomery-form powers, on the device.  `pw` holds
+// base^e R mod q, e < n.  Pair i = 2^s + k: base^((n / 2^(s+1)) (odd ? 1 + 2k :
+// k)), or its inverse, which is base^(n - e) for a base of order n and its
+// negative for one of order 2n (odd).  The plain root is a Montgomery product
+// by 1; its quotient floor(w R / q) = (w R - r) / q, with r = w R mod q the
+// table's own entry, is r * (-q^-1) mod R.
+template <class A>
+__global__ void shoup_pairs_kernel(typename A::elem* out, const typename A::elem* pw, uint32_t log_n, A ar, bool odd,
+                                   bool inverse) {
+    using E = typename A::elem;
+    const uint32_t n = 1u << log_n;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        E r = 0;
+        if (i) {
+            const uint32_t s = 31 - __clz(i), k = i - (1u << s), step = n >> (s + 1);
+            const uint32_t e = odd ? step * (1 + 2 * k) : step * k;
+            r = inverse && e ? pw[n - e] : pw[e];
+            if (inverse && odd) r = ar.q - r;
         }
+        out[2 * (size_t)i] = ar.mul(r, (E)1);
+        out[2 * (size_t)i + 1] = r * ar.qinv;
     }
 }
 
@@ -116,46 +122,69 @@ static int build_common(PlanT* p, uint32_t log_n, const uint64_t* moduli, uint32
         if (moduli[l] >= qmax) { *why = "modulus " + std::to_string(moduli[l]) + " too large for this path"; return 1; }
         if (!make_limb_host(moduli[l], n, negacyclic, &p->limbs[l], why)) return 1;
     }
-    // omega^e, omega^-e (, psi^e, n^-1 psi^-e) in Montgomery form, then the
-    // level-by-level Shoup pairs of the forward and inverse roots (2n words each)
-    const uint32_t tables = negacyclic ? 4 : 2;
-    const size_t per_limb = (size_t)(tables + 4) * n;
-    std::vector<E> host(per_limb * n_limbs);
+    // Powers in Montgomery form, uploaded: omega^e, omega^-e (, psi^e, n^-1
+    // psi^-e); a negacyclic plan of a size that the register-radix passes serve
+    // needs psi^e alone.  Behind them, made on the device, 2n words of Shoup
+    // pairs per direction: of psi for such a plan, else of omega (one table for
+    // the radix-2 and the register-radix passes).
+    const bool radix = radix_serves(log_n), lean = negacyclic && radix;
+    const uint32_t tables = lean ? 1 : negacyclic ? 4 : 2;
+    const size_t per_limb = (size_t)(tables + 4) * n, up = (size_t)tables * n;
+    std::vector<E> host(up), scale(4 * (size_t)n_limbs);
     std::vector<LimbDev<A>> devs(n_limbs);
-    E* d_tables = nullptr;
-    if (cudaMalloc(&d_tables, host.size() * sizeof(E)) != cudaSuccess) { *why = "cudaMalloc failed"; return 4; }
+    E *d_tables = nullptr, *d_scale = nullptr;
+    if (cudaMalloc(&d_tables, per_limb * n_limbs * sizeof(E)) != cudaSuccess) { *why = "cudaMalloc failed"; return 4; }
     p->allocations.push_back(d_tables);
+    if (cudaMalloc(&d_scale, scale.size() * sizeof(E)) != cudaSuccess) { *why = "cudaMalloc failed"; return 4; }
+    p->allocations.push_back(d_scale);
+    const unsigned grid = (unsigned)((n + 255) / 256 < 592 ? (n + 255) / 256 : 592);
     for (uint32_t l = 0; l < n_limbs; l++) {
         const LimbHost& L = p->limbs[l];
         const uint64_t q = L.q;
-        E* h = host.data() + per_limb * l;
-        E* d = d_tables + per_limb * l;
-        fill_powers(h, L.omega, 1, n, q, [&](uint64_t x) { return tm(x, q); });
-        fill_powers(h + n, L.omega_inv, 1, n, q, [&](uint64_t x) { return tm(x, q); });
+        E *h = host.data(), *d = d_tables + per_limb * l;
+        auto mont = [&](uint64_t x) { return tm(x, q); };
         LimbDev<A> dv{};
-        dv.tw = d;
-        dv.tw_inv = d + n;
-        if (negacyclic) {
-            fill_powers(h + 2 * n, L.psi, 1, n, q, [&](uint64_t x) { return tm(x, q); });
-            fill_powers(h + 3 * n, L.psi_inv, L.n_inv, n, q, [&](uint64_t x) { return tm(x, q); });
-            dv.psi = d + 2 * n;
-            dv.psi_inv = d + 3 * n;
-        }
-        fill_shoup_levels(h + (size_t)tables * n, L.omega, log_n, q);
-        fill_shoup_levels(h + (size_t)(tables + 2) * n, L.omega_inv, log_n, q);
-        dv.tw_sh = d + (size_t)tables * n;
-        dv.tw_inv_sh = d + (size_t)(tables + 2) * n;
+        dv.ar.q = (E)q;
+        if constexpr (sizeof(E) == 4) dv.ar.qinv = h_neg_inv32((uint32_t)q);
+        else dv.ar.qinv = h_neg_inv64(q);
         dv.ninv_m = (E)tm(L.n_inv, q);
+        E* pairs = d + up;
+        if (lean) {
+            fill_powers(h, L.psi, 1, n, q, mont);
+            dv.psi = d;
+        } else {
+            fill_powers(h, L.omega, 1, n, q, mont);
+            fill_powers(h + n, L.omega_inv, 1, n, q, mont);
+            dv.tw = d;
+            dv.tw_inv = d + n;
+            if (negacyclic) {
+                fill_powers(h + 2 * n, L.psi, 1, n, q, mont);
+                fill_powers(h + 3 * n, L.psi_inv, L.n_inv, n, q, mont);
+                dv.psi = d + 2 * n;
+                dv.psi_inv = d + 3 * n;
+            }
+        }
+        if (cudaMemcpy(d, h, up * sizeof(E), cudaMemcpyHostToDevice) != cudaSuccess) { *why = "cudaMemcpy failed"; return 3; }
+        // pair 0 is unused: the radix-2 levels start at pair 1 (radix-2 root of length 2)
+        for (int inv = 0; inv < 2; inv++) {
+            E* t = pairs + (size_t)inv * 2 * n;
+            shoup_pairs_kernel<A><<<grid, 256>>>(t, lean ? dv.psi : dv.tw, log_n, dv.ar, lean, inv != 0);
+            (inv ? dv.rt_inv : dv.rt) = t;
+            if (!lean) (inv ? dv.tw_inv_sh : dv.tw_sh) = t + 2;
+        }
+        // n^-1 and n^-1 W, W = the inverse's one root of stage 0 (psi^-(n/2) or 1)
+        const uint64_t w0 = lean ? h_mulmod(L.n_inv, h_powmod(L.psi_inv, n / 2, q), q) : L.n_inv;
+        const uint64_t sc[2] = {L.n_inv, w0};
+        for (int i = 0; i < 2; i++) {
+            scale[4 * l + 2 * i] = (E)sc[i];
+            scale[4 * l + 2 * i + 1] = (E)((((unsigned __int128)sc[i]) << (8 * sizeof(E))) / q);
+        }
+        dv.scale = d_scale + 4 * l;
         devs[l] = dv;
     }
-    for (uint32_t l = 0; l < n_limbs; l++) {
-        const uint64_t q = p->limbs[l].q;
-        devs[l].ar.q = (E)q;
-        if constexpr (sizeof(E) == 4) devs[l].ar.qinv = h_neg_inv32((uint32_t)q);
-        else devs[l].ar.qinv = h_neg_inv64(q);
-    }
-    if (cudaMemcpy(d_tables, host.data(), host.size() * sizeof(E), cudaMemcpyHostToDevice) != cudaSuccess) {
-        *why = "cudaMemcpy failed";
+    if (cudaMemcpy(d_scale, scale.data(), scale.size() * sizeof(E), cudaMemcpyHostToDevice) != cudaSuccess ||
+        cudaStreamSynchronize(0) != cudaSuccess) {
+        *why = "table set-up failed";
         return 3;
     }
     LimbDev<A>* d_limbs = nullptr;

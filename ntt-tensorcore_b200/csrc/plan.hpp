@@ -27,6 +27,13 @@ struct LimbDev {
     // so a pass of length L reads one contiguous run
     const typename A::elem* tw_sh;
     const typename A::elem* tw_inv_sh;
+    // Shoup pairs of the register-radix passes (radix.cuh), stage by stage: pair
+    // 2^s + i = root^((n / 2^(s+1)) (1 + 2 i)) (root = psi, negacyclic) or
+    // root^((n / 2^(s+1)) i) (root = omega, cyclic), i < 2^s; the inverse's
+    // roots in rt_inv; scale = the pairs of n^-1 and of n^-1 rt_inv[1]
+    const typename A::elem* rt;
+    const typename A::elem* rt_inv;
+    const typename A::elem* scale;
 };
 
 // Host view of one modulus at one transform size.
@@ -124,6 +131,8 @@ void free_plan64(Plan64* p);
 // words; data layout is [poly][limb][n].
 int scalar_transform32(Plan32& p, const void* src, void* dst, bool src_u64, uint32_t n_polys, bool inverse,
                        cudaStream_t s);
+// Whether a call of `units` (polynomial, limb) rows is within its grid limits.
+inline bool scalar_serves(const Plan32& p, uint64_t units) { return p.n_limbs <= 65535 && units / p.n_limbs <= 65535; }
 int scalar_transform64(Plan64& p, const void* src, void* dst, uint32_t n_polys, bool inverse, cudaStream_t s);
 // In-place uint32 transform staging its first pass in a caller-supplied buffer
 // `ws` (n_polys * n_limbs * n words); allocates nothing.
@@ -132,6 +141,16 @@ int scalar_transform32_ws(const Plan32& p, uint32_t* data, void* ws, uint32_t n_
 // Bytes of `ws` that scalar_transform32_ws stages in for n_polys polynomials
 // (0 when the shape runs as one pass and stages nothing).
 size_t scalar_transform32_ws_bytes(const Plan32& p, uint32_t n_polys);
+
+// Register-radix passes on CUDA cores (radix.cuh): sizes 2^5 .. 2^20.  Sizes
+// above 2^13 run two passes through `mid`, n_polys * n_limbs * n words (uint32
+// for the 31-bit plans, uint64 for the wide ones): the destination, if the
+// source is another buffer and the words have its size, or a workspace.
+constexpr uint32_t kRadixMinLog = 5, kRadixMaxLog = 20, kRadixSingleMax = 13;
+inline bool radix_serves(uint32_t log_n) { return log_n >= kRadixMinLog && log_n <= kRadixMaxLog; }
+int radix_u32(const Plan32& p, const void* src, void* dst, void* mid, uint32_t n_polys, bool inverse, cudaStream_t s);
+int radix_w64(const Plan32& p, const void* src, void* dst, void* mid, uint32_t n_polys, bool inverse, cudaStream_t s);
+int radix_q64(const Plan64& p, const void* src, void* dst, void* mid, uint32_t n_polys, bool inverse, cudaStream_t s);
 
 // INT8 tensor-core engine for the wide plans (tc_wide.cu): n = 2^20, cyclic,
 // moduli below 2^62 on byte planes of uint64 words.  Returns 1 when the plan

@@ -1,0 +1,373 @@
+// radix.cuh -- the register-radix NTT pass on CUDA cores: one kernel template
+// for the single-pass transforms and for both passes of the two-pass ones.
+//
+// Network.  The forward transform runs the Cooley-Tukey butterflies of the
+// ring splitting X^n -+ 1 (natural order in, bit-reversed positions): at
+// stage s (m = 2^s blocks) block i multiplies by root^((n / 2m) (1 + 2 rev(i)))
+// (negacyclic, root = psi) or root^((n / 2m) rev(i)) (cyclic, root = omega),
+// so the twist and the four-step twiddles cost no products of their own.  The
+// inverse is the same network backwards (Gentleman-Sande), n^-1 folded into
+// its last stage.  Roots are Shoup pairs, tab[2^s + rev(i)]: natural order
+// within a stage, so that neighbouring threads read neighbouring pairs.
+//
+// Two passes, n = N1 * N2, input index r N2 + c, output index k2 N1 + u:
+//   forward  A: columns c of [N1][N2], stages 0 .. a-1 (the same roots for
+//               every column), stored transposed: mid[c N1 + u];
+//            B: columns u of [N2][N1], the remaining stages (roots of row u),
+//               stored at the positions they were read from;
+//   inverse  A: columns u of [N2][N1] (roots of row u), stored mid[u N2 + c];
+//            B: columns c of [N1][N2] (the same roots for every column), in place.
+// Pass B reads and writes one set of positions per tile, so `mid` may be the
+// destination; pass A must not write over its source.
+//
+// Tile: V neighbouring columns of N = 2^LG elements, 2^LGE of them in the
+// registers of a thread.  The stages run in register rounds of up to LGE
+// stages; between rounds the tile is exchanged through shared memory, where
+// element bit i has its own stride (Lay) chosen so that every round's loads
+// and stores -- V columns x neighbouring positions, or 32 positions of one
+// column -- fall into distinct banks without any address arithmetic per
+// element.  A thread overwrites what it has read, so a round needs one barrier.
+#pragma once
+#include <cuda_runtime.h>
+
+#include <cstdint>
+
+#include "arith.cuh"
+#include "plan.hpp"
+
+namespace nttb {
+namespace rdx {
+
+struct Args {
+    const void* src;
+    void* dst;
+    uint64_t poly_stride;  // words between consecutive polynomials
+    uint32_t log_n;
+    uint32_t polys;        // polynomials in all
+    uint32_t polys_per_cta;
+    uint32_t units;        // single pass: (polynomial, limb) rows
+    uint32_t n_limbs;
+};
+
+__host__ __device__ constexpr uint32_t brv(uint32_t x, int bits) {
+    uint32_t r = 0;
+    for (int i = 0; i < bits; i++) r |= ((x >> i) & 1u) << (bits - 1 - i);
+    return r;
+}
+__device__ __forceinline__ uint32_t brv_dev(uint32_t x, int bits) { return bits ? __brev(x) >> (32 - bits) : 0u; }
+
+// Strides (in elements) of the LG position bits in shared memory; column v
+// sits at offset v.  NB = log2 of the banks counted in elements (5 for 4-byte,
+// 4 for 8-byte elements).  The bits next to either end get distinct
+// power-of-two residues mod 2^NB, in the order in which lanes enumerate them:
+// first those above the V columns', then the columns' own.
+template <int LG, int LGV, int NB>
+struct Lay {
+    uint32_t s[LG > 0 ? LG : 1] = {};
+    uint32_t words = 0;
+    constexpr Lay() {
+        uint32_t sum = (1u << LGV) - 1u;
+        const uint32_t mod = 1u << NB;
+        for (int i = 0; i < LG; i++) {
+            const int pos = i < LG / 2 ? i : LG - 1 - i;
+            uint32_t st = sum + 1u;
+            if (pos < NB) {
+                const int bit = pos < NB - LGV ? LGV + pos : NB - 1 - pos;
+                while ((st & (mod - 1u)) != (1u << bit)) st++;
+            }
+            s[i] = st;
+            sum += st;
+        }
+        words = sum + 1u;
+    }
+};
+
+// Stages per round: the last takes LGE, the ones before it share the rest.
+template <int LG, int LGE>
+struct Rounds {
+    int n = 0;
+    int r[8] = {}, s0[8] = {};
+    constexpr Rounds() {
+        const int rest = LG - LGE, k = (rest + LGE - 1) / LGE;
+        int done = 0;
+        for (int i = 0; i < k; i++) {
+            r[i] = (rest - done) / (k - i);
+            s0[i] = done;
+            done += r[i];
+        }
+        r[k] = LGE;
+        s0[k] = rest;
+        n = k + 1;
+    }
+};
+
+template <class A>
+struct PairOf;
+template <>
+struct PairOf<M32> { using type = uint2; };
+template <>
+struct PairOf<M64> { using type = ulonglong2; };
+
+// min(x, x - q) on unsigned words: x - q when x >= q (x < 2q), one instruction.
+__device__ __forceinline__ uint32_t sub_if(uint32_t x, uint32_t q) { return __viaddmin_u32(x, 0u - q, x); }
+
+// Forward butterfly: M32 keeps values in [0, 2q) (q < 2^31), M64 in [0, 4q) (q < 2^62).
+__device__ __forceinline__ void ct(const M32& ar, uint32_t& a, uint32_t& b, uint2 w) {
+    const uint32_t u = sub_if(a, ar.q);
+    const uint32_t t = sub_if(b * w.x - __umulhi(b, w.y) * ar.q, ar.q);
+    a = u + t;
+    b = u - t + ar.q;
+}
+__device__ __forceinline__ void ct(const M64& ar, uint64_t& a, uint64_t& b, ulonglong2 w) {
+    const uint64_t u = ar.below2q(a);
+    const uint64_t t = ar.mul_shoup_lazy(b, w.x, w.y);
+    a = u + t;
+    b = u - t + 2 * ar.q;
+}
+// Inverse butterfly: M32 keeps values in [0, q), M64 in [0, 2q).
+__device__ __forceinline__ void gs(const M32& ar, uint32_t& a, uint32_t& b, uint2 w) {
+    const uint32_t s = sub_if(a + b, ar.q), d = a - b + ar.q;
+    a = s;
+    b = sub_if(d * w.x - __umulhi(d, w.y) * ar.q, ar.q);
+}
+__device__ __forceinline__ void gs(const M64& ar, uint64_t& a, uint64_t& b, ulonglong2 w) {
+    const uint64_t s = ar.below2q(a + b), d = a - b + 2 * ar.q;
+    a = s;
+    b = ar.mul_shoup_lazy(d, w.x, w.y);
+}
+// The inverse's last stage: both outputs times n^-1 (c = n^-1, w carries it too).
+__device__ __forceinline__ void gs_scaled(const M32& ar, uint32_t& a, uint32_t& b, uint2 c, uint2 w) {
+    const uint32_t s = a + b, d = a - b + ar.q;
+    a = sub_if(s * c.x - __umulhi(s, c.y) * ar.q, ar.q);
+    b = sub_if(d * w.x - __umulhi(d, w.y) * ar.q, ar.q);
+}
+__device__ __forceinline__ void gs_scaled(const M64& ar, uint64_t& a, uint64_t& b, ulonglong2 c, ulonglong2 w) {
+    const uint64_t s = a + b, d = a - b + 2 * ar.q;
+    a = ar.mul_shoup_lazy(s, c.x, c.y);
+    b = ar.mul_shoup_lazy(d, w.x, w.y);
+}
+template <bool INV>
+__device__ __forceinline__ uint32_t canon_out(const M32& ar, uint32_t x) { return INV ? x : sub_if(x, ar.q); }
+template <bool INV>
+__device__ __forceinline__ uint64_t canon_out(const M64& ar, uint64_t x) {
+    return INV ? (x >= ar.q ? x - ar.q : x) : ar.canon4(x);
+}
+
+// Shoup pair from the constant tables; volatile, so that it is issued where it
+// stands: a round's pairs are fetched before the barrier (or the wait for the
+// previous grid) that its data waits for, when the data registers are free.
+__device__ __forceinline__ uint2 ld_pair(const uint2* p) {
+    uint2 v;
+    asm volatile("ld.global.nc.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ ulonglong2 ld_pair(const ulonglong2* p) {
+    ulonglong2 v;
+    asm volatile("ld.global.nc.v2.u64 {%0, %1}, [%2];" : "=l"(v.x), "=l"(v.y) : "l"(p));
+    return v;
+}
+
+// Roots of round I: w[2^j - 1 + kt] for the round's stage j and block bits kt.
+// `tw` points at tab + U (U the natural index of the thread's block at the
+// round's first stage S): stage S + j, bits kt sit at 2^(S+j) + rev_j(kt) 2^S.
+template <int LG, int LGE, int I, int S0, bool INV, class P>
+__device__ __forceinline__ void round_roots(P (&w)[(1 << LGE) - 1], const P* tw) {
+    constexpr Rounds<LG, LGE> R;
+    constexpr int r = R.r[I], S = S0 + R.s0[I];
+#pragma unroll
+    for (int jj = 0; jj < r; jj++) {
+        const int j = INV ? r - 1 - jj : jj;
+        if (INV && S + j == 0) continue;  // the inverse's last stage multiplies by its scale
+#pragma unroll
+        for (uint32_t kt = 0; kt < (1u << j); kt++)
+            w[(1u << j) - 1u + kt] = ld_pair(tw + ((size_t)1 << (S + j)) + ((size_t)brv(kt, j) << S));
+    }
+}
+
+// Stages of round I on the registers.
+template <class A, int LG, int LGE, int I, int S0, bool INV, class E, class P>
+__device__ __forceinline__ void round_stages(const A& ar, E (&x)[1 << LGE], const P (&w)[(1 << LGE) - 1], P c0, P c1) {
+    constexpr Rounds<LG, LGE> R;
+    constexpr int r = R.r[I], S = S0 + R.s0[I], xb = LGE - r;  // xb: extra held bits below the radix bits
+#pragma unroll
+    for (int jj = 0; jj < r; jj++) {
+        const int j = INV ? r - 1 - jj : jj;
+        const uint32_t half = 1u << (r - 1 - j);
+#pragma unroll
+        for (uint32_t kt = 0; kt < (1u << j); kt++)
+#pragma unroll
+            for (uint32_t lo = 0; lo < half; lo++)
+#pragma unroll
+                for (uint32_t g = 0; g < (1u << xb); g++) {
+                    const uint32_t ia = (((kt << (r - j)) + lo) << xb) + g, ib = ia + (half << xb);
+                    if (INV && S + j == 0) gs_scaled(ar, x[ia], x[ib], c0, c1);
+                    else if (INV) gs(ar, x[ia], x[ib], w[(1u << j) - 1u + kt]);
+                    else ct(ar, x[ia], x[ib], w[(1u << j) - 1u + kt]);
+                }
+    }
+}
+
+// One round's place of a thread: its base offset in shared memory, and the
+// natural index of its block within the pass.
+template <class E, int LG, int LGV, int LGE, int I>
+struct Place {
+    static constexpr int NB = sizeof(E) == 8 ? 4 : 5;
+    static constexpr Rounds<LG, LGE> R{};
+    static constexpr int s0 = R.s0[I], T = LG - s0, o = T - LGE;
+    static constexpr bool last = I == R.n - 1;
+    __device__ __forceinline__ static uint32_t base(uint32_t t) {
+        constexpr Lay<LG, LGV, NB> L;
+        uint32_t a = 0;
+#pragma unroll
+        for (int b = 0; b < LG - LGE; b++) {
+            // bits of t: low o bits are position bits 0 .. o-1, the others the
+            // block (bit-reversed in the last round, whose t is the natural index)
+            const int p = b < o ? b : last ? LG - 1 - (b - o) : T + (b - o);
+            a += ((t >> b) & 1u) * L.s[p];
+        }
+        return a;
+    }
+    __device__ __forceinline__ static uint32_t natural(uint32_t t) {
+        const uint32_t h = t >> o;
+        return last ? h : brv_dev(h, s0);
+    }
+    static constexpr uint32_t reg(uint32_t e) {
+        Lay<LG, LGV, NB> L;
+        uint32_t a = 0;
+        for (int b = 0; b < LGE; b++) a += ((e >> b) & 1u) * L.s[o + b];
+        return a;
+    }
+};
+
+template <class E, int LG, int LGV, int LGE, int I, bool ST>
+__device__ __forceinline__ void exchange(E* sm, E (&x)[1 << LGE]) {
+    using Pl = Place<E, LG, LGV, LGE, I>;
+#pragma unroll
+    for (uint32_t e = 0; e < (1u << LGE); e++) {
+        if (ST) sm[Pl::reg(e)] = x[e];
+        else x[e] = sm[Pl::reg(e)];
+    }
+}
+
+template <int LG, int LGV, int LGE>
+constexpr int kThreads = (1 << (LG + LGV - LGE)) > 128 ? (1 << (LG + LGV - LGE)) : 128;
+
+// SINGLE (LGV = 0, stride 1): rows of N = n elements, blockDim.y rows per CTA.
+// S0: first stage of the pass; above 0 the roots depend on the column (row u).
+// 2^LST: words between consecutive elements of a column.
+// CONT: outputs are stored column by column (transposed), else in place.
+// TSM: threads per SM that the registers are budgeted for.
+template <class A, class S, class D, int LG, int LGV, int LGE, bool INV, int S0, int LST, bool CONT, int TSM>
+__global__ void __launch_bounds__(kThreads<LG, LGV, LGE>, TSM / kThreads<LG, LGV, LGE> > 0 ? TSM / kThreads<LG, LGV, LGE> : 1)
+    radix_pass(const __grid_constant__ Args a, const LimbDev<A>* __restrict__ limbs) {
+    using E = typename A::elem;
+    using P = typename PairOf<A>::type;
+    constexpr uint32_t N = 1u << LG, NE = 1u << LGE, V = 1u << LGV, NT = N >> LGE;
+    constexpr Rounds<LG, LGE> R;
+    constexpr int NR = R.n;
+    constexpr bool kSingle = LGV == 0;
+    constexpr bool kLast = INV ? S0 == 0 : !CONT;  // the pass that leaves canonical residues
+    constexpr bool kReduce = sizeof(S) == 8 && sizeof(E) == 4;
+    extern __shared__ __align__(16) unsigned char rdx_smem[];
+    constexpr Lay<LG, LGV, sizeof(E) == 8 ? 4 : 5> L;
+    E* sm = reinterpret_cast<E*>(rdx_smem) + (kSingle ? threadIdx.y * L.words : 0u);
+
+    uint32_t limb, poly, col0 = 0, n_poly = 1;
+    bool active = true;
+    if (kSingle) {
+        uint32_t unit = blockIdx.x * blockDim.y + threadIdx.y;
+        active = unit < a.units;
+        if (!active) unit = a.units - 1;
+        limb = unit % a.n_limbs;
+        poly = unit / a.n_limbs;
+    } else {
+        limb = blockIdx.y;
+        poly = blockIdx.z * a.polys_per_cta;
+        n_poly = min(a.polys_per_cta, a.polys - poly);
+        col0 = blockIdx.x * V;
+    }
+    const uint32_t tid = threadIdx.x;
+    const uint32_t v_v = tid & (V - 1u), t_v = tid >> LGV;         // columns fastest
+    const uint32_t t_t = tid & (NT - 1u), v_t = tid / NT;          // positions fastest
+    const LimbDev<A>& ld = limbs[limb];
+    const A ar = ld.ar;
+    const P* tab = reinterpret_cast<const P*>(INV ? ld.rt_inv : ld.rt);
+    P c0{}, c1{}, one{};
+    if (INV && S0 == 0) {
+        c0 = __ldg(reinterpret_cast<const P*>(ld.scale));
+        c1 = __ldg(reinterpret_cast<const P*>(ld.scale) + 1);
+    }
+    if constexpr (kReduce) one = __ldg(tab + 1);  // cyclic tables: root^0 and floor(2^32 / q)
+    const uint64_t off = (uint64_t)poly * a.poly_stride + ((uint64_t)limb << a.log_n);
+    const S* src = reinterpret_cast<const S*>(a.src) + off;
+    D* dst = reinterpret_cast<D*>(a.dst) + off;
+    // round K's place of this thread and its roots
+    P w[NE - 1];
+    auto roots = [&](auto step) {
+        constexpr int K = decltype(step)::value, I = INV ? NR - 1 - K : K;
+        constexpr bool tfast = CONT && K == NR - 1;
+        using Pl = Place<E, LG, LGV, LGE, I>;
+        const uint32_t t = tfast ? t_t : t_v, col = col0 + (tfast ? v_t : v_v);
+        round_roots<LG, LGE, I, S0, INV>(w, tab + (S0 > 0 ? col : 0u) + ((size_t)Pl::natural(t) << S0));
+    };
+    roots(std::integral_constant<int, 0>{});
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+
+    E x[NE];
+    // strided load: element e of thread t is position t + e NT (forward), or the
+    // position whose natural index is rev(e) NT + t (inverse)
+    auto load = [&](uint32_t t, uint32_t col) {
+#pragma unroll
+        for (uint32_t e = 0; e < NE; e++) {
+            const uint32_t i = t + (INV ? brv(e, LGE) : e) * NT;
+            S w = __ldcg(src + ((kSingle ? (size_t)i : ((size_t)i << LST) + col)));
+            if constexpr (kReduce) {
+                const uint32_t y = (uint32_t)w;
+                x[e] = sub_if(y - __umulhi(y, one.y) * ar.q, ar.q);
+            } else {
+                x[e] = (E)w;
+            }
+        }
+    };
+    auto store = [&](uint32_t t, uint32_t col) {
+#pragma unroll
+        for (uint32_t e = 0; e < NE; e++) {
+            const uint32_t i = t + (INV ? e : brv(e, LGE)) * NT;
+            const E y = kLast ? canon_out<INV>(ar, x[e]) : x[e];
+            D* p = dst + (kSingle ? (size_t)i : CONT ? ((size_t)col << LG) + i : ((size_t)i << LST) + col);
+            if (active) *p = (D)y;
+        }
+    };
+    auto run = [&](auto self, auto step) -> void {
+        constexpr int K = decltype(step)::value;         // K-th round executed
+        constexpr int I = INV ? NR - 1 - K : K;          // its index in the forward order
+        constexpr bool tfast = CONT && K == NR - 1;
+        using Pl = Place<E, LG, LGV, LGE, I>;
+        const uint32_t t = tfast ? t_t : t_v, v = tfast ? v_t : v_v, col = col0 + v;
+        E* base = sm + (NR > 1 ? Pl::base(t) + v : 0u);
+        if constexpr (K == 0) load(t, col);
+        else exchange<E, LG, LGV, LGE, I, false>(base, x);
+        round_stages<A, LG, LGE, I, S0, INV>(ar, x, w, c0, c1);
+        if constexpr (K < NR - 1) {
+            exchange<E, LG, LGV, LGE, I, true>(base, x);
+            roots(std::integral_constant<int, K + 1>{});
+            __syncthreads();
+            self(self, std::integral_constant<int, K + 1>{});
+        } else {
+            store(t, col);
+        }
+    };
+    for (uint32_t k = 0; k < n_poly; k++) {
+        if (k) {
+            roots(std::integral_constant<int, 0>{});
+            __syncthreads();  // the tile's last reads precede the next polynomial's stores
+        }
+        run(run, std::integral_constant<int, 0>{});
+        src += a.poly_stride;
+        dst += a.poly_stride;
+    }
+}
+
+}  // namespace rdx
+}  // namespace nttb

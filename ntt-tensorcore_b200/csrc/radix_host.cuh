@@ -1,0 +1,128 @@
+// radix_host.cuh -- host side of the register-radix passes (radix.cuh): pass
+// geometry, tile choice and launches, instantiated per residue type by the
+// radix_*.cu files.
+#pragma once
+#include <cuda_runtime.h>
+
+#include "plan.hpp"
+#include "profiler.hpp"
+#include "radix.cuh"
+
+namespace nttb {
+namespace rdx {
+
+// Sizes served: one pass up to 2^kSingleMax (a tile holds the whole row), two
+// passes of 2^ceil(L/2) and 2^floor(L/2) points above.
+constexpr uint32_t kSingleMax = 13;
+constexpr uint32_t kThreadsMin = 128;  // rows are grouped into CTAs of at least this many threads
+
+template <class K>
+int launch(K kernel, const char* name, dim3 grid, dim3 block, size_t smem, const Args& a, const void* limbs,
+           cudaStream_t s) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    // the next pass sets up (addresses, roots) while this one drains; it reads
+    // no residue before this grid has completed (griddepcontrol.wait)
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    ProfScope prof(name, s);
+    void* params[2] = {const_cast<Args*>(&a), &limbs};
+    return launch_rc(cudaLaunchKernelExC(&cfg, reinterpret_cast<const void*>(kernel), params));
+}
+
+template <class A, class S, int LG, int LGE, bool INV>
+int launch_single(Args a, const LimbDev<A>* limbs, cudaStream_t s) {
+    using E = typename A::elem;
+    constexpr uint32_t NT = 1u << (LG - LGE);
+    constexpr Lay<LG, 0, sizeof(E) == 8 ? 4 : 5> L;
+    auto k = radix_pass<A, S, S, LG, 0, LGE, INV, 0, 0, false, 1024>;
+    uint32_t rows = NT < kThreadsMin ? kThreadsMin / NT : 1u;
+    while (rows > 1 && (a.units + rows - 1) / rows < 148) rows >>= 1;  // small calls spread over the SMs first
+    const size_t smem = (size_t)rows * L.words * sizeof(E);
+    if (smem > 48 * 1024) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    return launch(k, "scalar_pass_row", dim3((a.units + rows - 1) / rows), dim3(NT, rows), smem, a, limbs, s);
+}
+
+template <class A, class S, class D, int LG, int LGV, int LGE, bool INV, int S0, int LST, bool CONT>
+int launch_pass(Args a, const LimbDev<A>* limbs, cudaStream_t s) {
+    using E = typename A::elem;
+    constexpr Lay<LG, LGV, sizeof(E) == 8 ? 4 : 5> L;
+    constexpr size_t smem = (size_t)L.words * sizeof(E);
+    constexpr uint32_t tiles = 1u << (LST - LGV);
+    // a CTA keeps its columns' roots in L1 over several polynomials once the
+    // launch has CTAs to spare
+    const uint64_t ctas = (uint64_t)tiles * a.n_limbs * a.polys;
+    uint32_t ppc = (uint32_t)(ctas / 4096);
+    if (ppc < 1) ppc = 1;
+    if (ppc > a.polys) ppc = a.polys;
+    a.polys_per_cta = ppc;
+    // a grid of one wave is bound by each thread's own latency and runs faster
+    // with up to 128 registers a thread; larger ones are bound by L1 and issue
+    // and want twice the warps.  Forward / inverse of 24 x 2^16: 9.7 / 12.7 us
+    // against 11.9 / 14.8; of 192 x 2^16: 54.5 / 71.9 against 56.7 / 61.4;
+    // of 33 x 2^17: 26.5 / 30.4 against 22.8 / 26.0
+    constexpr uint32_t threads = 1u << (LG + LGV - LGE);
+    auto k = ctas * threads <= 148u * 1024u ? radix_pass<A, S, D, LG, LGV, LGE, INV, S0, LST, CONT, 512>
+                                            : radix_pass<A, S, D, LG, LGV, LGE, INV, S0, LST, CONT, 1024>;
+    if (smem > 48 * 1024) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    return launch(k, CONT ? "scalar_pass_col" : "scalar_pass_col_b",
+                  dim3(tiles, a.n_limbs, (a.polys + ppc - 1) / ppc), dim3(threads), smem, a, limbs, s);
+}
+
+// Columns per tile: a warp's loads touch 32 / V lines of 128 bytes, and at
+// V = 8 the L1 data pipe was 75 % busy with them (192 x 2^16: 72 % at V = 8,
+// 59 % at 16); 512 and 1024-point columns take half as many, which keeps two
+// CTAs on an SM (8 x 2^20: 54.9 us at V = 8, 62.8 at 16; 1 x 2^20: 10.0, 14.7).
+template <class A, class S, int L>
+constexpr int kLogCols = sizeof(typename A::elem) == 8 ? 2 : sizeof(S) == 8 ? 3 : L <= 17 ? 4 : 3;
+
+// Both passes of one size; S -> M -> S words (M: the workspace or destination).
+template <class A, class S, class M, int L, int LGE>
+int launch_two(Args a, void* mid, const LimbDev<A>* limbs, bool inverse, cudaStream_t s) {
+    constexpr int LA = (L + 1) / 2, LB = L / 2, LGV = kLogCols<A, S, L>;
+    void* dst = a.dst;
+    a.dst = mid;
+    int rc = inverse ? launch_pass<A, S, M, LB, LGV, LGE, true, LA, LA, true>(a, limbs, s)
+                     : launch_pass<A, S, M, LA, LGV, LGE, false, 0, LB, true>(a, limbs, s);
+    if (rc) return rc;
+    a.src = mid;
+    a.dst = dst;
+    return inverse ? launch_pass<A, M, S, LA, LGV, LGE, true, 0, LB, false>(a, limbs, s)
+                   : launch_pass<A, M, S, LB, LGV, LGE, false, LA, LA, false>(a, limbs, s);
+}
+
+// Runs one transform of n_polys x n_limbs rows; `mid` (two-pass sizes) holds
+// the first pass in words of M.  Returns 1 when the size is not served.
+template <class A, class S, class M, int LGE>
+int transform(const LimbDev<A>* limbs, uint32_t log_n, uint32_t n_limbs, const void* src, void* dst, void* mid,
+              uint32_t n_polys, bool inverse, cudaStream_t s) {
+    Args a{};
+    a.src = src;
+    a.dst = dst;
+    a.poly_stride = (uint64_t)n_limbs << log_n;
+    a.log_n = log_n;
+    a.polys = n_polys;
+    a.n_limbs = n_limbs;
+    a.units = n_polys * n_limbs;
+#define NTTB_SINGLE(l) \
+    case l: return inverse ? launch_single<A, S, l, LGE, true>(a, limbs, s) : launch_single<A, S, l, LGE, false>(a, limbs, s);
+#define NTTB_TWO(l) \
+    case l: return launch_two<A, S, M, l, LGE>(a, mid, limbs, inverse, s);
+    switch (log_n) {
+        NTTB_SINGLE(5) NTTB_SINGLE(6) NTTB_SINGLE(7) NTTB_SINGLE(8) NTTB_SINGLE(9)
+        NTTB_SINGLE(10) NTTB_SINGLE(11) NTTB_SINGLE(12) NTTB_SINGLE(13)
+        NTTB_TWO(14) NTTB_TWO(15) NTTB_TWO(16) NTTB_TWO(17) NTTB_TWO(18) NTTB_TWO(19) NTTB_TWO(20)
+        default: return 1;
+    }
+#undef NTTB_SINGLE
+#undef NTTB_TWO
+}
+
+}  // namespace rdx
+}  // namespace nttb

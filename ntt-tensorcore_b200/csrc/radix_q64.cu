@@ -1,0 +1,10 @@
+// radix_q64.cu -- register-radix passes (radix.cuh) for moduli below 2^62.
+#include "radix_host.cuh"
+
+namespace nttb {
+
+int radix_q64(const Plan64& p, const void* src, void* dst, void* mid, uint32_t n_polys, bool inverse, cudaStream_t s) {
+    return rdx::transform<M64, uint64_t, uint64_t, 3>(p.d_limbs, p.log_n, p.n_limbs, src, dst, mid, n_polys, inverse, s);
+}
+
+}  // namespace nttb

@@ -304,7 +304,8 @@ inline uint32_t tile_vectors(uint32_t e_max, uint32_t len, uint32_t n_vectors, u
     return v;
 }
 
-// Two-pass (or single-pass) forward/inverse over a plan.  E_max bounds the
+// Two-pass (or single-pass) forward/inverse over a plan, for the sizes that
+// the register-radix passes (radix.cuh) do not serve.  E_max bounds the
 // shared-memory tile in elements.  Two-pass layout for n = N1 * N2:
 //   pass A: columns b of x as [N1][N2]: U[d][b] = DFT_N1 * root^(d*b), stored
 //           transposed at b*N1 + d into `mid`;
@@ -312,16 +313,6 @@ inline uint32_t tile_vectors(uint32_t e_max, uint32_t len, uint32_t n_vectors, u
 //           the same positions of `dst` -- each tile reads and writes one set
 //           of positions, so pass B is safe in place.
 // Pass A cannot run in place; an in-place call stages it in `ws`.
-// Whether a transform runs as two passes: always above the tile size e_max;
-// from 2^12 on also when there are few (polynomial, limb) units, since a
-// single pass gives each unit one CTA and leaves the GPU idle (one
-// polynomial of 2^12 words: one CTA for all twelve stages).
-constexpr uint64_t kFewUnits = 8;
-inline bool two_pass(uint32_t log_n, uint32_t e_max, uint64_t units) {
-    const uint32_t n = 1u << log_n;
-    return n > e_max || (log_n >= 12 && units < kFewUnits);
-}
-
 template <class S, class A>
 int transform_generic(uint32_t log_n, uint32_t n_limbs, bool negacyclic, const LimbDev<A>* d_limbs,
                       const void* src, void* dst, void* ws, uint32_t n_polys, bool inverse, uint32_t e_max,
@@ -335,7 +326,7 @@ int transform_generic(uint32_t log_n, uint32_t n_limbs, bool negacyclic, const L
     a.inverse = inverse ? 1 : 0;
     uint32_t pre = (!inverse && negacyclic) ? F_PRE_PSI : 0u;
     uint32_t post = inverse ? (negacyclic ? F_POST_PSI_INV : F_POST_SCALE) : 0u;
-    if (!two_pass(log_n, e_max, (uint64_t)n_limbs * n_polys)) {
+    if (n <= e_max) {
         // single pass: one row of length n per (poly, limb)
         a.src = src;
         a.dst = dst;
@@ -377,38 +368,50 @@ int transform_generic(uint32_t log_n, uint32_t n_limbs, bool negacyclic, const L
 
 }  // namespace
 
+// Words that a transform stages outside source and destination: the two-pass
+// sizes' first pass, unless it can go to the destination.
+static size_t staged_words(uint32_t log_n, uint32_t e_max, uint32_t n_limbs, uint32_t n_polys) {
+    const bool two = radix_serves(log_n) ? log_n > kRadixSingleMax : (1u << log_n) > e_max;
+    return two ? ((size_t)n_polys * n_limbs) << log_n : 0;
+}
+
 int scalar_transform32(Plan32& p, const void* src, void* dst, bool src_u64, uint32_t n_polys, bool inverse,
                        cudaStream_t s) {
-    void* ws = nullptr;
-    if (src == dst && two_pass(p.log_n, 8192, (uint64_t)n_polys * p.n_limbs)) {
-        ws = plan_workspace(&p.ws, &p.ws_bytes, (size_t)n_polys * p.n_limbs * p.n * (src_u64 ? 8 : 4));
-        if (!ws) return 2;
+    const bool radix = radix_serves(p.log_n);
+    void* mid = dst;
+    if (const size_t words = staged_words(p.log_n, 8192, p.n_limbs, n_polys); words && (src == dst || (radix && src_u64))) {
+        mid = plan_workspace(&p.ws, &p.ws_bytes, words * (src_u64 && !radix ? 8 : 4));
+        if (!mid) return 2;
     }
+    if (n_polys > 65535 || p.n_limbs > 65535) return 1;
+    if (radix) return (src_u64 ? radix_w64 : radix_u32)(p, src, dst, mid, n_polys, inverse, s);
     if (src_u64)
-        return transform_generic<uint64_t, M32>(p.log_n, p.n_limbs, p.negacyclic, p.d_limbs, src, dst, ws, n_polys,
+        return transform_generic<uint64_t, M32>(p.log_n, p.n_limbs, p.negacyclic, p.d_limbs, src, dst, mid, n_polys,
                                                 inverse, 8192, s);
-    return transform_generic<uint32_t, M32>(p.log_n, p.n_limbs, p.negacyclic, p.d_limbs, src, dst, ws, n_polys,
+    return transform_generic<uint32_t, M32>(p.log_n, p.n_limbs, p.negacyclic, p.d_limbs, src, dst, mid, n_polys,
                                             inverse, 8192, s);
 }
 
 int scalar_transform32_ws(const Plan32& p, uint32_t* data, void* ws, uint32_t n_polys, bool inverse,
                           cudaStream_t s) {
+    if (radix_serves(p.log_n)) return p.n_limbs > 65535 ? 1 : radix_u32(p, data, data, ws, n_polys, inverse, s);
     return transform_generic<uint32_t, M32>(p.log_n, p.n_limbs, p.negacyclic, p.d_limbs, data, data, ws, n_polys,
                                             inverse, 8192, s);
 }
 
 size_t scalar_transform32_ws_bytes(const Plan32& p, uint32_t n_polys) {
-    if (!two_pass(p.log_n, 8192, (uint64_t)n_polys * p.n_limbs)) return 0;
-    return (size_t)n_polys * p.n_limbs * p.n * sizeof(uint32_t);
+    return staged_words(p.log_n, 8192, p.n_limbs, n_polys) * sizeof(uint32_t);
 }
 
 int scalar_transform64(Plan64& p, const void* src, void* dst, uint32_t n_polys, bool inverse, cudaStream_t s) {
-    void* ws = nullptr;
-    if (src == dst && two_pass(p.log_n, 4096, (uint64_t)n_polys * p.n_limbs)) {
-        ws = plan_workspace(&p.ws, &p.ws_bytes, (size_t)n_polys * p.n_limbs * p.n * 8);
-        if (!ws) return 2;
+    void* mid = dst;
+    if (const size_t words = staged_words(p.log_n, 4096, p.n_limbs, n_polys); words && src == dst) {
+        mid = plan_workspace(&p.ws, &p.ws_bytes, words * 8);
+        if (!mid) return 2;
     }
-    return transform_generic<uint64_t, M64>(p.log_n, p.n_limbs, p.negacyclic, p.d_limbs, src, dst, ws, n_polys,
+    if (n_polys > 65535 || p.n_limbs > 65535) return 1;
+    if (radix_serves(p.log_n)) return radix_q64(p, src, dst, mid, n_polys, inverse, s);
+    return transform_generic<uint64_t, M64>(p.log_n, p.n_limbs, p.negacyclic, p.d_limbs, src, dst, mid, n_polys,
                                             inverse, 4096, s);
 }
 
