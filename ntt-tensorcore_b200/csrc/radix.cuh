@@ -58,21 +58,26 @@ __device__ __forceinline__ uint32_t brv_dev(uint32_t x, int bits) { return bits 
 
 // Strides (in elements) of the LG position bits in shared memory; column v
 // sits at offset v.  NB = log2 of the banks counted in elements (5 for 4-byte,
-// 4 for 8-byte elements).  The bits next to either end get distinct
-// power-of-two residues mod 2^NB, in the order in which lanes enumerate them:
-// first those above the V columns', then the columns' own.
-template <int LG, int LGV, int NB>
+// 4 for 8-byte elements).  The NP bits next to either end, those that a warp's
+// lanes enumerate, get distinct power-of-two residues mod 2^NB: first those
+// above the V columns' own (lanes that run over columns, then positions), then
+// the highest of the columns' (lanes that run over positions, then columns).
+// Any order of one set does; the one taken keeps the padding below 13 % (a
+// descending one took up to 50 %).
+template <int LG, int LGV, int NB, int NP>
 struct Lay {
     uint32_t s[LG > 0 ? LG : 1] = {};
     uint32_t words = 0;
     constexpr Lay() {
         uint32_t sum = (1u << LGV) - 1u;
         const uint32_t mod = 1u << NB;
+        const int above = NB > LGV ? NB - LGV : 0;
         for (int i = 0; i < LG; i++) {
-            const int pos = i < LG / 2 ? i : LG - 1 - i;
+            const bool top = i >= LG / 2;
+            const int pos = top ? LG - 1 - i : i;
             uint32_t st = sum + 1u;
-            if (pos < NB) {
-                const int bit = pos < NB - LGV ? LGV + pos : NB - 1 - pos;
+            if (pos < NP) {
+                const int bit = LGV == 0 && top && LG >= 2 * NB ? NB - 1 - pos : pos < above ? LGV + pos : NB - NP + pos - above;
                 while ((st & (mod - 1u)) != (1u << bit)) st++;
             }
             s[i] = st;
@@ -81,6 +86,11 @@ struct Lay {
         words = sum + 1u;
     }
 };
+template <class E>
+constexpr int kBankBits = sizeof(E) == 8 ? 4 : 5;
+// Lanes of the passes below: up to NB positions of one column.
+template <class E, int LG, int LGV, int LGE>
+constexpr int kLanePos = LGV == 0 || LG - LGE > kBankBits<E> ? kBankBits<E> : LG - LGE;
 
 // Stages per round: the last takes LGE, the ones before it share the rest.
 template <int LG, int LGE>
@@ -170,53 +180,50 @@ __device__ __forceinline__ ulonglong2 ld_pair(const ulonglong2* p) {
 // Roots of round I: w[2^j - 1 + kt] for the round's stage j and block bits kt.
 // `tw` points at tab + U (U the natural index of the thread's block at the
 // round's first stage S): stage S + j, bits kt sit at 2^(S+j) + rev_j(kt) 2^S.
-template <int LG, int LGE, int I, int S0, bool INV, class P>
+template <int LG, int LGE, int I, int S0, bool INV, int JJ = 0, class P>
 __device__ __forceinline__ void round_roots(P (&w)[(1 << LGE) - 1], const P* tw) {
     constexpr Rounds<LG, LGE> R;
-    constexpr int r = R.r[I], S = S0 + R.s0[I];
-#pragma unroll
-    for (int jj = 0; jj < r; jj++) {
-        const int j = INV ? r - 1 - jj : jj;
-        if (INV && S + j == 0) continue;  // the inverse's last stage multiplies by its scale
+    constexpr int r = R.r[I], S = S0 + R.s0[I], j = INV ? r - 1 - JJ : JJ;
+    if constexpr (!(INV && S + j == 0)) {  // the inverse's last stage multiplies by its scale
 #pragma unroll
         for (uint32_t kt = 0; kt < (1u << j); kt++)
             w[(1u << j) - 1u + kt] = ld_pair(tw + ((size_t)1 << (S + j)) + ((size_t)brv(kt, j) << S));
     }
+    if constexpr (JJ + 1 < r) round_roots<LG, LGE, I, S0, INV, JJ + 1>(w, tw);
 }
 
-// Stages of round I on the registers.
-template <class A, int LG, int LGE, int I, int S0, bool INV, class E, class P>
+// Stages of round I on the registers.  One instance per stage: as one loop nest
+// the compiler kept the inverse's registers in local memory.
+template <class A, int LG, int LGE, int I, int S0, bool INV, int JJ = 0, class E, class P>
 __device__ __forceinline__ void round_stages(const A& ar, E (&x)[1 << LGE], const P (&w)[(1 << LGE) - 1], P c0, P c1) {
     constexpr Rounds<LG, LGE> R;
     constexpr int r = R.r[I], S = S0 + R.s0[I], xb = LGE - r;  // xb: extra held bits below the radix bits
+    constexpr int j = INV ? r - 1 - JJ : JJ;
+    constexpr uint32_t half = 1u << (r - 1 - j);
 #pragma unroll
-    for (int jj = 0; jj < r; jj++) {
-        const int j = INV ? r - 1 - jj : jj;
-        const uint32_t half = 1u << (r - 1 - j);
+    for (uint32_t kt = 0; kt < (1u << j); kt++)
 #pragma unroll
-        for (uint32_t kt = 0; kt < (1u << j); kt++)
+        for (uint32_t lo = 0; lo < half; lo++)
 #pragma unroll
-            for (uint32_t lo = 0; lo < half; lo++)
-#pragma unroll
-                for (uint32_t g = 0; g < (1u << xb); g++) {
-                    const uint32_t ia = (((kt << (r - j)) + lo) << xb) + g, ib = ia + (half << xb);
-                    if (INV && S + j == 0) gs_scaled(ar, x[ia], x[ib], c0, c1);
-                    else if (INV) gs(ar, x[ia], x[ib], w[(1u << j) - 1u + kt]);
-                    else ct(ar, x[ia], x[ib], w[(1u << j) - 1u + kt]);
-                }
-    }
+            for (uint32_t g = 0; g < (1u << xb); g++) {
+                const uint32_t ia = (((kt << (r - j)) + lo) << xb) + g, ib = ia + (half << xb);
+                if constexpr (INV && S + j == 0) gs_scaled(ar, x[ia], x[ib], c0, c1);
+                else if constexpr (INV) gs(ar, x[ia], x[ib], w[(1u << j) - 1u + kt]);
+                else ct(ar, x[ia], x[ib], w[(1u << j) - 1u + kt]);
+            }
+    if constexpr (JJ + 1 < r) round_stages<A, LG, LGE, I, S0, INV, JJ + 1>(ar, x, w, c0, c1);
 }
 
 // One round's place of a thread: its base offset in shared memory, and the
 // natural index of its block within the pass.
-template <class E, int LG, int LGV, int LGE, int I>
+template <class E, int LG, int LGV, int LGE, int I, int NP = kLanePos<E, LG, LGV, LGE>>
 struct Place {
-    static constexpr int NB = sizeof(E) == 8 ? 4 : 5;
+    static constexpr int NB = kBankBits<E>;
     static constexpr Rounds<LG, LGE> R{};
     static constexpr int s0 = R.s0[I], T = LG - s0, o = T - LGE;
     static constexpr bool last = I == R.n - 1;
     __device__ __forceinline__ static uint32_t base(uint32_t t) {
-        constexpr Lay<LG, LGV, NB> L;
+        constexpr Lay<LG, LGV, NB, NP> L;
         uint32_t a = 0;
 #pragma unroll
         for (int b = 0; b < LG - LGE; b++) {
@@ -232,18 +239,17 @@ struct Place {
         return last ? h : brv_dev(h, s0);
     }
     static constexpr uint32_t reg(uint32_t e) {
-        Lay<LG, LGV, NB> L;
+        Lay<LG, LGV, NB, NP> L;
         uint32_t a = 0;
         for (int b = 0; b < LGE; b++) a += ((e >> b) & 1u) * L.s[o + b];
         return a;
     }
 };
 
-template <class E, int LG, int LGV, int LGE, int I, bool ST>
-__device__ __forceinline__ void exchange(E* sm, E (&x)[1 << LGE]) {
-    using Pl = Place<E, LG, LGV, LGE, I>;
+template <class Pl, bool ST, class E, int NE>
+__device__ __forceinline__ void exchange(E* sm, E (&x)[NE]) {
 #pragma unroll
-    for (uint32_t e = 0; e < (1u << LGE); e++) {
+    for (uint32_t e = 0; e < NE; e++) {
         if (ST) sm[Pl::reg(e)] = x[e];
         else x[e] = sm[Pl::reg(e)];
     }
@@ -269,7 +275,7 @@ __global__ void __launch_bounds__(kThreads<LG, LGV, LGE>, TSM / kThreads<LG, LGV
     constexpr bool kLast = INV ? S0 == 0 : !CONT;  // the pass that leaves canonical residues
     constexpr bool kReduce = sizeof(S) == 8 && sizeof(E) == 4;
     extern __shared__ __align__(16) unsigned char rdx_smem[];
-    constexpr Lay<LG, LGV, sizeof(E) == 8 ? 4 : 5> L;
+    constexpr Lay<LG, LGV, kBankBits<E>, kLanePos<E, LG, LGV, LGE>> L;
     E* sm = reinterpret_cast<E*>(rdx_smem) + (kSingle ? threadIdx.y * L.words : 0u);
 
     uint32_t limb, poly, col0 = 0, n_poly = 1;
@@ -316,12 +322,13 @@ __global__ void __launch_bounds__(kThreads<LG, LGV, LGE>, TSM / kThreads<LG, LGV
 
     E x[NE];
     // strided load: element e of thread t is position t + e NT (forward), or the
-    // position whose natural index is rev(e) NT + t (inverse)
+    // position whose natural index is rev(e) NT + t (inverse); the parts share no
+    // bit, so every address is a thread's base plus a constant
     auto load = [&](uint32_t t, uint32_t col) {
+        const S* p = src + (((size_t)t << LST) + col);
 #pragma unroll
         for (uint32_t e = 0; e < NE; e++) {
-            const uint32_t i = t + (INV ? brv(e, LGE) : e) * NT;
-            S w = __ldcg(src + ((kSingle ? (size_t)i : ((size_t)i << LST) + col)));
+            const S w = __ldcg(p + ((size_t)((INV ? brv(e, LGE) : e) * NT) << LST));
             if constexpr (kReduce) {
                 const uint32_t y = (uint32_t)w;
                 x[e] = sub_if(y - __umulhi(y, one.y) * ar.q, ar.q);
@@ -331,12 +338,11 @@ __global__ void __launch_bounds__(kThreads<LG, LGV, LGE>, TSM / kThreads<LG, LGV
         }
     };
     auto store = [&](uint32_t t, uint32_t col) {
+        D* p = dst + (CONT ? ((size_t)col << LG) + t : ((size_t)t << LST) + col);
 #pragma unroll
         for (uint32_t e = 0; e < NE; e++) {
-            const uint32_t i = t + (INV ? e : brv(e, LGE)) * NT;
             const E y = kLast ? canon_out<INV>(ar, x[e]) : x[e];
-            D* p = dst + (kSingle ? (size_t)i : CONT ? ((size_t)col << LG) + i : ((size_t)i << LST) + col);
-            if (active) *p = (D)y;
+            if (active) p[(size_t)((INV ? e : brv(e, LGE)) * NT) << (CONT ? 0 : LST)] = (D)y;
         }
     };
     auto run = [&](auto self, auto step) -> void {
@@ -347,10 +353,10 @@ __global__ void __launch_bounds__(kThreads<LG, LGV, LGE>, TSM / kThreads<LG, LGV
         const uint32_t t = tfast ? t_t : t_v, v = tfast ? v_t : v_v, col = col0 + v;
         E* base = sm + (NR > 1 ? Pl::base(t) + v : 0u);
         if constexpr (K == 0) load(t, col);
-        else exchange<E, LG, LGV, LGE, I, false>(base, x);
+        else exchange<Pl, false>(base, x);
         round_stages<A, LG, LGE, I, S0, INV>(ar, x, w, c0, c1);
         if constexpr (K < NR - 1) {
-            exchange<E, LG, LGV, LGE, I, true>(base, x);
+            exchange<Pl, true>(base, x);
             roots(std::integral_constant<int, K + 1>{});
             __syncthreads();
             self(self, std::integral_constant<int, K + 1>{});

@@ -40,7 +40,7 @@ template <class A, class S, int LG, int LGE, bool INV>
 int launch_single(Args a, const LimbDev<A>* limbs, cudaStream_t s) {
     using E = typename A::elem;
     constexpr uint32_t NT = 1u << (LG - LGE);
-    constexpr Lay<LG, 0, sizeof(E) == 8 ? 4 : 5> L;
+    constexpr Lay<LG, 0, kBankBits<E>, kLanePos<E, LG, 0, LGE>> L;
     auto k = radix_pass<A, S, S, LG, 0, LGE, INV, 0, 0, false, 1024>;
     uint32_t rows = NT < kThreadsMin ? kThreadsMin / NT : 1u;
     while (rows > 1 && (a.units + rows - 1) / rows < 148) rows >>= 1;  // small calls spread over the SMs first
@@ -52,7 +52,7 @@ int launch_single(Args a, const LimbDev<A>* limbs, cudaStream_t s) {
 template <class A, class S, class D, int LG, int LGV, int LGE, bool INV, int S0, int LST, bool CONT>
 int launch_pass(Args a, const LimbDev<A>* limbs, cudaStream_t s) {
     using E = typename A::elem;
-    constexpr Lay<LG, LGV, sizeof(E) == 8 ? 4 : 5> L;
+    constexpr Lay<LG, LGV, kBankBits<E>, kLanePos<E, LG, LGV, LGE>> L;
     constexpr size_t smem = (size_t)L.words * sizeof(E);
     constexpr uint32_t tiles = 1u << (LST - LGV);
     // a CTA keeps its columns' roots in L1 over several polynomials once the
@@ -64,9 +64,8 @@ int launch_pass(Args a, const LimbDev<A>* limbs, cudaStream_t s) {
     a.polys_per_cta = ppc;
     // a grid of one wave is bound by each thread's own latency and runs faster
     // with up to 128 registers a thread; larger ones are bound by L1 and issue
-    // and want twice the warps.  Forward / inverse of 24 x 2^16: 9.7 / 12.7 us
-    // against 11.9 / 14.8; of 192 x 2^16: 54.5 / 71.9 against 56.7 / 61.4;
-    // of 33 x 2^17: 26.5 / 30.4 against 22.8 / 26.0
+    // and want twice the warps.  Forward of 24 x 2^16: 9.7 us against 11.9; of
+    // 33 x 2^17: 26.5 against 22.8
     constexpr uint32_t threads = 1u << (LG + LGV - LGE);
     auto k = ctas * threads <= 148u * 1024u ? radix_pass<A, S, D, LG, LGV, LGE, INV, S0, LST, CONT, 512>
                                             : radix_pass<A, S, D, LG, LGV, LGE, INV, S0, LST, CONT, 1024>;
