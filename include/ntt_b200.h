@@ -41,7 +41,7 @@ enum {
 
 /* Inner-DFT engines.  AUTO picks one that serves the request: out of place the
  * CUDA-core engine; in place the INT8 tensor-core kernel at N = 2^16 from 8
- * (polynomial, limb) units on, the batch queue's tensor tiles at N = 2^17 ..
+ * (polynomial, limb) units on, the batch queue at N = 2^17 ..
  * 2^20 once a call holds 2^20 residues, the CUDA-core engine otherwise (it
  * stages its first pass in the plan's workspace).  The tiles engine keeps up
  * to eight prepared queues per plan (one per source, destination, count,
@@ -51,7 +51,8 @@ enum {
     NTTB_ENGINE_SCALAR = 1, /* CUDA-core radix-2 stages in registers and shared memory */
     NTTB_ENGINE_DMMA = 2,   /* FP64 mma.sync m8n8k4 radix-8 contractions (the plain drop-in form) */
     NTTB_ENGINE_INT8 = 3,   /* tcgen05 kind::i8, byte-plane radix-64 contractions, INT32 in TMEM */
-    NTTB_ENGINE_TILES = 4   /* the batch queue's tcgen05 tensor tiles (two-pass four-step, 2^13 .. 2^20) */
+    NTTB_ENGINE_TILES = 4   /* the batch queue's tcgen05 tensor tiles (two-pass four-step, 2^13 .. 2^20);
+                               AUTO's calls run the queue's register-radix tiles instead */
 };
 
 NTTB_API const char* nttb_version(void);
@@ -133,7 +134,7 @@ NTTB_API int nttb_plan_get_info(const nttb_plan* plan, nttb_plan_info* out);
  * (src/ntt_basic.cu:268-334, src/ntt_optimized.cu:515-613) and
  * ntt_forward/inverse_batch (src/ntt_basic.cu:337-389).  NTTB_ENGINE_AUTO
  * runs, for q < 2^31, the INT8 tensor-core kernel on the words directly for
- * n = 2^16 from 8 polynomials on, the batch queue's tensor tiles for
+ * n = 2^16 from 8 polynomials on, the batch queue for
  * n = 2^17 .. 2^20 from 2^20 words per call, the CUDA-core engine otherwise
  * (residues must be below 2^32, as the reference's kernels assume them below
  * q). */
@@ -280,9 +281,11 @@ typedef struct {
     uint32_t lag;         /* two-pass units between a unit's first and second pass in the queue (1..64) */
     uint32_t ctas_per_sm; /* 0: as many as fit */
     uint32_t group;       /* radix-2 stages per register group inside a tile: 1, 3 or 4 */
-    uint32_t tensor;      /* 1: two-pass units of 2^13 .. 2^20 residues (the sizes above the tile) run
-                             tensor-core tiles (INT8 DFT-64 + radix-2 DFT of up to 16 points) where the
-                             shape allows: threads 256 and tile_elems 4096 or 8192; otherwise ignored */
+    uint32_t tensor;      /* 1 (threads 256 and tile_elems 4096 or 8192; otherwise ignored): a batch with
+                             units of 2^10 .. 2^20 residues runs the queue's register-radix tiles, which
+                             take the lag alone; where a job is off a 16-byte boundary or their root
+                             tables do not fit in memory, tensor-core tiles (INT8 DFT-64 + radix-2 DFT of
+                             up to 16 points) for the two-pass units of 2^13 .. 2^20 above the tile */
 } nttb_batch_config;
 
 /* flags: NTTB_NEGACYCLIC to allow negacyclic jobs (moduli then need 2^(max_log_n+1) | q-1). */

@@ -38,6 +38,13 @@
 // barrier and one shared-memory round trip per group.  Twiddles and twists
 // come from two-level power tables (8 KB per base and modulus, L2-resident).
 //
+// Batches with units of 2^10 .. 2^20 residues run register-radix tiles instead
+// (batch_radix.cuh, the default configuration): 145 - 260 G residues/s by size,
+// against 80 - 100 on the tensor tiles below and less on the CUDA-core tiles.
+// 96 mixed polynomials (283 M residues): 3.01 -> 1.53 ms; twelve products of
+// 12 x 2^14: 107 -> 49 us.  The tensor tiles serve the named tiles engine and
+// jobs off a 16-byte boundary.
+//
 // Tuning knobs (nttb_batch_config): shared-memory tile size and CTA width
 // (4096/256, 8192/256, 8192/512, 16384/512), stages per register group (3,
 // 4, or 1 = stage by stage), the radix split of two-pass units (first pass 2^ceil(L/2) or
@@ -48,6 +55,7 @@
 #include <algorithm>
 #include <cstring>
 #include <deque>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -58,6 +66,7 @@
 #include "engines.hpp"
 #include "plan.hpp"
 #include "profiler.hpp"
+#include "radix.cuh"
 #include "tc_arith.cuh"
 #include "tcgen05.cuh"
 
@@ -73,9 +82,9 @@ namespace {
 
 constexpr uint32_t BF_INV = 1, BF_PRE_PSI = 2, BF_POST_TW = 4, BF_STORE_T = 8, BF_POST_SCALE = 16, BF_POST_PSI = 32,
                    BF_PRE_MUL = 64;
-// UF_TC: tensor-core tiles; UF_W64: the unit's data (and its source) are
-// uint64 words holding residues (tensor-tile two-pass units only)
-constexpr uint32_t UF_INV = 1, UF_NEGA = 2, UF_TC = 4, UF_W64 = 8;
+// UF_TC: tensor-core tiles; UF_RX: register-radix tiles; UF_W64: the unit's data (and its source) are
+// uint64 words holding residues (two-pass units of either kind only)
+constexpr uint32_t UF_INV = 1, UF_NEGA = 2, UF_TC = 4, UF_W64 = 8, UF_RX = 16;
 constexpr uint32_t kMaxRows = 32;
 
 // Power tables: x^e R for e < 2^max_log as hi[e >> kLoBits] * lo[e & lo_mask]
@@ -100,6 +109,17 @@ __device__ __forceinline__ uint32_t pw(const BModulus& M, const M32& ar, uint32_
     return ar.mul(__ldg(t + (e >> M.lo_bits)), __ldg(t + M.hi_len + (e & ((1u << M.lo_bits) - 1))));
 }
 
+// Register-radix tiles (batch_radix.cuh): per-modulus roots by kind (bit 0
+// inverse, bit 1 negacyclic; null until a batch needs the kind) and the
+// inverse's scale [negacyclic][product][log2 n]: Shoup pairs of c and c W, c =
+// n^-1 (times 2^32 for a product), W the inverse's root of its last stage.
+struct RxModulus {
+    M32 ar;
+    const uint2* pairs[4];
+    const uint32_t* quot[4];
+    uint2 scale[2][2][25][2];
+};
+
 struct BUnit {
     uint32_t* data;    // row 0 of the unit; row r (limb) at data + r n (uint64 words with UF_W64)
     const void* in;    // pass A reads here instead of data (same layout), or null
@@ -120,7 +140,10 @@ struct BUnit {
     uint32_t after_ctr[2];
     uint32_t dis;      // tensor-tile two-pass units: first of the unit's discard-group counters
                        // (after the 1 + 2 n_units queue counters), else kNoDiscard
-    uint32_t pad_[2];
+    M32 ar;            // register-radix two-pass units: the modulus, its roots and scale
+    const uint2* pairs;
+    const uint32_t* quot;
+    uint2 scale[2], one, pad_;
 };
 static_assert(sizeof(BUnit) % 16 == 0, "unit records are copied in 16-byte pieces");
 
@@ -159,6 +182,7 @@ struct BArgs {
     const uint32_t* ws;     // the workspace rings, ws_words words
     uint64_t ws_words;
     uint32_t n_dis;         // discard-group counters after the queue counters
+    const RxModulus* rx;
 };
 
 // NTT_DEBUG_BOUNDS build: the tile's unit, its tile index and its workspace
@@ -194,9 +218,14 @@ __device__ __forceinline__ bool wait_ge(const uint32_t* p, uint32_t target) {
 // One tile: V vectors of length len, in shared memory.  COL mode (DIT after
 // a bit-reversed load): vectors are columns vec of a [len][C] matrix; ROW
 // mode (DIF, bit-reversed read at the store): vectors are rows of n words.
-template <uint32_t T, uint32_t kGroup>
+// kNamed: the T threads are not the whole CTA and meet on barrier 1.
+template <uint32_t T, uint32_t kGroup, bool kNamed = false>
 __device__ __forceinline__ void run_tile(const BArgs& a, const BUnit& u, uint32_t pass, uint32_t tile, uint32_t* sm,
                                          M32* s_ar) {
+    auto tile_sync = []() {
+        if constexpr (kNamed) asm volatile("bar.sync 1, %0;" ::"n"(T) : "memory");
+        else __syncthreads();
+    };
     const uint32_t L = u.log_n, n = 1u << L, shift = a.max_log - L;
     const bool inv = u.flags & UF_INV, nega = u.flags & UF_NEGA;
     bool row;
@@ -248,7 +277,7 @@ __device__ __forceinline__ void run_tile(const BArgs& a, const BUnit& u, uint32_
         const BModulus& M = a.mods[u.mod0 + r];
         tws[i] = pw(M, M.ar, inv ? PW_OMEGA_INV : PW_OMEGA, k << (a.max_log - lg));
     }
-    __syncthreads();
+    tile_sync();
     // ---- load ----
     const uint32_t total = V * len;
     for (uint32_t idx = threadIdx.x; idx < total; idx += T) {
@@ -278,7 +307,7 @@ __device__ __forceinline__ void run_tile(const BArgs& a, const BUnit& u, uint32_
         const uint32_t jj = row ? j : bitrev(j, (int)lg);
         t[v * stride + jj + (jj >> 5)] = x;
     }
-    __syncthreads();
+    tile_sync();
     // ---- radix-2 stages, up to kGroup at a time in registers ----
     // A group of r stages s0 .. s0+r-1 touches, for each base index with
     // zero bits [s0, s0 + r), exactly the 2^r elements base + k 2^s0; one
@@ -322,7 +351,7 @@ __device__ __forceinline__ void run_tile(const BArgs& a, const BUnit& u, uint32_
                         rw[i + (i >> 5)] = x[k];
                     }
             }
-            __syncthreads();
+            tile_sync();
         }
     } else {
         // DIF: stages from lg-1 down, groups [s_lo, s_lo + r)
@@ -363,7 +392,7 @@ __device__ __forceinline__ void run_tile(const BArgs& a, const BUnit& u, uint32_
                         rw[i + (i >> 5)] = x[k];
                     }
             }
-            __syncthreads();
+            tile_sync();
         }
     }
     // ---- store ----
@@ -977,6 +1006,30 @@ __global__ void __launch_bounds__(T, (G == 1 ? 1536u : G == 3 ? 768u : 512u) / T
     }
 }
 
+#include "batch_radix.cuh"
+
+// Roots of one kind for every modulus (blockIdx.y): quotients floor(w 2^32 / q)
+// of the entries 2^s + i, s < log_r, and the Shoup pairs (w, quotient) of the
+// first 2^log_p.  The quotient is (w 2^32 mod q) (-q^-1) mod 2^32.
+__global__ void rx_roots_kernel(const BModulus* mods, uint32_t max_log, uint32_t log_r, uint32_t log_p, uint32_t kind,
+                                uint2* pairs, uint32_t* quot) {
+    const BModulus& M = mods[blockIdx.y];
+    const M32 ar = M.ar;
+    const bool nega = kind & 2u;
+    const uint32_t base = nega ? (kind & 1u ? PW_PSI_INV : PW_PSI) : (kind & 1u ? PW_OMEGA_INV : PW_OMEGA);
+    pairs += (size_t)blockIdx.y << log_p;
+    quot += (size_t)blockIdx.y << log_r;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < (1u << log_r); i += gridDim.x * blockDim.x) {
+        uint32_t r = 0;
+        if (i) {
+            const uint32_t s = 31 - __clz(i), k = i - (1u << s);
+            r = pw(M, ar, base, (nega ? 1u + 2u * k : k) << (max_log - s - 1));
+        }
+        quot[i] = r * ar.qinv;
+        if (i < (1u << log_p)) pairs[i] = make_uint2(ar.mul(r, 1u), r * ar.qinv);
+    }
+}
+
 // ---- host ------------------------------------------------------------------------
 struct Variant {
     uint32_t E, T, G, tensor;
@@ -994,6 +1047,9 @@ const Variant kVariants[] = {
     {4096, 256, 4, 1, batch_queue_tc<4>},            {8192, 256, 1, 1, batch_queue_tc<1>},
     {8192, 256, 3, 1, batch_queue_tc<3>},            {8192, 256, 4, 1, batch_queue_tc<4>},
 };
+// the register-radix tiles, over uint32 and over uint64 words (tensor 2: not a configuration)
+const Variant kRadixVariant = {kRxTile, kRxThreads, 3, 2, batch_queue_radix<false>};
+const Variant kRadixW64Variant = {kRxTile, kRxThreads, 3, 2, batch_queue_radix<true>};
 
 const Variant* find_variant(uint32_t E, uint32_t T, uint32_t G, uint32_t tensor) {
     for (const Variant& v : kVariants)
@@ -1003,7 +1059,12 @@ const Variant* find_variant(uint32_t E, uint32_t T, uint32_t G, uint32_t tensor)
 
 // padded tile (E + E/32 + one word per vector) + root powers + slack, in bytes
 size_t smem_bytes(uint32_t E) { return ((size_t)E + E / 16 + kMaxRows + E / 2) * 4 + 64; }
-size_t smem_bytes(const Variant* v) { return v->tensor ? kTcSmem : smem_bytes(v->E); }
+size_t smem_bytes(const Variant* v) {
+    if (v->tensor == 2) return std::max<size_t>((2 * kRxTile + 2 * kRxFew) * 4 + smem_bytes(kRxCoreTile), (size_t)kRxWords * 4);
+    return v->tensor ? kTcSmem : smem_bytes(v->E);
+}
+// CTA width: the radix kernel has a warp that feeds its tiles.
+uint32_t cta_threads(const Variant* v) { return v->tensor == 2 ? v->T + 32 : v->T; }
 
 // Byte-plane image of an 8 x 8 matrix for the level-2 contraction: 32 rows
 // (a, k) x 32 bytes (j, p), K-major SW32 (1 KB).
@@ -1027,11 +1088,11 @@ int resident_ctas(const Variant* v, uint32_t ctas_per_sm) {
     int dev = 0, sms = 0, occ = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, v->fn, (int)v->T, smem) != cudaSuccess) {
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, v->fn, (int)cta_threads(v), smem) != cudaSuccess) {
         cudaGetLastError();
         occ = 1;
     }
-    if (v->tensor) {
+    if (v->tensor == 1) {
         // The runtime's answer for the tcgen05 kernel is one CTA per SM; its
         // registers and shared memory fit two (and TMEM holds two 256-column
         // allocations), so count from the resources themselves.
@@ -1063,6 +1124,9 @@ uint32_t ilog2(uint64_t x) {
 
 struct BatchPlan::Mods {
     BModulus* d = nullptr;
+    RxModulus* rx = nullptr;         // device copy of rx_host
+    std::vector<RxModulus> rx_host;
+    std::mutex mu;                   // guards the lazy tables (rx, images)
 };
 
 struct Batch {
@@ -1122,21 +1186,35 @@ bool tensor_tiles(const nttb_batch_config& cfg) {
     return cfg.tensor && find_variant(cfg.tile_elems, cfg.threads, cfg.group, 1);
 }
 
+// Which tiles a batch runs: the configured CUDA-core ones alone, with tensor
+// tiles for the two-pass units, or the register-radix ones.
+enum class Tiles { kCore, kTensor, kRadix };
+
 // Pass geometry of a unit of 2^L residues (rows: limbs per single-pass tile).
 struct UnitShape {
     uint32_t lg1 = 0, per = 1, va = 0, vb = 0, tiles_a = 1, tiles_b = 0;
-    bool tc = false;
+    bool tc = false, rx = false;
 };
-bool unit_shape(const BatchPlan& P, const nttb_batch_config& cfg, uint32_t L, UnitShape* s) {
-    const uint32_t E = cfg.tile_elems, lgE = ilog2(E), n = 1u << L;
+bool unit_shape(const nttb_batch_config& cfg, Tiles kind, uint32_t L, UnitShape* s) {
     *s = UnitShape();
+    s->rx = kind == Tiles::kRadix && L >= kRxMinLog && L <= kRxMaxLog;
+    const uint32_t E = s->rx ? kRxTile : kind == Tiles::kRadix ? kRxCoreTile : cfg.tile_elems;
+    const uint32_t lgE = ilog2(E), n = 1u << L;
     // tensor-core two-pass units: both pass lengths 64 r', r' in 1..16
-    s->tc = tensor_tiles(cfg) && P.images && L > lgE && L >= 13 && L <= 20;
+    s->tc = kind == Tiles::kTensor && L > lgE && L >= 13 && L <= 20;
     if (L <= lgE) {
         s->per = std::min<uint32_t>(E >> L, kMaxRows);
         return true;
     }
     uint32_t lg1 = cfg.split ? L / 2 : (L + 1) / 2;
+    if (s->rx) {
+        lg1 = (L + 1) / 2;
+        s->va = kRxTile >> lg1;
+        s->vb = kRxTile >> (L - lg1);
+        s->tiles_a = s->tiles_b = n / kRxTile;
+        s->lg1 = lg1;
+        return true;
+    }
     if (s->tc) {
         lg1 = std::max<uint32_t>(lg1, std::max<uint32_t>(6, L - 10));
         lg1 = std::min<uint32_t>(lg1, std::min<uint32_t>(10, L - 6));
@@ -1166,11 +1244,11 @@ struct WsLayout {
     uint32_t slots[25] = {};
     uint64_t words = 0;
 };
-WsLayout ws_layout(const BatchPlan& P, const nttb_batch_config& cfg, const uint32_t* count) {
+WsLayout ws_layout(const BatchPlan& P, const nttb_batch_config& cfg, Tiles kind, const uint32_t* count) {
     WsLayout w;
     for (uint32_t L = 1; L <= P.max_log; L++) {
         UnitShape sh;
-        if (!unit_shape(P, cfg, L, &sh) || !sh.lg1) continue;
+        if (!unit_shape(cfg, kind, L, &sh) || !sh.lg1) continue;
         if (count && !count[L]) continue;
         uint32_t S = std::max<uint32_t>(16, cfg.lag + 2);
         if (count) S = std::min(std::max(S, (1024 + sh.tiles_a - 1) / sh.tiles_a), count[L]);
@@ -1186,7 +1264,7 @@ WsLayout ws_layout(const BatchPlan& P, const nttb_batch_config& cfg, const uint3
 // largest first; phase 1 holds the inverse units of products, which depend
 // on phase-0 units.  Every pass B tile deferred by the lag is flushed at the
 // phase boundary, so each awaited tile precedes its waiter in the queue.
-int plan_batch(const BatchPlan& P, const nttb_batch_job* jobs, uint32_t n_jobs, const nttb_batch_config& cfg,
+int plan_batch(BatchPlan& P, const nttb_batch_job* jobs, uint32_t n_jobs, const nttb_batch_config& cfg, Tiles kind,
                std::vector<BUnit>& units, std::vector<BTile>& tiles, const WsLayout* fixed, WsLayout* layout_out) {
     const uint32_t E = cfg.tile_elems;
     struct Pending {
@@ -1202,12 +1280,12 @@ int plan_batch(const BatchPlan& P, const nttb_batch_job* jobs, uint32_t n_jobs, 
                          const std::vector<uint32_t>* dep_a, const std::vector<uint32_t>* dep_b) -> int {
         const uint32_t n = 1u << L;
         UnitShape sh;
-        if (!unit_shape(P, cfg, L, &sh))
+        if (!unit_shape(cfg, kind, L, &sh))
             return fail(NTTB_ERR_INVALID_ARG, "batch job %u: log_n %u too large for tile %u", j, L, E);
         const uint32_t lg1 = sh.lg1, per = sh.per;
         const bool tcu = sh.tc;
-        if ((uf & UF_W64 || in) && !(tcu && lg1))
-            return fail(NTTB_ERR_UNSUPPORTED, "batch job %u: uint64 words or a separate source need tensor tiles", j);
+        if ((uf & UF_W64 || in) && !((tcu || sh.rx) && lg1))
+            return fail(NTTB_ERR_UNSUPPORTED, "batch job %u: uint64 words or a separate source need tensor or radix tiles", j);
         const size_t es = (uf & UF_W64) ? 8 : 4;  // bytes per residue of data and in
         uint32_t k = 0;
         for (uint32_t l0 = 0; l0 < n_limbs; l0 += per, k++) {
@@ -1218,13 +1296,23 @@ int plan_batch(const BatchPlan& P, const nttb_batch_job* jobs, uint32_t n_jobs, 
             u.pre_mul = pre_mul ? pre_mul + (size_t)l0 * n : nullptr;
             u.mod0 = first + l0;
             u.log_n = L;
-            u.flags = uf | (tcu ? UF_TC : 0u);
+            u.flags = uf | (tcu ? UF_TC : 0u) | (sh.rx ? UF_RX : 0u);
             u.lg1 = lg1;
             u.rows = lg1 ? 1u : std::min(per, n_limbs - l0);
             u.va = sh.va;
             u.vb = sh.vb;
             u.tiles_a = sh.tiles_a;
             u.tiles_b = sh.tiles_b;
+            if (sh.rx && lg1) {
+                const RxModulus& M = P.mods->rx_host[u.mod0];
+                const uint32_t nega = uf & UF_NEGA ? 1u : 0u, k = 2 * nega + (uf & UF_INV ? 1u : 0u);
+                u.ar = M.ar;
+                u.pairs = M.pairs[k];
+                u.quot = M.quot[k];
+                u.one = make_uint2(1u, (uint32_t)((1ull << 32) / M.ar.q));
+                u.scale[0] = M.scale[nega][pre_mul ? 1 : 0][L][0];
+                u.scale[1] = M.scale[nega][pre_mul ? 1 : 0][L][1];
+            }
             u.prev = -1;
             u.after[0] = u.after[1] = -1;
             p.work = (uint64_t)u.rows * n * L;
@@ -1276,17 +1364,23 @@ int plan_batch(const BatchPlan& P, const nttb_batch_job* jobs, uint32_t n_jobs, 
     }
     // phase by phase, largest units first
     std::stable_sort(list.begin(), list.end(), [](const Pending& x, const Pending& y) {
-        return x.phase != y.phase ? x.phase < y.phase : x.work > y.work;
+        if (x.phase != y.phase || x.work != y.work) return x.phase != y.phase ? x.phase < y.phase : x.work > y.work;
+        // radix units of one size: those that share a root table next to each other
+        return (x.u.flags & UF_RX) && x.u.lg1 && (y.u.flags & UF_RX) && x.u.quot < y.u.quot;
     });
     std::vector<int32_t> index_of(list.size());
     for (size_t i = 0; i < list.size(); i++) index_of[list[i].id] = (int32_t)i;
     uint32_t count[25] = {};
     for (const Pending& p : list)
         if (p.u.lg1) count[p.u.log_n]++;
-    const WsLayout lay = fixed ? *fixed : ws_layout(P, cfg, count);
+    const WsLayout lay = fixed ? *fixed : ws_layout(P, cfg, kind, count);
     for (uint32_t L = 1; L < 25; L++)
         if (count[L] && !lay.slots[L]) return fail(NTTB_ERR_INVALID_ARG, "batch: no workspace ring for log_n %u", L);
-    const uint32_t lag = cfg.lag;
+    // A unit's second pass follows its first by `lag` two-pass units; radix tiles
+    // are shorter than the time a CTA holds its next ticket, so there also by
+    // twice the tiles that the grid can hold, as far as the ring has slots
+    // (units of 2^14 are two tiles each: four of them would not fill the GPU).
+    const uint32_t lag = cfg.lag, lag_tiles = kind == Tiles::kRadix ? 2 * kRxCtas * 148 * 2 : 0;
     units.clear();
     tiles.clear();
     std::vector<std::vector<int32_t>> slot_owner(25);
@@ -1294,6 +1388,7 @@ int plan_batch(const BatchPlan& P, const nttb_batch_job* jobs, uint32_t n_jobs, 
     uint32_t next_slot[25] = {};
     uint32_t n_dis = 0;
     std::deque<uint32_t> pend_b;
+    std::vector<size_t> a_end;  // tiles emitted up to the end of each unit's first pass
     uint32_t phase = 0;
     auto emit_b = [&](uint32_t ui) {
         for (uint32_t t = 0; t < units[ui].tiles_b; t++) tiles.push_back({ui, 0x80000000u | t});
@@ -1327,6 +1422,12 @@ int plan_batch(const BatchPlan& P, const nttb_batch_job* jobs, uint32_t n_jobs, 
         }
         if (u.lg1) {
             const uint32_t L = u.log_n, slot = next_slot[L]++ % lay.slots[L];
+            // the slot's previous owner must be queued in full before this unit
+            while (slot_owner[L][slot] >= 0 &&
+                   std::find(pend_b.begin(), pend_b.end(), (uint32_t)slot_owner[L][slot]) != pend_b.end()) {
+                emit_b(pend_b.front());
+                pend_b.pop_front();
+            }
             // word offset, rebased on the workspace allocation later
             u.ws = reinterpret_cast<uint32_t*>((uintptr_t)((lay.base[L] + ((uint64_t)slot << L)) * 4u));
             u.prev = slot_owner[L][slot];
@@ -1335,9 +1436,10 @@ int plan_batch(const BatchPlan& P, const nttb_batch_job* jobs, uint32_t n_jobs, 
         }
         units.push_back(u);
         for (uint32_t t = 0; t < u.tiles_a; t++) tiles.push_back({ui, t});
+        a_end.push_back(tiles.size());
         if (u.lg1) {
             pend_b.push_back(ui);
-            while (pend_b.size() > lag) {
+            while (pend_b.size() > lag && tiles.size() - a_end[pend_b.front()] >= lag_tiles) {
                 emit_b(pend_b.front());
                 pend_b.pop_front();
             }
@@ -1359,21 +1461,157 @@ uint32_t discard_counters(const std::vector<BUnit>& units) {
     return n;
 }
 
-int create_batch(BatchPlan* P, const nttb_batch_job* jobs, uint32_t n_jobs, const nttb_batch_config& cfg, Batch** out) {
+// The tensor tiles' DFT images, made on first use: per modulus forward
+// (omega_64), inverse, and the negacyclic forward with psi_128^j on the input
+// index, then those of DFT-16 and DFT-8.
+bool ensure_images(BatchPlan& P) {
+    std::lock_guard<std::mutex> lock(P.mods->mu);
+    if (P.images) return true;
+    if (P.max_log < 13) return false;
+    const size_t per = kImgPerMod, nm = P.limbs.size();
+    const uint64_t N = 1ull << P.max_log;
+    std::vector<uint8_t> img(per * nm, 0);
+    for (size_t l = 0; l < nm; l++) {
+        const LimbHost& H = P.limbs[l];
+        const uint64_t q = H.q;
+        const uint64_t w64 = h_powmod(H.omega, N / 64, q), w64i = h_powmod(H.omega_inv, N / 64, q);
+        uint8_t* d = img.data() + per * l;
+        tc_build_image64(d, tc_dft_matrix(64, w64, q), q);
+        tc_build_image64(d + kImgBytes, tc_dft_matrix(64, w64i, q), q);
+        if (P.negacyclic)
+            tc_build_image64(d + 2 * kImgBytes, tc_dft_matrix(64, w64, q, 1, h_powmod(H.psi, N / 64, q)), q);
+        // DFT-16 and DFT-8 of level 2: forward, inverse, and the negacyclic
+        // inverse with psi_max^-(2^max_log k2 / r') on output k2
+        for (uint32_t r : {16u, 8u}) {
+            const uint64_t w = h_powmod(H.omega, N / r, q), wi = h_powmod(H.omega_inv, N / r, q);
+            uint8_t* o = d + (r == 16 ? kImg16Off : kImg8Off);
+            const uint32_t bytes = r == 16 ? 4096 : 1024;
+            auto build = r == 16 ? tc_build_image16 : build_image8;
+            build(o, tc_dft_matrix(r, w, q), q);
+            build(o + bytes, tc_dft_matrix(r, wi, q), q);
+            if (P.negacyclic) build(o + 2 * bytes, tc_dft_matrix(r, wi, q, h_powmod(H.psi_inv, N / r, q)), q);
+        }
+    }
+    uint8_t* d = nullptr;
+    if (cudaMalloc(&d, img.size()) != cudaSuccess ||
+        cudaMemcpy(d, img.data(), img.size(), cudaMemcpyHostToDevice) != cudaSuccess) {
+        cudaGetLastError();
+        if (d) cudaFree(d);
+        return false;
+    }
+    P.allocations.push_back(d);
+    P.images = d;
+    P.table_bytes += img.size();
+    return true;
+}
+
+// Device tables of the register-radix tiles for one kind of root (bit 0
+// inverse, bit 1 negacyclic), made on first use: per modulus 4 bytes per root
+// up to 2^min(max_log, 20) and 8 per root up to 2^10 (the uniform passes').
+bool ensure_roots(BatchPlan& P, uint32_t kind) {
+    BatchPlan::Mods& M = *P.mods;
+    std::lock_guard<std::mutex> lock(M.mu);
+    const size_t nm = P.limbs.size();
+    if (M.rx_host.empty()) {
+        M.rx_host.resize(nm);
+        for (size_t l = 0; l < nm; l++) {
+            const LimbHost& H = P.limbs[l];
+            const uint64_t q = H.q;
+            RxModulus& R = M.rx_host[l];
+            R = RxModulus{};
+            R.ar.q = (uint32_t)q;
+            R.ar.qinv = h_neg_inv32((uint32_t)q);
+            // the inverse's one root of its last stage: zeta_4^-1 (negacyclic) or 1
+            const uint64_t w0 = P.negacyclic ? h_powmod(H.psi_inv, (1ull << P.max_log) / 2, q) : 1;
+            for (uint32_t nega = 0; nega < 2; nega++)
+                for (uint32_t prod = 0; prod < 2; prod++) {
+                    uint64_t c = prod ? (1ull << 32) % q : 1;
+                    const uint64_t half = (q + 1) / 2;
+                    for (uint32_t L = 0; L < 25; L++, c = h_mulmod(c, half, q)) {
+                        const uint64_t v[2] = {c, nega ? h_mulmod(c, w0, q) : c};
+                        for (int i = 0; i < 2; i++)
+                            R.scale[nega][prod][L][i] = make_uint2((uint32_t)v[i], (uint32_t)((v[i] << 32) / q));
+                    }
+                }
+        }
+    }
+    if (M.rx_host[0].quot[kind]) return true;
+    const uint32_t log_r = std::min(P.max_log, kRxMaxLog), log_p = std::min(P.max_log, kRxMaxLog / 2);
+    uint2* pairs = nullptr;
+    uint32_t* quot = nullptr;
+    const size_t pair_bytes = (nm << log_p) * sizeof(uint2), quot_bytes = (nm << log_r) * sizeof(uint32_t);
+    bool ok = cudaMalloc(&pairs, pair_bytes) == cudaSuccess && cudaMalloc(&quot, quot_bytes) == cudaSuccess;
+    ok = ok && (M.rx || cudaMalloc(&M.rx, nm * sizeof(RxModulus)) == cudaSuccess);
+    if (ok) {
+        const dim3 grid(std::max(1u, std::min(64u, (1u << log_r) / 256u)), (unsigned)nm);
+        rx_roots_kernel<<<grid, 256>>>(M.d, P.max_log, log_r, log_p, kind, pairs, quot);
+        for (size_t l = 0; l < nm; l++) {
+            M.rx_host[l].pairs[kind] = pairs + (l << log_p);
+            M.rx_host[l].quot[kind] = quot + (l << log_r);
+        }
+        ok = cudaMemcpy(M.rx, M.rx_host.data(), nm * sizeof(RxModulus), cudaMemcpyHostToDevice) == cudaSuccess &&
+             cudaStreamSynchronize(0) == cudaSuccess;
+    }
+    if (!ok) {
+        cudaGetLastError();
+        for (RxModulus& R : M.rx_host) {
+            R.pairs[kind] = nullptr;
+            R.quot[kind] = nullptr;
+        }
+        cudaFree(pairs);
+        cudaFree(quot);
+        return false;
+    }
+    P.allocations.push_back(pairs);
+    P.allocations.push_back(quot);
+    P.table_bytes += pair_bytes + quot_bytes;
+    return true;
+}
+
+// The tiles a job list runs: with tensor set (and a 256-thread configuration)
+// the register-radix tiles if any unit is in their range and the tables fit in
+// memory, else the tensor tiles; the configured CUDA-core tiles otherwise.
+Tiles pick_tiles(BatchPlan& P, const nttb_batch_job* jobs, uint32_t n_jobs, const nttb_batch_config& cfg) {
+    if (!tensor_tiles(cfg)) return Tiles::kCore;
+    uint32_t kinds = 0;
+    for (uint32_t j = 0; j < n_jobs; j++) {
+        if (jobs[j].log_n < kRxMinLog || jobs[j].log_n > kRxMaxLog || jobs[j].log_n > P.max_log) continue;
+        if ((reinterpret_cast<uintptr_t>(jobs[j].data) | reinterpret_cast<uintptr_t>(jobs[j].pointwise)) & 15u) {
+            kinds = 0;  // the tiles copy 16 bytes at a time
+            break;
+        }
+        const uint32_t nega = (jobs[j].flags & NTTB_NEGACYCLIC) && P.negacyclic ? 2u : 0u;
+        if (jobs[j].flags & NTTB_BATCH_POLYMUL) kinds |= 3u << nega;
+        else kinds |= 1u << (nega + (jobs[j].flags & NTTB_BATCH_INVERSE ? 1u : 0u));
+    }
+    bool ok = kinds != 0;
+    for (uint32_t k = 0; k < 4 && ok; k++)
+        if (kinds >> k & 1u) ok = ensure_roots(P, k);
+    if (ok) return Tiles::kRadix;
+    return ensure_images(P) ? Tiles::kTensor : Tiles::kCore;
+}
+
+int create_batch(BatchPlan* P, const nttb_batch_job* jobs, uint32_t n_jobs, const nttb_batch_config& cfg, Batch** out,
+                 bool tensor_only = false) {
     if (int rc = check_config(cfg)) return rc;
+    const Tiles kind = tensor_only ? (ensure_images(*P) ? Tiles::kTensor : Tiles::kCore) : pick_tiles(*P, jobs, n_jobs, cfg);
     std::vector<BUnit> units;
     std::vector<BTile> tiles;
     WsLayout lay;
-    if (int rc = plan_batch(*P, jobs, n_jobs, cfg, units, tiles, nullptr, &lay)) return rc;
+    if (int rc = plan_batch(*P, jobs, n_jobs, cfg, kind, units, tiles, nullptr, &lay)) return rc;
     if (tiles.size() >= 0x7fffffffu || units.size() >= 0x7fffffffu)
         return fail(NTTB_ERR_INVALID_ARG, "batch: too many tiles");
     Batch* b = new Batch();
     b->plan = P;
     b->cfg = cfg;
     // without tensor-core units the CUDA-core kernel runs (more CTAs per SM)
-    bool any_tc = false;
-    for (const BUnit& u : units) any_tc = any_tc || (u.flags & UF_TC);
-    b->var = find_variant(cfg.tile_elems, cfg.threads, cfg.group, cfg.tensor && any_tc ? 1u : 0u);
+    bool any_tc = false, w64 = false;
+    for (const BUnit& u : units) {
+        any_tc = any_tc || (u.flags & UF_TC);
+        w64 = w64 || (u.flags & UF_W64);
+    }
+    b->var = kind == Tiles::kRadix ? (w64 ? &kRadixW64Variant : &kRadixVariant)
+                                   : find_variant(cfg.tile_elems, cfg.threads, cfg.group, cfg.tensor && any_tc ? 1u : 0u);
     b->n_units = (uint32_t)units.size();
     b->n_tiles = (uint32_t)tiles.size();
     b->n_dis = discard_counters(units);
@@ -1415,13 +1653,14 @@ int launch_batch(Batch* b, cudaStream_t s, bool count) {
     a.ws = b->d_ws;
     a.ws_words = b->ws_bytes / 4;
     a.n_dis = b->n_dis;
+    a.rx = b->plan->mods->rx;
     if (cudaMemsetAsync(b->d_ctr, 0, (1 + 2 * (size_t)b->n_units + b->n_dis) * 4, s) != cudaSuccess)
         return fail(NTTB_ERR_CUDA, "batch: counter reset failed");
     if (count) {
         ProfScope prof("batch_queue", s);
-        b->var->fn<<<b->grid, b->var->T, smem_bytes(b->var), s>>>(a);
+        b->var->fn<<<b->grid, cta_threads(b->var), smem_bytes(b->var), s>>>(a);
     } else {
-        b->var->fn<<<b->grid, b->var->T, smem_bytes(b->var), s>>>(a);
+        b->var->fn<<<b->grid, cta_threads(b->var), smem_bytes(b->var), s>>>(a);
     }
     return cudaGetLastError() == cudaSuccess ? 0 : fail(NTTB_ERR_CUDA, "batch: launch failed");
 }
@@ -1432,6 +1671,7 @@ int launch_batch(Batch* b, cudaStream_t s, bool count) {
 struct BatchRunner {
     BatchPlan* plan = nullptr;
     nttb_batch_config cfg{};
+    Tiles kind = Tiles::kCore;
     const Variant* var = nullptr;
     BUnit* d_units = nullptr;
     BTile* d_tiles = nullptr;
@@ -1479,13 +1719,24 @@ int runner_reserve(BatchRunner* r, size_t units, size_t tiles) {
 }
 }  // namespace
 
+// A runner's tiles: its job lists are all of the plan's twist, in both directions.
+static Tiles runner_tiles(BatchPlan* P, const nttb_batch_config& cfg) {
+    if (!tensor_tiles(cfg)) return Tiles::kCore;
+    if (P->max_log >= kRxMinLog && ensure_roots(*P, P->negacyclic ? 2 : 0) && ensure_roots(*P, P->negacyclic ? 3 : 1))
+        return Tiles::kRadix;
+    return ensure_images(*P) ? Tiles::kTensor : Tiles::kCore;
+}
+void batch_plan_prepare(BatchPlan* P, const nttb_batch_config& cfg) { runner_tiles(P, cfg); }
+
 int runner_create(BatchPlan* P, const nttb_batch_config& cfg, BatchRunner** out) {
     if (int rc = check_config(cfg)) return rc;
     auto* r = new BatchRunner();
     r->plan = P;
     r->cfg = cfg;
-    r->var = find_variant(cfg.tile_elems, cfg.threads, cfg.group, tensor_tiles(cfg) ? 1u : 0u);
-    r->layout = ws_layout(*P, cfg, nullptr);  // rings for every size class the plan allows
+    r->kind = runner_tiles(P, cfg);
+    r->var = r->kind == Tiles::kRadix ? &kRadixVariant
+                                      : find_variant(cfg.tile_elems, cfg.threads, cfg.group, r->kind == Tiles::kTensor);
+    r->layout = ws_layout(*P, cfg, r->kind, nullptr);  // rings for every size class the plan allows
     r->ws_bytes = (size_t)r->layout.words * 4;
     if ((r->ws_bytes && cudaMalloc(&r->d_ws, r->ws_bytes) != cudaSuccess) || runner_reserve(r, 256, 4096)) {
         runner_destroy(r);
@@ -1510,7 +1761,7 @@ size_t runner_device_bytes(const BatchRunner* r) {
 // Plans the jobs, uploads the queue from pinned staging and launches, all on
 // `s`.  One run per runner may be in flight: the staging is reused.
 int runner_run(BatchRunner* r, const nttb_batch_job* jobs, uint32_t n_jobs, cudaStream_t s) {
-    if (int rc = plan_batch(*r->plan, jobs, n_jobs, r->cfg, r->units, r->tiles, &r->layout, nullptr)) return rc;
+    if (int rc = plan_batch(*r->plan, jobs, n_jobs, r->cfg, r->kind, r->units, r->tiles, &r->layout, nullptr)) return rc;
     if (r->tiles.empty()) return 0;
     if (r->units.size() > r->cap_units || r->tiles.size() > r->cap_tiles) {
         cudaStreamSynchronize(s);  // the previous run may still read the queue
@@ -1534,6 +1785,7 @@ int runner_run(BatchRunner* r, const nttb_batch_job* jobs, uint32_t n_jobs, cuda
     a.ws = r->d_ws;
     a.ws_words = r->ws_bytes / 4;
     a.n_dis = discard_counters(r->units);
+    a.rx = r->plan->mods->rx;
     bool ok = cudaMemcpyAsync(r->d_units, r->h_units, r->units.size() * sizeof(BUnit), cudaMemcpyHostToDevice, s) ==
               cudaSuccess;
     ok = ok && cudaMemcpyAsync(r->d_tiles, r->h_tiles, r->tiles.size() * sizeof(BTile), cudaMemcpyHostToDevice, s) ==
@@ -1542,14 +1794,14 @@ int runner_run(BatchRunner* r, const nttb_batch_job* jobs, uint32_t n_jobs, cuda
     if (!ok) return fail(NTTB_ERR_CUDA, "batch runner: queue upload failed");
     const int grid = (int)std::min<size_t>((size_t)r->grid, r->tiles.size());
     ProfScope prof("batch_queue", s);
-    r->var->fn<<<grid, r->var->T, smem_bytes(r->var), s>>>(a);
+    r->var->fn<<<grid, cta_threads(r->var), smem_bytes(r->var), s>>>(a);
     return cudaGetLastError() == cudaSuccess ? 0 : fail(NTTB_ERR_CUDA, "batch runner: launch failed");
 }
 
 size_t batch_plan_device_bytes(const BatchPlan* P) {
     const uint32_t lo = std::min<uint32_t>(kLoBits, P->max_log);
     return (size_t)P->limbs.size() * 4 * 4 * (((size_t)1 << (P->max_log - lo)) + ((size_t)1 << lo)) +
-           P->limbs.size() * sizeof(BModulus) + (P->images ? P->limbs.size() * (size_t)kImgPerMod : 0);
+           P->limbs.size() * (sizeof(BModulus) + (P->mods->rx ? sizeof(RxModulus) : 0)) + P->table_bytes;
 }
 
 uint32_t batch_bounds_errors(bool clear) {
@@ -1589,7 +1841,7 @@ struct TileEntry {
     const void* src;
     void* dst;
     uint32_t n_polys;
-    bool inverse, u64;
+    bool inverse, u64, tensor;
     Batch* b;
     uint64_t used;
 };
@@ -1617,7 +1869,7 @@ TileCache* tile_cache(Plan32& p) {
 
 bool tiles_serve(const Plan32& p) { return p.log_n >= 13 && p.log_n <= 20; }
 
-int tiles_transform32(Plan32& p, const void* src, void* dst, bool u64, uint32_t n_polys, bool inverse,
+int tiles_transform32(Plan32& p, const void* src, void* dst, bool u64, uint32_t n_polys, bool inverse, bool tensor,
                       cudaStream_t s) {
     if (!tiles_serve(p)) return 1;
     TileCache* c = tile_cache(p);
@@ -1625,7 +1877,9 @@ int tiles_transform32(Plan32& p, const void* src, void* dst, bool u64, uint32_t 
     std::lock_guard<std::mutex> lock(c->mu);
     TileEntry* e = nullptr;
     for (TileEntry& t : c->entries)
-        if (t.src == src && t.dst == dst && t.n_polys == n_polys && t.inverse == inverse && t.u64 == u64) e = &t;
+        if (t.src == src && t.dst == dst && t.n_polys == n_polys && t.inverse == inverse && t.u64 == u64 &&
+            t.tensor == tensor)
+            e = &t;
     if (!e) {
         const size_t es = u64 ? 8 : 4, poly = (size_t)p.n_limbs << p.log_n;
         std::vector<nttb_batch_job> jobs(n_polys);
@@ -1645,7 +1899,7 @@ int tiles_transform32(Plan32& p, const void* src, void* dst, bool u64, uint32_t 
         nttb_batch_config cfg = default_config();
         cfg.tensor = 1;
         Batch* b = nullptr;
-        if (create_batch(&c->plan->p, jobs.data(), n_polys, cfg, &b)) return 2;
+        if (create_batch(&c->plan->p, jobs.data(), n_polys, cfg, &b, tensor)) return 2;
         if (c->entries.size() >= kTileQueues) {
             auto lru = std::min_element(c->entries.begin(), c->entries.end(),
                                         [](const TileEntry& x, const TileEntry& y) { return x.used < y.used; });
@@ -1653,7 +1907,7 @@ int tiles_transform32(Plan32& p, const void* src, void* dst, bool u64, uint32_t 
             free_batch(lru->b);
             c->entries.erase(lru);
         }
-        c->entries.push_back({src, dst, n_polys, inverse, u64, b, 0});
+        c->entries.push_back({src, dst, n_polys, inverse, u64, tensor, b, 0});
         e = &c->entries.back();
     }
     e->used = ++c->clock;
@@ -1762,45 +2016,6 @@ NTTB_API int nttb_batch_plan_create(const uint64_t* moduli, uint32_t n_moduli, u
         for (uint32_t L = 0; L < 25; L++) M.ninv[L] = nttb::h_to_mont32(nttb::h_invmod((1ull << L) % q, q), q);
         M.r2 = nttb::h_to_mont32(nttb::h_to_mont32(1, q), q);
     }
-    if (max_log_n >= 13) {
-        // DFT-64 images per modulus: forward (omega_64), inverse, and the
-        // negacyclic forward with psi_128^j on the input index
-        const size_t per = nttb::kImgPerMod;
-        std::vector<uint8_t> img(per * n_moduli, 0);
-        for (uint32_t l = 0; l < n_moduli; l++) {
-            const nttb::LimbHost& H = P.limbs[l];
-            const uint64_t q = H.q;
-            const uint64_t w64 = nttb::h_powmod(H.omega, N / 64, q), w64i = nttb::h_powmod(H.omega_inv, N / 64, q);
-            uint8_t* d = img.data() + per * l;
-            nttb::tc_build_image64(d, nttb::tc_dft_matrix(64, w64, q), q);
-            nttb::tc_build_image64(d + nttb::kImgBytes, nttb::tc_dft_matrix(64, w64i, q), q);
-            if (nega)
-                nttb::tc_build_image64(d + 2 * nttb::kImgBytes,
-                                       nttb::tc_dft_matrix(64, w64, q, 1, nttb::h_powmod(H.psi, N / 64, q)), q);
-            // DFT-16 and DFT-8 of level 2: forward, inverse, and the negacyclic
-            // inverse with psi_max^-(2^max_log k2 / r') on output k2
-            for (uint32_t r : {16u, 8u}) {
-                const uint64_t w = nttb::h_powmod(H.omega, N / r, q), wi = nttb::h_powmod(H.omega_inv, N / r, q);
-                uint8_t* o = d + (r == 16 ? nttb::kImg16Off : nttb::kImg8Off);
-                const uint32_t bytes = r == 16 ? 4096 : 1024;
-                auto build = r == 16 ? nttb::tc_build_image16 : nttb::build_image8;
-                build(o, nttb::tc_dft_matrix(r, w, q), q);
-                build(o + bytes, nttb::tc_dft_matrix(r, wi, q), q);
-                if (nega) build(o + 2 * bytes, nttb::tc_dft_matrix(r, wi, q, nttb::h_powmod(H.psi_inv, N / r, q)), q);
-            }
-        }
-        uint8_t* d = nullptr;
-        if (cudaMalloc(&d, img.size()) != cudaSuccess ||
-            cudaMemcpy(d, img.data(), img.size(), cudaMemcpyHostToDevice) != cudaSuccess) {
-            if (d) cudaFree(d);
-            for (void* a : P.allocations) cudaFree(a);
-            delete P.mods;
-            delete h;
-            return fail(NTTB_ERR_NO_MEMORY, "nttb_batch_plan_create: DFT-64 images");
-        }
-        P.allocations.push_back(d);
-        P.images = d;
-    }
     if (cudaMalloc(&P.mods->d, mods.size() * sizeof(nttb::BModulus)) != cudaSuccess ||
         cudaMemcpy(P.mods->d, mods.data(), mods.size() * sizeof(nttb::BModulus), cudaMemcpyHostToDevice) != cudaSuccess) {
         for (void* a : P.allocations) cudaFree(a);
@@ -1816,6 +2031,7 @@ NTTB_API int nttb_batch_plan_create(const uint64_t* moduli, uint32_t n_moduli, u
 NTTB_API int nttb_batch_plan_destroy(nttb_batch_plan* plan) {
     if (!plan) return NTTB_OK;
     for (void* a : plan->p.allocations) cudaFree(a);
+    if (plan->p.mods->rx) cudaFree(plan->p.mods->rx);
     delete plan->p.mods;
     delete plan;
     return NTTB_OK;
@@ -1959,7 +2175,8 @@ NTTB_API int nttb_batch_autotune(nttb_batch_plan* plan, const nttb_batch_job* jo
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
     float best = 1e30f;
-    nttb_batch_config best_cfg = nttb::default_config();
+    const nttb_batch_config c0 = nttb::default_config();
+    nttb_batch_config best_cfg = c0;
     int rc = 0;
     for (const auto& sh : shapes)
         for (uint32_t split = 0; split < 2; split++)
@@ -1970,7 +2187,8 @@ NTTB_API int nttb_batch_autotune(nttb_batch_plan* plan, const nttb_batch_job* jo
                     c.tile_elems = sh[0];
                     c.threads = sh[1];
                     c.tensor = sh[2];
-                    if (c.tensor && !plan->p.images) continue;
+                    // the radix tiles of a tensor configuration ignore tile, split and group
+                    if (c.tensor && (sh[0] != 4096 || split != c0.split || grp != c0.group)) continue;
                     c.split = split;
                     c.lag = lag;
                     c.group = grp;

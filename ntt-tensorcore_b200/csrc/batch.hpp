@@ -18,7 +18,8 @@ struct BatchPlan {
     bool negacyclic = false;
     std::vector<LimbHost> limbs;
     Mods* mods = nullptr;
-    uint8_t* images = nullptr;  // DFT-64 images of the tensor-core tiles (max_log >= 13), 3 x 64 KB per modulus
+    uint8_t* images = nullptr;  // DFT images of the tensor-core tiles (made on first use)
+    size_t table_bytes = 0;     // device bytes of the tables made on first use
     std::vector<void*> allocations;
     nttb_batch_config tuned{};
     bool have_tuned = false;
@@ -33,6 +34,8 @@ int runner_create(BatchPlan* plan, const nttb_batch_config& cfg, BatchRunner** o
 int runner_run(BatchRunner* r, const nttb_batch_job* jobs, uint32_t n_jobs, cudaStream_t s);
 void runner_destroy(BatchRunner* r);
 size_t runner_device_bytes(const BatchRunner* r);
+// Makes the tables that a runner of this configuration needs.
+void batch_plan_prepare(BatchPlan* plan, const nttb_batch_config& cfg);
 size_t batch_plan_device_bytes(const BatchPlan* plan);
 
 }  // namespace nttb

@@ -10,107 +10,69 @@
 //     second pass's tiles -- block k holds its columns V k .. V k + V - 1, row
 //     after row -- so that pass B reads one contiguous run of 32 KB per tile
 //     and pass A writes runs of at least 32 bytes times the lanes that share a row.
-// The passes whose roots are the same for every column read Shoup pairs (the
-// first 2^13 of a modulus); the row passes read the roots in Montgomery form, 4
-// bytes instead of 8 (they stream one root per residue, and a product costs
-// 10 instead of 8 cycles of the multiply pipe).  Tables are per modulus,
-// direction and twist, and one table serves every size: root 2^s + i is
-// zeta^(1 + 2 i), zeta of order 2^(s+2) (negacyclic), or zeta^i, zeta of order
-// 2^(s+1) (cyclic).
+// Roots.  Butterflies multiply by Shoup pairs (7.1 instructions, 12.4 per clock
+// and SM when nothing else runs; Montgomery-form roots take 9.1 and reach 8.7).
+// A pass whose roots are the same for every column reads pairs; a row pass and
+// whole rows, which use one root per residue, read the pair's quotient ws =
+// floor(w 2^32 / q) alone, 4 bytes, and make w = floor(ws q / 2^32) + 1 (ws q =
+// w 2^32 - r with 0 < r < q).  Tables are per modulus, direction and twist, and
+// one table serves every size: root 2^s + i is zeta^(1 + 2 i), zeta of order
+// 2^(s+2) (negacyclic), or zeta^i, zeta of order 2^(s+1) (cyclic).
 //
 // A seventeenth warp feeds the tiles: while the 512 threads run one, it claims
 // the next ticket, copies the tile's record to shared memory, waits (bounded)
-// for its dependencies and copies its words into an inbox (cp.async), so that a
-// tile starts on data that is there.  Words are copied 16 bytes at a time: a
+// for its dependencies and copies its roots and words into shared memory
+// (cp.async), so that a tile starts on data that is there.  Words are copied 16 bytes at a time: a
 // batch with a job off that alignment runs the other tiles.
 #pragma once
 
-constexpr uint32_t kRxThreads = 512, kRxTile = 8192, kRxLogTile = 13, kRxE = 4;
+constexpr uint32_t kRxLogTile = 13, kRxTile = 1u << kRxLogTile, kRxE = 4, kRxThreads = kRxTile >> kRxE;
+constexpr uint32_t kRxCtas = 2;  // per SM
 constexpr uint32_t kRxMinLog = 10, kRxMaxLog = 20;
+constexpr uint32_t kRxFew = kRxTile >> kRxE;  // words of a tile's roots outside the last round
 constexpr uint32_t rx_max(uint32_t a, uint32_t b) { return a > b ? a : b; }
 
-__device__ __forceinline__ void rx_sync() { asm volatile("bar.sync 1, 512;" ::: "memory"); }
+__device__ __forceinline__ void rx_sync() { asm volatile("bar.sync 1, %0;" ::"n"(kRxThreads) : "memory"); }
 
-// The tile's threads have read the roots: the feeding warp may refill them.
-__device__ __forceinline__ void rx_roots_free() { asm volatile("bar.arrive 7, 544;" ::: "memory"); }
+// The last round's roots (the stages with most of them) have their own
+// hand-over: ready (the tile waits), and read (the feeding warp may refill them).
+__device__ __forceinline__ void rx_roots_ready() { asm volatile("bar.sync 8, %0;" ::"n"(kRxThreads + 32) : "memory"); }
+__device__ __forceinline__ void rx_roots_free() { asm volatile("bar.arrive 7, %0;" ::"n"(kRxThreads + 32) : "memory"); }
 // The tile's threads have read the inbox: the feeding warp may refill it.
-__device__ __forceinline__ void rx_inbox_free() { asm volatile("bar.arrive 6, 544;" ::: "memory"); }
+__device__ __forceinline__ void rx_inbox_free() { asm volatile("bar.arrive 6, %0;" ::"n"(kRxThreads + 32) : "memory"); }
 
-// a b 2^-32 mod q in [0, 2q) for any a < 2^32 and b < q
-__device__ __forceinline__ uint32_t rx_mont(const M32& ar, uint32_t a, uint32_t b) {
-    return tca::mont_lazy(a, b, ar.q, ar.qinv);
+// The root at index i (within the pass) of a thread whose block and column
+// `box` points at: pairs, or quotients 2^LGV words apart.
+template <int LGV>
+__device__ __forceinline__ uint2 rx_root(const M32&, const uint2* box, uint32_t i) { return box[i]; }
+template <int LGV>
+__device__ __forceinline__ uint2 rx_root(const M32& ar, const uint32_t* box, uint32_t i) {
+    const uint32_t ws = box[i << LGV];
+    return make_uint2(__umulhi(ws, ar.q) + 1u, ws);
 }
-// Butterflies by a Montgomery-form root (radix.cuh's by a Shoup pair).
-__device__ __forceinline__ void ct(const M32& ar, uint32_t& a, uint32_t& b, uint32_t r) {
-    const uint32_t u = rdx::sub_if(a, ar.q), t = rdx::sub_if(rx_mont(ar, b, r), ar.q);
-    a = u + t;
-    b = u - t + ar.q;
-}
-__device__ __forceinline__ void gs(const M32& ar, uint32_t& a, uint32_t& b, uint32_t r) {
-    const uint32_t s = rdx::sub_if(a + b, ar.q), d = a - b + ar.q;
-    a = s;
-    b = rdx::sub_if(rx_mont(ar, d, r), ar.q);
-}
-using rdx::ct;
-using rdx::gs;
 
-__device__ __forceinline__ uint32_t rx_root(const uint32_t* p) {
-    uint32_t v;
-    asm volatile("ld.global.nc.u32 %0, [%1];" : "=r"(v) : "l"(p));
-    return v;
-}
-__device__ __forceinline__ uint2 rx_root(const uint2* p) { return rdx::ld_pair(p); }
-
-// Roots and stages of round I (rdx::round_roots / round_stages over either root form).
-template <int LG, int I, int S0, bool INV, class P>
-__device__ __forceinline__ void rx_roots(P (&w)[(1 << kRxE) - 1], const P* tw) {
+// Stages of round I from its J-th on (S0 > 0: none is the transform's first stage).
+template <int LG, int LGV, int I, int S0, bool INV, int JJ = 0, class P>
+__device__ __forceinline__ void rx_stages(const M32& ar, uint32_t (&x)[1 << kRxE], const P* box, uint2 c0, uint2 c1) {
     constexpr rdx::Rounds<LG, kRxE> R;
-    constexpr int r = R.r[I], S = S0 + R.s0[I];
+    constexpr int r = R.r[I], S = R.s0[I], xb = kRxE - r, j = INV ? r - 1 - JJ : JJ;
+    constexpr uint32_t half = 1u << (r - 1 - j);
+    constexpr bool scaled = INV && S0 + S + j == 0;
 #pragma unroll
-    for (int jj = 0; jj < r; jj++) {
-        const int j = INV ? r - 1 - jj : jj;
-        if (INV && S + j == 0) continue;
+    for (uint32_t kt = 0; kt < (1u << j); kt++) {
+        uint2 w = c1;
+        if constexpr (!scaled) w = rx_root<LGV>(ar, box, (1u << (S + j)) + (rdx::brv(kt, j) << S));
 #pragma unroll
-        for (uint32_t kt = 0; kt < (1u << j); kt++)
-            w[(1u << j) - 1u + kt] = rx_root(tw + (1u << (S + j)) + (rdx::brv(kt, j) << S));
+        for (uint32_t lo = 0; lo < half; lo++)
+#pragma unroll
+            for (uint32_t g = 0; g < (1u << xb); g++) {
+                const uint32_t ia = (((kt << (r - j)) + lo) << xb) + g, ib = ia + (half << xb);
+                if constexpr (scaled) rdx::gs_scaled(ar, x[ia], x[ib], c0, w);
+                else if constexpr (INV) rdx::gs(ar, x[ia], x[ib], w);
+                else rdx::ct(ar, x[ia], x[ib], w);
+            }
     }
-}
-// The same from the tile's roots in shared memory (row passes): entry e = 2^s +
-// i of the pass (s counted from its first stage) and column v at (e << LGV) + v;
-// `tw` points at the thread's block and column.
-template <int LG, int LGV, int I, bool INV>
-__device__ __forceinline__ void rx_row_roots(uint32_t (&w)[(1 << kRxE) - 1], const uint32_t* tw) {
-    constexpr rdx::Rounds<LG, kRxE> R;
-    constexpr int r = R.r[I], S = R.s0[I];
-#pragma unroll
-    for (int jj = 0; jj < r; jj++) {
-        const int j = INV ? r - 1 - jj : jj;
-#pragma unroll
-        for (uint32_t kt = 0; kt < (1u << j); kt++)
-            w[(1u << j) - 1u + kt] = tw[((1u << (S + j)) + (rdx::brv(kt, j) << S)) << LGV];
-    }
-}
-template <int LG, int I, int S0, bool INV, class P>
-__device__ __forceinline__ void rx_stages(const M32& ar, uint32_t (&x)[1 << kRxE], const P (&w)[(1 << kRxE) - 1],
-                                          uint2 c0, uint2 c1) {
-    constexpr rdx::Rounds<LG, kRxE> R;
-    constexpr int r = R.r[I], S = S0 + R.s0[I], xb = kRxE - r;
-#pragma unroll
-    for (int jj = 0; jj < r; jj++) {
-        const int j = INV ? r - 1 - jj : jj;
-        const uint32_t half = 1u << (r - 1 - j);
-#pragma unroll
-        for (uint32_t kt = 0; kt < (1u << j); kt++)
-#pragma unroll
-            for (uint32_t lo = 0; lo < half; lo++)
-#pragma unroll
-                for (uint32_t g = 0; g < (1u << xb); g++) {
-                    const uint32_t ia = (((kt << (r - j)) + lo) << xb) + g, ib = ia + (half << xb);
-                    if (INV && S + j == 0) rdx::gs_scaled(ar, x[ia], x[ib], c0, c1);
-                    else if (INV) gs(ar, x[ia], x[ib], w[(1u << j) - 1u + kt]);
-                    else ct(ar, x[ia], x[ib], w[(1u << j) - 1u + kt]);
-                }
-    }
+    if constexpr (JJ + 1 < r) rx_stages<LG, LGV, I, S0, INV, JJ + 1>(ar, x, box, c0, c1);
 }
 
 // Position lanes of a tile's blocked store (rows: all five lane bits).
@@ -119,17 +81,19 @@ constexpr int kRxTL = LB < LG - kRxE ? LB : LG - kRxE;
 template <int LG, int LGV, int LB>
 constexpr int kRxNP = LGV == 0 ? 5 : kRxTL<LG, LB> < 5 ? kRxTL<LG, LB> : 5;
 
-// What a tile reads and writes.  LSI, LSO: log2 of the words between a column's
-// elements in and out; LB >= 0: the output goes to the workspace in blocks of
-// 2^LB (the second pass's columns).  LBP: the LB that the placement is made for.
-// `rbox`: a row pass's roots in shared memory (rx_row_roots).
-// `in`: the tile in shared memory, element i of column v at (i << LGV) + v, or
-// null to read `src` (uint64 words).
-template <int LG, int LGV, bool INV, int S0, int LSI, int LSO, int LB, int LBP, class S, class D>
-__device__ __forceinline__ void rx_tile(const M32& ar, const uint32_t* in, const S* src, D* dst, const uint32_t* pre, const uint2* pairs,
-                                        const uint32_t* rbox, uint2 c0, uint2 c1, uint32_t col0, uint32_t tid,
+// One tile.  LSI, LSO: log2 of the words between a column's elements in and
+// out; LB >= 0: the output goes to the workspace in blocks of 2^LB (the second
+// pass's columns); LBP: the LB that the placement is made for.  S0: the pass's
+// first stage (above 0: a row pass).  In shared memory: `in`, element i of
+// column v at (i << LGV) + v (uint64 words are read from `src` instead), and
+// the roots: pairs, or (kQuot) quotients, root i of column v at (i << LGV) + v;
+// `box` those of the last round (in the forward order), `few` the others.
+template <int LG, int LGV, bool INV, int S0, bool kQuot, int LSI, int LSO, int LB, int LBP, class S, class D>
+__device__ __forceinline__ void rx_tile(const M32& ar, const uint32_t* in, const uint32_t* few,
+                                        const uint32_t* box, const S* src, D* dst,
+                                        const uint32_t* pre, uint2 one, uint2 c0, uint2 c1, uint32_t col0, uint32_t tid,
                                         uint32_t* sm, bool active, const uint32_t* drop) {
-    using P = typename std::conditional<(S0 > 0), uint32_t, uint2>::type;
+    using P = typename std::conditional<kQuot, uint32_t, uint2>::type;
     constexpr uint32_t NE = 1u << kRxE, V = 1u << LGV, NT = 1u << (LG - kRxE);
     constexpr rdx::Rounds<LG, kRxE> R;
     constexpr int NR = R.n;
@@ -139,23 +103,15 @@ __device__ __forceinline__ void rx_tile(const M32& ar, const uint32_t* in, const
     const uint32_t v_v = tid & (V - 1u), t_v = tid >> LGV;
     const uint32_t v_b = kBlock ? (tid >> TL) & (V - 1u) : v_v;
     const uint32_t t_b = kBlock ? (tid & ((1u << TL) - 1u)) | ((tid >> (TL + LGV)) << TL) : t_v;
-    P w[NE - 1];
     uint32_t x[NE];
-    auto roots = [&](auto step) {
-        constexpr int K = decltype(step)::value, I = INV ? NR - 1 - K : K;
-        constexpr bool blk = kBlock && K == NR - 1;
-        using Pl = rdx::Place<uint32_t, LG, LGV, kRxE, I, kRxNP<LG, LGV, LBP>>;
-        const uint32_t t = blk ? t_b : t_v;
-        if constexpr (S0 > 0) rx_row_roots<LG, LGV, I, INV>(w, rbox + (Pl::natural(t) << LGV) + (blk ? v_b : v_v));
-        else rx_roots<LG, I, 0, INV>(w, pairs + Pl::natural(t));
-        if constexpr (S0 > 0 && K == NR - 1) rx_roots_free();
-    };
     auto run = [&](auto self, auto step) -> void {
         constexpr int K = decltype(step)::value, I = INV ? NR - 1 - K : K;
         constexpr bool blk = kBlock && K == NR - 1;
         using Pl = rdx::Place<uint32_t, LG, LGV, kRxE, I, kRxNP<LG, LGV, LBP>>;
         const uint32_t t = blk ? t_b : t_v, v = blk ? v_b : v_v;
         uint32_t* base = sm + Pl::base(t) + v;
+        const P* roots = reinterpret_cast<const P*>(I == NR - 1 ? box : few) +
+                         (kQuot ? (Pl::natural(t) << LGV) + v : Pl::natural(t));
         if constexpr (K == 0) {
             // position t + rev(e) NT (inverse) or t + e NT: the parts share no bit, so
             // every address is a thread's base plus a constant
@@ -163,10 +119,8 @@ __device__ __forceinline__ void rx_tile(const M32& ar, const uint32_t* in, const
             const uint32_t* isrc = in + ((t << LGV) + v);
 #pragma unroll
             for (uint32_t e = 0; e < NE; e++) {
-                constexpr uint32_t kNT = NT;
-                const uint32_t ie = (INV ? rdx::brv(e, kRxE) : e) * kNT;
+                const uint32_t ie = (INV ? rdx::brv(e, kRxE) : e) * NT;
                 if constexpr (sizeof(S) == 8) {  // any word below 2^32: its residue
-                    const uint2 one = __ldg(pairs + 1);
                     const uint32_t y = (uint32_t)__ldcs(gsrc + ((size_t)ie << LSI));
                     x[e] = rdx::sub_if(y - __umulhi(y, one.y) * ar.q, ar.q);
                 } else {
@@ -178,41 +132,45 @@ __device__ __forceinline__ void rx_tile(const M32& ar, const uint32_t* in, const
                 const uint32_t* p = pre + (((size_t)t << LSI) + v);
 #pragma unroll
                 for (uint32_t e = 0; e < NE; e++)
-                    x[e] = rdx::sub_if(rx_mont(ar, x[e], __ldcg(p + ((size_t)(rdx::brv(e, kRxE) * NT) << LSI))), ar.q);
+                    x[e] = rdx::sub_if(tca::mont_lazy(x[e], __ldcg(p + ((size_t)(rdx::brv(e, kRxE) * NT) << LSI)), ar.q, ar.qinv),
+                                       ar.q);
             }
         } else {
             rdx::exchange<Pl, false>(base, x);
         }
-        rx_stages<LG, I, S0, INV>(ar, x, w, c0, c1);
+        if constexpr (I == NR - 1) rx_roots_ready();
+        rx_stages<LG, LGV, I, S0, INV>(ar, x, roots, c0, c1);
+        if constexpr (I == NR - 1) rx_roots_free();
         if constexpr (K < NR - 1) {
             rdx::exchange<Pl, true>(base, x);
-            roots(std::integral_constant<int, K + 1>{});
             rx_sync();
             // every load of the block has returned: drop its lines from the L2
             // (the slot's next owner rewrites them; otherwise they reach DRAM)
             if (K == 0 && drop && tid < kRxTile / 32)
                 asm volatile("discard.global.L2 [%0], 128;" ::"l"(drop + 32u * tid) : "memory");
             self(self, std::integral_constant<int, K + 1>{});
-        } else if constexpr (kBlock) {
-            const uint64_t keep = tc::l2_policy_evict_last();
-            auto at = [](uint32_t i) { return ((size_t)(i >> LB) << (LSI + LB)) + (i & ((1u << LB) - 1u)); };
-            D* p = dst + (at(t) + ((size_t)(col0 + v) << LB));
+        } else {
+            if constexpr (kBlock) {
+                const uint64_t keep = tc::l2_policy_evict_last();
+                auto at = [](uint32_t i) { return ((size_t)(i >> LB) << (LSI + LB)) + (i & ((1u << LB) - 1u)); };
+                D* p = dst + (at(t) + ((size_t)(col0 + v) << LB));
 #pragma unroll
-            for (uint32_t e = 0; e < NE; e++) st_keep(p + at((INV ? e : rdx::brv(e, kRxE)) * NT), x[e], keep);
-        } else if (active) {
-            D* p = dst + (((size_t)t << LSO) + v);
+                for (uint32_t e = 0; e < NE; e++) st_keep(p + at((INV ? e : rdx::brv(e, kRxE)) * NT), x[e], keep);
+            } else if (active) {
+                D* p = dst + (((size_t)t << LSO) + v);
 #pragma unroll
-            for (uint32_t e = 0; e < NE; e++)
-                __stcs(p + ((size_t)((INV ? e : rdx::brv(e, kRxE)) * NT) << LSO), (D)rdx::canon_out<INV>(ar, x[e]));
+                for (uint32_t e = 0; e < NE; e++)
+                    __stcs(p + ((size_t)((INV ? e : rdx::brv(e, kRxE)) * NT) << LSO), (D)rdx::canon_out<INV>(ar, x[e]));
+            }
         }
     };
-    roots(std::integral_constant<int, 0>{});
     run(run, std::integral_constant<int, 0>{});
 }
 
 // One pass of a two-pass unit of 2^L residues.
 template <int L, bool INV, int PASS, bool W64>
-__device__ __noinline__ void rx_pass(const BUnit& u, uint32_t tile, uint32_t* sm, const uint32_t* in) {
+__device__ __forceinline__ void rx_pass(const BUnit& u, uint32_t tile, uint32_t* sm, const uint32_t* in,
+                                        const uint32_t* few) {
     constexpr int LA = (L + 1) / 2, LBB = L / 2;  // points of the uniform and of the row pass
     constexpr bool kRow = INV ? PASS == 0 : PASS == 1;
     constexpr int LG = kRow ? LBB : LA, LGV = kRxLogTile - LG, S0 = kRow ? LA : 0;
@@ -221,22 +179,24 @@ __device__ __noinline__ void rx_pass(const BUnit& u, uint32_t tile, uint32_t* sm
     using W = typename std::conditional<W64, uint64_t, uint32_t>::type;
     const M32 ar = u.ar;
     const uint32_t col0 = tile << LGV;
+    const uint32_t* box = in + kRxTile;
     if constexpr (PASS == 0) {
         const W* src = static_cast<const W*>(u.in ? u.in : u.data) + col0;
-        rx_tile<LG, LGV, INV, S0, LC, 0, LB, LB, W, uint32_t>(ar, in, src, u.ws, INV && u.pre_mul ? u.pre_mul + col0 : nullptr,
-                                                          u.pairs, in + kRxTile, u.scale[0], u.scale[1], col0, threadIdx.x,
-                                                              sm, true, nullptr);
+        rx_tile<LG, LGV, INV, S0, kRow, LC, 0, LB, LB, W, uint32_t>(
+            ar, in, few, box, src, u.ws, INV && u.pre_mul ? u.pre_mul + col0 : nullptr, u.one, u.scale[0], u.scale[1], col0,
+            threadIdx.x, sm, true, nullptr);
     } else {
         const uint32_t* src = u.ws + (size_t)tile * kRxTile;
-        rx_tile<LG, LGV, INV, S0, LGV, LC, -1, LB, uint32_t, W>(ar, in, src, reinterpret_cast<W*>(u.data) + col0, nullptr, u.pairs,
-                                                                in + kRxTile, u.scale[0], u.scale[1], col0, threadIdx.x,
-                                                                sm, true, src);
+        rx_tile<LG, LGV, INV, S0, kRow, LGV, LC, -1, LB, uint32_t, W>(
+            ar, in, few, box, src, reinterpret_cast<W*>(u.data) + col0, nullptr, u.one, u.scale[0], u.scale[1], col0, threadIdx.x,
+            sm, true, src);
     }
 }
 
 // Whole rows of 2^L residues, one limb each.
 template <int L, bool INV>
-__device__ __noinline__ void rx_rows(const BArgs& a, const BUnit& u, uint32_t* sm, const uint32_t* in) {
+__device__ __forceinline__ void rx_rows(const BArgs& a, const BUnit& u, uint32_t* sm, const uint32_t* in,
+                                        const uint32_t* few) {
     constexpr uint32_t NT = 1u << (L - kRxE);
     constexpr rdx::Lay<L, 0, 5, 5> Y;
     const uint32_t tid = threadIdx.x & (NT - 1u);
@@ -246,7 +206,6 @@ __device__ __noinline__ void rx_rows(const BArgs& a, const BUnit& u, uint32_t* s
     if (!active) row = u.rows - 1u;
     const RxModulus& M = a.rx[u.mod0 + row];
     const M32 ar = M.ar;
-    const uint32_t kind = (u.flags & UF_NEGA ? 2u : 0u) + (INV ? 1u : 0u);
     uint2 c0 = make_uint2(0, 0), c1 = c0;
     if (INV) {
         const uint2* sc = M.scale[u.flags & UF_NEGA ? 1 : 0][u.pre_mul ? 1 : 0][L];
@@ -254,8 +213,9 @@ __device__ __noinline__ void rx_rows(const BArgs& a, const BUnit& u, uint32_t* s
         c1 = __ldg(sc + 1);
     }
     uint32_t* x = u.data + ((size_t)row << L);
-    rx_tile<L, 0, INV, 0, 0, 0, -1, 0, uint32_t, uint32_t>(ar, in + (row << L), x, x, INV && u.pre_mul ? u.pre_mul + ((size_t)row << L) : nullptr,
-                                                        M.pairs[kind], nullptr, c0, c1, 0, tid, sm, active, nullptr);
+    rx_tile<L, 0, INV, 0, true, 0, 0, -1, 0, uint32_t, uint32_t>(
+        ar, in + (row << L), few + (row << (L - kRxE)), in + kRxTile + (row << L), x, x, INV && u.pre_mul ? u.pre_mul + ((size_t)row << L) : nullptr,
+        make_uint2(0, 0), c0, c1, 0, tid, sm, active, nullptr);
 }
 
 struct RxSlot {
@@ -263,22 +223,28 @@ struct RxSlot {
     uint32_t unit, pass, tile, stop;
 };
 
-// The feeding warp: `chunks` 16-byte pieces (a multiple of 32), 2^lgc <= 32 of
-// them per row, rows `pitch` words apart, to shared memory past L1 (asynchronous).
-// A lane keeps its place in the row: one addition per copy, since this one warp
-// shares the issue slots with the tiles' thirty-two.
+// The feeding warp: `chunks` 16-byte pieces, 2^lgc <= 32 of them per row, rows
+// `pitch` words apart, to shared memory past L1 (asynchronous).  A lane keeps
+// its place in the row: one addition per copy, since this one warp shares the
+// issue slots with the tiles' thirty-two.
 __device__ __forceinline__ void rx_copy(const uint32_t* src, uint32_t lgc, size_t pitch, uint32_t chunks, uint32_t to,
                                         uint32_t lane) {
     const char* g = reinterpret_cast<const char*>(src + (size_t)(lane >> lgc) * pitch + 4 * (lane & ((1u << lgc) - 1u)));
     const size_t step = (pitch << (5 - lgc)) * 4;
     to += 16 * lane;
-    for (uint32_t k = 0; k < chunks / 32; k += 8) {
+    uint32_t i = 0;
+    for (; i + 256 <= chunks; i += 256) {
 #pragma unroll
-        for (uint32_t i = 0; i < 8; i++) {
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to + 512 * i), "l"(g) : "memory");
+        for (uint32_t k = 0; k < 8; k++) {
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to + 512 * k), "l"(g) : "memory");
             g += step;
         }
         to += 4096;
+    }
+    for (i += lane; i < chunks; i += 32) {
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to), "l"(g) : "memory");
+        g += step;
+        to += 512;
     }
 }
 
@@ -303,31 +269,46 @@ __device__ __forceinline__ void rx_fetch(const BUnit& u, uint32_t pass, uint32_t
     rx_copy(src, lgc, pitch, chunks, inbox, lane);
 }
 
-// A row pass's roots behind the inbox: columns V tile .. of the unit's root
-// table seen as [2^LG][2^LA] (entry (e << LA) + u is root e of row u).
-__device__ __forceinline__ void rx_fetch_roots(const BUnit& u, uint32_t tile, uint32_t inbox, uint32_t lane) {
-    const uint32_t L = u.log_n, la = (L + 1) / 2, lgv = kRxLogTile - L / 2;
-    rx_copy(u.mont + ((size_t)tile << lgv), lgv - 2, (size_t)1 << la, kRxTile / 4, inbox + 4 * kRxTile, lane);
+// A tile's roots.  A row pass: columns V tile .. of the unit's quotients seen as
+// [2^LG][2^LA] (entry (e << LA) + u is root e of row u); a uniform pass: its 2^LG
+// pairs; whole rows: each row's 2^L quotients.  FEW: the entries below 1/16 (every
+// round but the last); else all of them.
+template <bool FEW>
+__device__ __forceinline__ void rx_fetch_roots(const BArgs& a, const BUnit& u, uint32_t pass, uint32_t tile, uint32_t to,
+                                               uint32_t lane) {
+    const uint32_t L = u.log_n, la = (L + 1) / 2;
+    constexpr int kF = FEW ? kRxE : 0;
+    if (!u.lg1) {
+        const uint32_t kind = (u.flags & UF_NEGA ? 2u : 0u) + (u.flags & UF_INV ? 1u : 0u);
+        for (uint32_t r = 0; r < u.rows; r++)  // 4 quotients per piece
+            rx_copy(a.rx[u.mod0 + r].quot[kind], 5, 128, 1u << (L - 2 - kF), to + ((4 * r) << (L - kF)), lane);
+    } else if ((pass == 1) == !(u.flags & UF_INV)) {
+        const uint32_t lgv = kRxLogTile - L / 2;
+        rx_copy(u.quot + ((size_t)tile << lgv), lgv - 2, (size_t)1 << la, kRxTile >> (2 + kF), to, lane);
+    } else {
+        rx_copy(reinterpret_cast<const uint32_t*>(u.pairs), 5, 128, 1u << (la - 1 - kF), to, lane);  // 2 pairs per piece
+    }
 }
 
 template <bool W64>
-__device__ __forceinline__ void rx_dispatch(const BArgs& a, const RxSlot& s, uint32_t* sm, const uint32_t* in, M32* s_ar) {
+__device__ __forceinline__ void rx_dispatch(const BArgs& a, const RxSlot& s, uint32_t* sm, const uint32_t* in,
+                                            const uint32_t* few, M32* s_ar) {
     const BUnit& u = s.u;
     const bool inv = u.flags & UF_INV;
 #define NTTB_RX_TWO(l)                                                             \
     case l:                                                                        \
         if (s.pass == 0) {                                                         \
-            if (inv) rx_pass<l, true, 0, W64>(u, s.tile, sm, in);                      \
-            else rx_pass<l, false, 0, W64>(u, s.tile, sm, in);                         \
+            if (inv) rx_pass<l, true, 0, W64>(u, s.tile, sm, in, few);                      \
+            else rx_pass<l, false, 0, W64>(u, s.tile, sm, in, few);                         \
         } else {                                                                   \
-            if (inv) rx_pass<l, true, 1, W64>(u, s.tile, sm, in);                      \
-            else rx_pass<l, false, 1, W64>(u, s.tile, sm, in);                         \
+            if (inv) rx_pass<l, true, 1, W64>(u, s.tile, sm, in, few);                      \
+            else rx_pass<l, false, 1, W64>(u, s.tile, sm, in, few);                         \
         }                                                                          \
         return;
 #define NTTB_RX_ROWS(l)                        \
     case l:                                    \
-        if (inv) rx_rows<l, true>(a, u, sm, in); \
-        else rx_rows<l, false>(a, u, sm, in); \
+        if (inv) rx_rows<l, true>(a, u, sm, in, few); \
+        else rx_rows<l, false>(a, u, sm, in, few); \
         return;
     if constexpr (W64) {
         switch (u.log_n) {
@@ -351,26 +332,27 @@ __device__ __forceinline__ void rx_dispatch(const BArgs& a, const RxSlot& s, uin
 
 // Two CTAs of 16 + 1 warps per SM.
 template <bool W64>
-__global__ void __launch_bounds__(kRxThreads + 32, 2) batch_queue_radix(const __grid_constant__ BArgs a) {
+__global__ void __launch_bounds__(kRxThreads + 32, kRxCtas) batch_queue_radix(const __grid_constant__ BArgs a) {
     extern __shared__ __align__(16) uint32_t rx_sm[];
     __shared__ __align__(16) RxSlot slot[2];
     __shared__ M32 s_ar[kMaxRows];
     static_assert(sizeof(BUnit) % 16 == 0 && sizeof(BUnit) / 16 <= 32, "one 16-byte piece per lane");
-    uint32_t* inbox = rx_sm;                // the next tile's words, 32 KB, and a row pass's roots, 32 KB
-    uint32_t* work = rx_sm + 2 * kRxTile;   // the running tile's exchanges
+    uint32_t* inbox = rx_sm;                 // the next tile's words, 32 KB, and its last round's roots, 32 KB
+    uint32_t* few = rx_sm + 2 * kRxTile;     // the other roots, 2 KB for each slot
+    uint32_t* work = few + 2 * kRxFew;       // the running tile's exchanges
     // named barriers: 1 the tile's threads, 2 + s slot s filled, 4 + s slot s
-    // free, 6 the inbox free (uint64 words are read by the tile itself), 7
-    // the roots free
+    // free, 6 the inbox free (uint64 words are read by the tile itself), 7 the
+    // last round's roots free, 8 filled
     if (threadIdx.x >= kRxThreads) {
         const uint32_t lane = threadIdx.x & 31u;
         bool inbox_used = false, roots_used = false;  // a tile that reads them precedes
         for (uint32_t k = 0;; k++) {
             const uint32_t s = k & 1u;
-            if (k >= 2) asm volatile("bar.sync %0, 544;" ::"r"(4u + s) : "memory");
+            if (k >= 2) asm volatile("bar.sync %0, %1;" ::"r"(4u + s), "n"(kRxThreads + 32) : "memory");
             uint32_t ticket = 0;
             if (lane == 0) ticket = atomicAdd(a.ctr, 1u);
             ticket = __shfl_sync(~0u, ticket, 0);
-            bool stop = ticket >= a.n_tiles;
+            bool stop = ticket >= a.n_tiles, rx = false;
             if (!stop) {
                 const BTile tl = a.tiles[ticket];
 #if NTTB_DEBUG_BOUNDS
@@ -388,15 +370,12 @@ __global__ void __launch_bounds__(kRxThreads + 32, 2) batch_queue_radix(const __
                     __syncwarp();
                     const BUnit& u = slot[s].u;
                     const uint32_t pass = tl.pass_tile >> 31, tile = tl.pass_tile & 0x7fffffffu;
-                    if ((u.flags & UF_RX) && u.lg1 && (pass == 1) == !(u.flags & UF_INV)) {  // a row pass
-                        if (roots_used) asm volatile("bar.sync 7, 544;" ::: "memory");
-                        roots_used = true;
-                        rx_fetch_roots(u, tile, tc::smem_u32(inbox), lane);
-                    }
+                    rx = u.flags & UF_RX;
+                    if (rx) rx_fetch_roots<true>(a, u, pass, tile, tc::smem_u32(few + s * kRxFew), lane);
                     if (lane == 0 && !wait_deps(a, u, tl.unit, pass)) atomicOr(&g_batch_error, 1u);
                     __syncwarp();
-                    if (!(W64 && pass == 0) && (u.flags & UF_RX)) {
-                        if (inbox_used) asm volatile("bar.sync 6, 544;" ::: "memory");
+                    if (rx && !(W64 && pass == 0)) {
+                        if (inbox_used) asm volatile("bar.sync 6, %0;" ::"n"(kRxThreads + 32) : "memory");
                         inbox_used = true;
                         rx_fetch(u, pass, tile, tc::smem_u32(inbox), lane);
                     }
@@ -405,18 +384,25 @@ __global__ void __launch_bounds__(kRxThreads + 32, 2) batch_queue_radix(const __
             }
             if (lane == 0) slot[s].stop = stop;
             __syncwarp();
-            asm volatile("bar.arrive %0, 544;" ::"r"(2u + s) : "memory");
+            asm volatile("bar.arrive %0, %1;" ::"r"(2u + s), "n"(kRxThreads + 32) : "memory");
             if (stop) return;
+            if (rx) {  // the roots of the running tile's last round are in use until then
+                if (roots_used) asm volatile("bar.sync 7, %0;" ::"n"(kRxThreads + 32) : "memory");
+                roots_used = true;
+                rx_fetch_roots<false>(a, slot[s].u, slot[s].pass, slot[s].tile, tc::smem_u32(inbox + kRxTile), lane);
+                asm volatile("cp.async.wait_all;" ::: "memory");
+                asm volatile("bar.arrive 8, %0;" ::"n"(kRxThreads + 32) : "memory");
+            }
         }
     }
     for (uint32_t k = 0;; k++) {
         const uint32_t s = k & 1u;
-        asm volatile("bar.sync %0, 544;" ::"r"(2u + s) : "memory");
+        asm volatile("bar.sync %0, %1;" ::"r"(2u + s), "n"(kRxThreads + 32) : "memory");
         if (slot[s].stop) return;
-        rx_dispatch<W64>(a, slot[s], work, inbox, s_ar);
+        rx_dispatch<W64>(a, slot[s], work, inbox, few + s * kRxFew, s_ar);
         rx_sync();
         if (threadIdx.x == 0) signal_done(a.ctr + 1 + 2 * slot[s].unit + slot[s].pass);
-        asm volatile("bar.arrive %0, 544;" ::"r"(4u + s) : "memory");
+        asm volatile("bar.arrive %0, %1;" ::"r"(4u + s), "n"(kRxThreads + 32) : "memory");
     }
 }
 
@@ -434,6 +420,6 @@ constexpr uint32_t kRxWork = rx_max(
     rx_max(rx_max(rx_two_words<14>(), rx_two_words<15>()), rx_max(rx_two_words<16>(), rx_two_words<17>())),
     rx_max(rx_max(rx_max(rx_two_words<18>(), rx_two_words<19>()), rx_two_words<20>()),
            rx_max(rx_max(rx_rows_words<10>(), rx_rows_words<11>()), rx_max(rx_rows_words<12>(), rx_rows_words<13>()))));
-constexpr uint32_t kRxWords = 2 * kRxTile + kRxWork;
+constexpr uint32_t kRxWords = 2 * kRxTile + 2 * kRxFew + kRxWork;
 // units of other sizes run CUDA-core tiles of this many residues in the exchange buffer
 constexpr uint32_t kRxCoreTile = 4096;

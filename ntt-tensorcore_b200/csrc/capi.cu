@@ -636,8 +636,8 @@ int nttb_rns_forward_inverse(const nttb_rns_plan* P, uint32_t* d, uint32_t n_pol
     if (eng == NTTB_ENGINE_INT8) {
         rc = int8_forward_inverse32(p, d, n_polys, s);
     } else {
-        rc = run_transform32(p, d, d, false, n_polys, false, eng, s);
-        if (!rc) rc = run_transform32(p, d, d, false, n_polys, true, eng, s);
+        rc = run_transform32(p, d, d, false, n_polys, false, engine, s);
+        if (!rc) rc = run_transform32(p, d, d, false, n_polys, true, engine, s);
     }
     return engine_status(rc, "rns_forward_inverse");
 }
@@ -701,11 +701,11 @@ int nttb_rns_stream_host(nttb_rns_plan* P, const uint32_t* h_src, uint32_t* h_ds
         int rc = 0;
         if (mode == 2) {
             rc = eng == NTTB_ENGINE_INT8 ? int8_forward_inverse32(p, H->dbuf[k], n_polys, s)
-                                         : run_transform32(p, H->dbuf[k], H->dbuf[k], false, n_polys, false, eng, s);
+                                         : run_transform32(p, H->dbuf[k], H->dbuf[k], false, n_polys, false, engine, s);
             if (!rc && eng != NTTB_ENGINE_INT8)
-                rc = run_transform32(p, H->dbuf[k], H->dbuf[k], false, n_polys, true, eng, s);
+                rc = run_transform32(p, H->dbuf[k], H->dbuf[k], false, n_polys, true, engine, s);
         } else {
-            rc = run_transform32(p, H->dbuf[k], H->dbuf[k], false, n_polys, mode == 1, eng, s);
+            rc = run_transform32(p, H->dbuf[k], H->dbuf[k], false, n_polys, mode == 1, engine, s);
         }
         if (rc) return engine_status(rc, "rns_stream_host");
         cudaEventRecord(H->ev_c[k], s);

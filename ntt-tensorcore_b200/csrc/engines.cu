@@ -19,13 +19,13 @@ static int env_engine() {
 
 // Out of place, the CUDA-core engine's register-radix passes (radix.cuh) are
 // the fastest at every size (us, forward, this engine / the other): 8 x 2^16
-// 6.9 / 16.6 (INT8), 24 x 2^16 9.7 / 17.4 (INT8), 192 x 2^16 57 / 95 (INT8),
-// 33 x 2^17 22.8 / 62 (tiles), 1 x 2^20 10 / 25 (tiles).  In place they stage
-// their first pass in the plan's workspace, which ties the plan's calls to one
-// stream; the sizes and counts below keep an engine that does not:
-// the INT8 cluster kernel at 2^16 from kInt8MinUnits (polynomial, limb) units
-// on, and the batch queue's tensor tiles at 2^17 .. 2^20 once a call holds
-// 2^20 residues (each prepared queue has a ring of its own).
+// 6.6 / 16.6 (INT8), 24 x 2^16 9.7 / 17.4 (INT8), 192 x 2^16 54 / 95 (INT8),
+// 33 x 2^17 22.5 / 62 (tensor tiles), 1 x 2^20 10 / 25 (queue).  In place they
+// stage their first pass in the plan's workspace, which ties the plan's calls
+// to one stream; the sizes and counts below keep an engine that does not: the
+// INT8 cluster kernel at 2^16 from kInt8MinUnits (polynomial, limb) units on,
+// and the batch queue at 2^17 .. 2^20 once a call holds 2^20 residues (each
+// prepared queue has a ring of its own).
 constexpr uint64_t kInt8MinUnits = 8;
 constexpr uint32_t kTilesMinLog = 17;
 constexpr uint64_t kTilesMinResidues = 1ull << 20;
@@ -40,7 +40,8 @@ int auto_engine32(const Plan32& p, bool src_u64, uint64_t units, bool in_place) 
 int run_transform32(Plan32& p, const void* src, void* dst, bool src_u64, uint32_t n_polys, bool inverse,
                     int engine, cudaStream_t s) {
     if (engine == NTTB_ENGINE_AUTO) engine = env_engine();
-    if (engine == NTTB_ENGINE_AUTO) engine = auto_engine32(p, src_u64, (uint64_t)n_polys * p.n_limbs, src == dst);
+    const bool named = engine != NTTB_ENGINE_AUTO;
+    if (!named) engine = auto_engine32(p, src_u64, (uint64_t)n_polys * p.n_limbs, src == dst);
     switch (engine) {
         case NTTB_ENGINE_SCALAR:
             return scalar_transform32(p, src, dst, src_u64, n_polys, inverse, s);
@@ -49,7 +50,7 @@ int run_transform32(Plan32& p, const void* src, void* dst, bool src_u64, uint32_
         case NTTB_ENGINE_DMMA:
             return dmma_transform32(p, src, dst, src_u64, n_polys, inverse, s);
         case NTTB_ENGINE_TILES:
-            return tiles_transform32(p, src, dst, src_u64, n_polys, inverse, s);
+            return tiles_transform32(p, src, dst, src_u64, n_polys, inverse, named, s);
         default:
             return 1;
     }

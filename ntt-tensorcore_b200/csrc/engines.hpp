@@ -22,7 +22,9 @@ void engines_release32(Plan32* p);
 
 // The batch queue's tensor tiles as a plan engine (batch.cu): 2^13 .. 2^20.
 bool tiles_serve(const Plan32& p);
-int tiles_transform32(Plan32& p, const void* src, void* dst, bool u64, uint32_t n_polys, bool inverse, cudaStream_t s);
+// `tensor`: on the tensor tiles (the engine named), else on the queue's fastest tiles.
+int tiles_transform32(Plan32& p, const void* src, void* dst, bool u64, uint32_t n_polys, bool inverse, bool tensor,
+                      cudaStream_t s);
 void tiles_release(Plan32* p);
 
 int fail(int code, const char* fmt, ...);

@@ -235,6 +235,7 @@ NTTB_API int nttb_server_create(const uint64_t* moduli, uint32_t n_moduli, const
         delete s;
         return rc;
     }
+    nttb::batch_plan_prepare(&s->plan->p, cfg->batch);
     s->resident = nttb::batch_plan_device_bytes(&s->plan->p);
     s->slots.resize(cfg->slots);
     for (nttb::Slot& sl : s->slots) {
