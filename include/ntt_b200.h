@@ -39,13 +39,17 @@ enum {
     NTTB_ERR_BUDGET = 6       /* serving admission refused: HBM budget exceeded */
 };
 
-/* Inner-DFT engines.  AUTO picks one that serves the request: out of place the
- * CUDA-core engine; in place the INT8 tensor-core kernel at N = 2^16 from 8
- * (polynomial, limb) units on, the batch queue at N = 2^17 ..
- * 2^20 once a call holds 2^20 residues, the CUDA-core engine otherwise (it
- * stages its first pass in the plan's workspace).  The tiles engine keeps up
- * to eight prepared queues per plan (one per source, destination, count,
- * direction), each with its own workspace ring of up to 16 x N words. */
+/* Inner-DFT engines.  AUTO takes the CUDA-core engine for RNS plans and wide
+ * plans.  Its in-place calls above 2^13 stage a pass in a workspace of the plan's
+ * (one for each of the first four streams, then one per call, in stream order:
+ * streams and threads may share a plan).  Where that memory cannot be had, while
+ * the stream is captured, and for the drop-in's uint64 words and the host stream,
+ * AUTO takes the INT8 tensor-core kernel at N = 2^16 from 8 (polynomial, limb)
+ * units on, the batch queue at N = 2^17 .. 2^20 once a call holds 2^20 residues,
+ * the CUDA-core engine otherwise (captured in place, it stages in the plan's own
+ * buffer: order those calls).  The queue route keeps up to eight prepared queues
+ * per plan (one per source, destination, count, direction), each with its own
+ * workspace ring of up to 16 x N words. */
 enum {
     NTTB_ENGINE_AUTO = 0,
     NTTB_ENGINE_SCALAR = 1, /* CUDA-core radix-2 stages in registers and shared memory */
@@ -188,8 +192,9 @@ NTTB_API int nttb_rns_transform(const nttb_rns_plan* plan, uint32_t* d_dst, cons
                        int inverse, int engine, void* stream);
 /* Forward then inverse transform of d_data in place (the round trip of the
  * reference's test_ntt_inverse, tests/test_ntt.cu:60-123, for a whole RNS
- * batch).  The INT8 engine runs both in one persistent launch with
- * per-(poly, limb) stage dependencies; other engines run two transforms. */
+ * batch).  The CUDA-core engine runs one launch up to 2^13 and three above (the
+ * rows' two directions in one); the INT8 engine one persistent launch with
+ * per-(poly, limb) stage dependencies; other engines two transforms. */
 NTTB_API int nttb_rns_forward_inverse(const nttb_rns_plan* plan, uint32_t* d_data, uint32_t n_polys, int engine,
                                       void* stream);
 /* Streams n_batches consecutive batches of n_polys polynomials from host

@@ -58,6 +58,7 @@ int launch_rc(cudaError_t e) {
 int engine_status(int rc, const char* what) {
     if (rc == 0) return cuda_status(what);
     if (rc == 1) return fail(NTTB_ERR_UNSUPPORTED, "%s: shape not served by the requested engine", what);
+    if (rc == kNoWorkspace) return fail(NTTB_ERR_NO_MEMORY, "%s: no memory for the workspace", what);
     cudaError_t e = g_launch_error;
     g_launch_error = cudaSuccess;
     if (e == cudaSuccess) e = cudaGetLastError();
@@ -620,8 +621,12 @@ int nttb_rns_transform(const nttb_rns_plan* P, uint32_t* dst, const uint32_t* sr
     if (!P || !dst || !src) return fail(NTTB_ERR_INVALID_ARG, "rns_transform: null argument");
     if (n_polys == 0) return NTTB_OK;
     if ((((uintptr_t)dst) | ((uintptr_t)src)) & 15) return fail(NTTB_ERR_INVALID_ARG, "rns_transform: pointers must be 16-byte aligned");
-    int rc = run_transform32(const_cast<Plan32&>(P->p), src, dst, false, n_polys, inverse != 0, engine,
-                             (cudaStream_t)stream);
+    Plan32& p = const_cast<Plan32&>(P->p);
+    cudaStream_t s = (cudaStream_t)stream;
+    int rc = kNoWorkspace;
+    if (auto_radix32(p, (uint64_t)n_polys * p.n_limbs, engine, s))
+        rc = scalar_transform32(p, src, dst, false, n_polys, inverse != 0, s);
+    if (rc == kNoWorkspace) rc = run_transform32(p, src, dst, false, n_polys, inverse != 0, engine, s);
     return engine_status(rc, "rns_transform");
 }
 
@@ -631,9 +636,12 @@ int nttb_rns_forward_inverse(const nttb_rns_plan* P, uint32_t* d, uint32_t n_pol
     if (((uintptr_t)d) & 15) return fail(NTTB_ERR_INVALID_ARG, "rns_forward_inverse: pointer must be 16-byte aligned");
     Plan32& p = const_cast<Plan32&>(P->p);
     cudaStream_t s = (cudaStream_t)stream;
-    int eng = engine == NTTB_ENGINE_AUTO ? auto_engine32(p, false, (uint64_t)n_polys * p.n_limbs, true) : engine;
-    int rc;
-    if (eng == NTTB_ENGINE_INT8) {
+    const uint64_t units = (uint64_t)n_polys * p.n_limbs;
+    int rc = kNoWorkspace;
+    if (auto_radix32(p, units, engine, s) || (engine == NTTB_ENGINE_SCALAR && radix_serves(p.log_n)))
+        rc = scalar_round_trip32(p, d, n_polys, s);
+    if (rc != kNoWorkspace) return engine_status(rc, "rns_forward_inverse");
+    if ((engine == NTTB_ENGINE_AUTO ? auto_engine32(p, false, units, true) : engine) == NTTB_ENGINE_INT8) {
         rc = int8_forward_inverse32(p, d, n_polys, s);
     } else {
         rc = run_transform32(p, d, d, false, n_polys, false, engine, s);

@@ -17,15 +17,15 @@ static int env_engine() {
     return NTTB_ENGINE_AUTO;
 }
 
-// Out of place, the CUDA-core engine's register-radix passes (radix.cuh) are
-// the fastest at every size (us, forward, this engine / the other): 8 x 2^16
-// 6.6 / 16.6 (INT8), 24 x 2^16 9.7 / 17.4 (INT8), 192 x 2^16 54 / 95 (INT8),
-// 33 x 2^17 22.5 / 62 (tensor tiles), 1 x 2^20 10 / 25 (queue).  In place they
-// stage their first pass in the plan's workspace, which ties the plan's calls
-// to one stream; the sizes and counts below keep an engine that does not: the
-// INT8 cluster kernel at 2^16 from kInt8MinUnits (polynomial, limb) units on,
-// and the batch queue at 2^17 .. 2^20 once a call holds 2^20 residues (each
-// prepared queue has a ring of its own).
+// The CUDA-core engine's register-radix passes (radix.cuh) are the fastest at
+// every size (us, forward, this engine / the other): 8 x 2^16 6.6 / 16.6 (INT8),
+// 24 x 2^16 9.7 / 17.4 (INT8), 192 x 2^16 54 / 95 (INT8), 33 x 2^17 22.5 / 62
+// (tensor tiles), 1 x 2^20 10 / 25 (queue).  In place they stage their first pass
+// in a workspace; calls that must not need one (it could not be had, or the
+// stream is captured) and the drop-in's and the host stream's calls, whose
+// engines those entry points name, take the INT8 cluster kernel at 2^16 from
+// kInt8MinUnits (polynomial, limb) units on and the batch queue at 2^17 .. 2^20
+// once a call holds 2^20 residues (each prepared queue has a ring of its own).
 constexpr uint64_t kInt8MinUnits = 8;
 constexpr uint32_t kTilesMinLog = 17;
 constexpr uint64_t kTilesMinResidues = 1ull << 20;
@@ -35,6 +35,11 @@ int auto_engine32(const Plan32& p, bool src_u64, uint64_t units, bool in_place) 
     if (int8_serves(p, src_u64) && units >= kInt8MinUnits) return NTTB_ENGINE_INT8;
     if (tiles_serve(p) && p.log_n >= kTilesMinLog && (units << p.log_n) >= kTilesMinResidues) return NTTB_ENGINE_TILES;
     return NTTB_ENGINE_SCALAR;
+}
+
+bool auto_radix32(const Plan32& p, uint64_t units, int engine, cudaStream_t s) {
+    return engine == NTTB_ENGINE_AUTO && env_engine() == NTTB_ENGINE_AUTO && radix_serves(p.log_n) &&
+           scalar_serves(p, units) && (p.log_n <= kRadixSingleMax || !stream_capturing(s));
 }
 
 int run_transform32(Plan32& p, const void* src, void* dst, bool src_u64, uint32_t n_polys, bool inverse,

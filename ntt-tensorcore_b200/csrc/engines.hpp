@@ -17,6 +17,10 @@ int run_transform32(Plan32& p, const void* src, void* dst, bool src_u64, uint32_
 // Which engine AUTO resolves to for this plan (NTTB_ENGINE_*).
 int auto_engine32(const Plan32& p, bool src_u64, uint64_t units, bool in_place);
 
+// Whether an RNS call with this engine argument runs the register-radix passes,
+// in place too; if they then return kNoWorkspace, AUTO's other engines take it.
+bool auto_radix32(const Plan32& p, uint64_t units, int engine, cudaStream_t s);
+
 // Frees engine caches attached to a plan.
 void engines_release32(Plan32* p);
 

@@ -223,7 +223,83 @@ void* plan_workspace(void** ws, size_t* ws_bytes, size_t bytes) {
     return *ws;
 }
 
+bool stream_capturing(cudaStream_t s) {
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &st) != cudaSuccess) {
+        cudaGetLastError();  // the legacy stream while another stream is captured
+        return true;
+    }
+    return st != cudaStreamCaptureStatusNone;
+}
+
+static cudaMemPool_t plan_pool(PlanPool& pp) {  // pp.mu held
+    if (pp.tried) return pp.pool;
+    pp.tried = true;
+    cudaMemPoolProps props{};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    if (cudaGetDevice(&props.location.id) != cudaSuccess || cudaMemPoolCreate(&pp.pool, &props) != cudaSuccess) {
+        cudaGetLastError();
+        pp.pool = nullptr;
+        return nullptr;
+    }
+    uint64_t keep = ~0ull;  // what one call frees, the next takes; the pool goes with the plan
+    int off = 0;            // streams never wait for one another for memory
+    cudaMemPoolSetAttribute(pp.pool, cudaMemPoolAttrReleaseThreshold, &keep);
+    cudaMemPoolSetAttribute(pp.pool, cudaMemPoolReuseAllowInternalDependencies, &off);
+    return pp.pool;
+}
+
+StreamWorkspace::StreamWorkspace(PlanPool& pp, void** ws, size_t* ws_bytes, size_t bytes, cudaStream_t s)
+    : lock_(pp.mu), stream_(s) {
+    unsigned long long id = 0;
+    if (stream_capturing(s) || !plan_pool(pp) || cudaStreamGetId(s, &id) != cudaSuccess) {
+        cudaGetLastError();
+        ptr = plan_workspace(ws, ws_bytes, bytes);
+        if (!ptr) cudaGetLastError();
+        return;
+    }
+    PlanPool::Slot* slot = nullptr;
+    for (PlanPool::Slot& t : pp.slot)
+        if (t.ptr && t.stream == id) slot = &t;
+    if (!slot)
+        for (PlanPool::Slot& t : pp.slot)
+            if (!t.ptr && !slot) slot = &t;
+    if (slot && slot->bytes >= bytes) {
+        ptr = slot->ptr;
+        return;
+    }
+    if (slot && slot->ptr) {  // grown: freed behind the stream's earlier calls
+        cudaFreeAsync(slot->ptr, s);
+        *slot = PlanPool::Slot{};
+    }
+    if (cudaMallocFromPoolAsync(&ptr, bytes, pp.pool, s) != cudaSuccess) {
+        cudaGetLastError();
+        ptr = nullptr;
+    } else if (slot) {
+        *slot = {id, ptr, bytes};
+    } else {
+        per_call_ = true;
+        lock_.unlock();
+    }
+}
+
+StreamWorkspace::~StreamWorkspace() {
+    if (per_call_) cudaFreeAsync(ptr, stream_);
+}
+
+static void free_pool(PlanPool& pp) {
+    for (PlanPool::Slot& t : pp.slot) {
+        if (t.ptr) cudaFree(t.ptr);
+        t = PlanPool::Slot{};
+    }
+    if (pp.pool) cudaMemPoolDestroy(pp.pool);  // its memory goes once the last free has been reached
+    pp.pool = nullptr;
+    pp.tried = false;
+}
+
 void free_plan32(Plan32* p) {
+    free_pool(p->pool);
     if (p->ws) cudaFree(p->ws);
     p->ws = nullptr;
     p->ws_bytes = 0;
@@ -233,6 +309,7 @@ void free_plan32(Plan32* p) {
 }
 
 void free_plan64(Plan64* p) {
+    free_pool(p->pool);
     if (p->ws) cudaFree(p->ws);
     p->ws = nullptr;
     p->ws_bytes = 0;

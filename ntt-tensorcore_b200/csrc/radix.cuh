@@ -258,21 +258,72 @@ __device__ __forceinline__ void exchange(E* sm, E (&x)[NE]) {
 template <int LG, int LGV, int LGE>
 constexpr int kThreads = (1 << (LG + LGV - LGE)) > 128 ? (1 << (LG + LGV - LGE)) : 128;
 
-// SINGLE (LGV = 0, stride 1): rows of N = n elements, blockDim.y rows per CTA.
+// The rounds of one pass for a thread of a tile: where its registers sit before
+// and after, the roots of a round (fetched ahead of the wait that the round's
+// data needs), and the rounds.  TF: the first executed round's (else, TL, the
+// last's) threads run over positions before columns, for contiguous columns in
+// global memory.
+template <class A, int LG, int LGV, int LGE, bool INV, int S0, bool TF, bool TL>
+struct Pass {
+    using E = typename A::elem;
+    using P = typename PairOf<A>::type;
+    static constexpr uint32_t N = 1u << LG, NE = 1u << LGE, V = 1u << LGV, NT = N >> LGE;
+    static constexpr Rounds<LG, LGE> R{};
+    static constexpr int NR = R.n;
+    template <int K>
+    static constexpr bool kT = (TF && K == 0) || (TL && K == NR - 1);
+    template <int K>
+    static constexpr int kI = INV ? NR - 1 - K : K;
+    template <int K>
+    using Pl = Place<E, LG, LGV, LGE, kI<K>>;
+    // position t + (forward: e NT, natural; inverse: natural index t + rev(e) NT) of register e
+    __device__ __forceinline__ static constexpr uint32_t in(uint32_t e) { return (INV ? brv(e, LGE) : e) * NT; }
+    __device__ __forceinline__ static constexpr uint32_t out(uint32_t e) { return (INV ? e : brv(e, LGE)) * NT; }
+    template <int K>
+    __device__ __forceinline__ static uint32_t t() { return kT<K> ? threadIdx.x & (NT - 1u) : threadIdx.x >> LGV; }
+    template <int K>
+    __device__ __forceinline__ static uint32_t v() { return kT<K> ? threadIdx.x / NT : threadIdx.x & (V - 1u); }
+
+    template <int K>
+    __device__ __forceinline__ static void roots(P (&w)[NE - 1], const P* tab, uint32_t col0) {
+        round_roots<LG, LGE, kI<K>, S0, INV>(w, tab + (S0 > 0 ? col0 + v<K>() : 0u) + ((size_t)Pl<K>::natural(t<K>()) << S0));
+    }
+    template <int K = 0>
+    __device__ __forceinline__ static void run(const A& ar, E (&x)[NE], P (&w)[NE - 1], E* sm, const P* tab, uint32_t col0,
+                                               P c0, P c1) {
+        E* base = sm + (NR > 1 ? Pl<K>::base(t<K>()) + v<K>() : 0u);
+        if constexpr (K > 0) exchange<Pl<K>, false>(base, x);
+        round_stages<A, LG, LGE, kI<K>, S0, INV>(ar, x, w, c0, c1);
+        if constexpr (K < NR - 1) {
+            exchange<Pl<K>, true>(base, x);
+            roots<K + 1>(w, tab, col0);
+            __syncthreads();
+            run<K + 1>(ar, x, w, sm, tab, col0, c0, c1);
+        }
+    }
+};
+
+// How a pass reads and writes its columns in global memory.
+enum : int { kStrided = 0, kContOut = 1, kContIn = 2 };
+// What it runs: the forward or the inverse stages, or the forward ones and then
+// the inverse ones (a round trip's rows, which continue in registers).
+enum : int { kFwd = 0, kInv = 1, kBoth = 2 };
+
+// SINGLE (LGV = 0): rows of N = n elements, blockDim.y rows per CTA.
 // S0: first stage of the pass; above 0 the roots depend on the column (row u).
-// 2^LST: words between consecutive elements of a column.
-// CONT: outputs are stored column by column (transposed), else in place.
+// 2^LST: words between consecutive elements of a strided column.
 // TSM: threads per SM that the registers are budgeted for.
-template <class A, class S, class D, int LG, int LGV, int LGE, bool INV, int S0, int LST, bool CONT, int TSM>
+template <class A, class S, class D, int LG, int LGV, int LGE, int DIR, int S0, int LST, int MODE, int TSM>
 __global__ void __launch_bounds__(kThreads<LG, LGV, LGE>, TSM / kThreads<LG, LGV, LGE> > 0 ? TSM / kThreads<LG, LGV, LGE> : 1)
     radix_pass(const __grid_constant__ Args a, const LimbDev<A>* __restrict__ limbs) {
     using E = typename A::elem;
     using P = typename PairOf<A>::type;
-    constexpr uint32_t N = 1u << LG, NE = 1u << LGE, V = 1u << LGV, NT = N >> LGE;
-    constexpr Rounds<LG, LGE> R;
-    constexpr int NR = R.n;
+    using First = Pass<A, LG, LGV, LGE, DIR == kInv, S0, MODE == kContIn, MODE == kContOut>;
+    using Last = Pass<A, LG, LGV, LGE, DIR != kFwd, S0, MODE == kContIn, MODE == kContOut>;
+    constexpr uint32_t NE = 1u << LGE, V = 1u << LGV;
     constexpr bool kSingle = LGV == 0;
-    constexpr bool kLast = INV ? S0 == 0 : !CONT;  // the pass that leaves canonical residues
+    // the pass that leaves canonical residues
+    constexpr bool kLast = DIR == kFwd ? MODE != kContOut : S0 == 0;
     constexpr bool kReduce = sizeof(S) == 8 && sizeof(E) == 4;
     extern __shared__ __align__(16) unsigned char rdx_smem[];
     constexpr Lay<LG, LGV, kBankBits<E>, kLanePos<E, LG, LGV, LGE>> L;
@@ -292,14 +343,12 @@ __global__ void __launch_bounds__(kThreads<LG, LGV, LGE>, TSM / kThreads<LG, LGV
         n_poly = min(a.polys_per_cta, a.polys - poly);
         col0 = blockIdx.x * V;
     }
-    const uint32_t tid = threadIdx.x;
-    const uint32_t v_v = tid & (V - 1u), t_v = tid >> LGV;         // columns fastest
-    const uint32_t t_t = tid & (NT - 1u), v_t = tid / NT;          // positions fastest
     const LimbDev<A>& ld = limbs[limb];
     const A ar = ld.ar;
-    const P* tab = reinterpret_cast<const P*>(INV ? ld.rt_inv : ld.rt);
-    P c0{}, c1{}, one{};
-    if (INV && S0 == 0) {
+    const P* itab = reinterpret_cast<const P*>(ld.rt_inv);
+    const P* tab = DIR == kInv ? itab : reinterpret_cast<const P*>(ld.rt);
+    P c0{}, c1{}, one{}, w[NE - 1];
+    if (DIR != kFwd && S0 == 0) {
         c0 = __ldg(reinterpret_cast<const P*>(ld.scale));
         c1 = __ldg(reinterpret_cast<const P*>(ld.scale) + 1);
     }
@@ -307,69 +356,49 @@ __global__ void __launch_bounds__(kThreads<LG, LGV, LGE>, TSM / kThreads<LG, LGV
     const uint64_t off = (uint64_t)poly * a.poly_stride + ((uint64_t)limb << a.log_n);
     const S* src = reinterpret_cast<const S*>(a.src) + off;
     D* dst = reinterpret_cast<D*>(a.dst) + off;
-    // round K's place of this thread and its roots
-    P w[NE - 1];
-    auto roots = [&](auto step) {
-        constexpr int K = decltype(step)::value, I = INV ? NR - 1 - K : K;
-        constexpr bool tfast = CONT && K == NR - 1;
-        using Pl = Place<E, LG, LGV, LGE, I>;
-        const uint32_t t = tfast ? t_t : t_v, col = col0 + (tfast ? v_t : v_v);
-        round_roots<LG, LGE, I, S0, INV>(w, tab + (S0 > 0 ? col : 0u) + ((size_t)Pl::natural(t) << S0));
-    };
-    roots(std::integral_constant<int, 0>{});
+    First::template roots<0>(w, tab, col0);
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
-    E x[NE];
-    // strided load: element e of thread t is position t + e NT (forward), or the
-    // position whose natural index is rev(e) NT + t (inverse); the parts share no
-    // bit, so every address is a thread's base plus a constant
-    auto load = [&](uint32_t t, uint32_t col) {
-        const S* p = src + (((size_t)t << LST) + col);
-#pragma unroll
-        for (uint32_t e = 0; e < NE; e++) {
-            const S w = __ldcg(p + ((size_t)((INV ? brv(e, LGE) : e) * NT) << LST));
-            if constexpr (kReduce) {
-                const uint32_t y = (uint32_t)w;
-                x[e] = sub_if(y - __umulhi(y, one.y) * ar.q, ar.q);
-            } else {
-                x[e] = (E)w;
-            }
-        }
-    };
-    auto store = [&](uint32_t t, uint32_t col) {
-        D* p = dst + (CONT ? ((size_t)col << LG) + t : ((size_t)t << LST) + col);
-#pragma unroll
-        for (uint32_t e = 0; e < NE; e++) {
-            const E y = kLast ? canon_out<INV>(ar, x[e]) : x[e];
-            if (active) p[(size_t)((INV ? e : brv(e, LGE)) * NT) << (CONT ? 0 : LST)] = (D)y;
-        }
-    };
-    auto run = [&](auto self, auto step) -> void {
-        constexpr int K = decltype(step)::value;         // K-th round executed
-        constexpr int I = INV ? NR - 1 - K : K;          // its index in the forward order
-        constexpr bool tfast = CONT && K == NR - 1;
-        using Pl = Place<E, LG, LGV, LGE, I>;
-        const uint32_t t = tfast ? t_t : t_v, v = tfast ? v_t : v_v, col = col0 + v;
-        E* base = sm + (NR > 1 ? Pl::base(t) + v : 0u);
-        if constexpr (K == 0) load(t, col);
-        else exchange<Pl, false>(base, x);
-        round_stages<A, LG, LGE, I, S0, INV>(ar, x, w, c0, c1);
-        if constexpr (K < NR - 1) {
-            exchange<Pl, true>(base, x);
-            roots(std::integral_constant<int, K + 1>{});
-            __syncthreads();
-            self(self, std::integral_constant<int, K + 1>{});
-        } else {
-            store(t, col);
-        }
-    };
+    // register e's position is a thread's base plus a constant: the parts share no bit
+    constexpr int LI = MODE == kContIn ? 0 : LST, LO = MODE == kContOut ? 0 : LST, NR = First::NR;
     for (uint32_t k = 0; k < n_poly; k++) {
         if (k) {
-            roots(std::integral_constant<int, 0>{});
+            First::template roots<0>(w, tab, col0);
             __syncthreads();  // the tile's last reads precede the next polynomial's stores
         }
-        run(run, std::integral_constant<int, 0>{});
+        E x[NE];
+        {
+            const uint32_t t = First::template t<0>(), col = col0 + First::template v<0>();
+            const S* p = src + (MODE == kContIn ? ((size_t)col << LG) + t : ((size_t)t << LST) + col);
+#pragma unroll
+            for (uint32_t e = 0; e < NE; e++) {
+                const S y = __ldcg(p + ((size_t)First::in(e) << LI));
+                if constexpr (kReduce) {  // any word below 2^32: its residue
+                    x[e] = sub_if((uint32_t)y - __umulhi((uint32_t)y, one.y) * ar.q, ar.q);
+                } else {
+                    x[e] = (E)y;
+                }
+            }
+        }
+        First::run(ar, x, w, sm, tab, col0, c0, c1);
+        if constexpr (DIR == kBoth) {
+            // the forward stages' last positions are the inverse's first, and a
+            // thread overwrites the shared memory that it has read: no barrier
+#pragma unroll
+            for (uint32_t e = 0; e < NE; e++) x[e] = canon_out<false>(ar, x[e]);
+            Last::template roots<0>(w, itab, col0);
+            Last::run(ar, x, w, sm, itab, col0, c0, c1);
+        }
+        {
+            const uint32_t t = Last::template t<NR - 1>(), col = col0 + Last::template v<NR - 1>();
+            D* p = dst + (MODE == kContOut ? ((size_t)col << LG) + t : ((size_t)t << LST) + col);
+#pragma unroll
+            for (uint32_t e = 0; e < NE; e++) {
+                const E y = kLast ? canon_out<(DIR != kFwd)>(ar, x[e]) : x[e];
+                if (active) p[(size_t)Last::out(e) << LO] = (D)y;
+            }
+        }
         src += a.poly_stride;
         dst += a.poly_stride;
     }

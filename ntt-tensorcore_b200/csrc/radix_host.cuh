@@ -4,6 +4,8 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <atomic>
+
 #include "plan.hpp"
 #include "profiler.hpp"
 #include "radix.cuh"
@@ -15,6 +17,20 @@ namespace rdx {
 // passes of 2^ceil(L/2) and 2^floor(L/2) points above.
 constexpr uint32_t kSingleMax = 13;
 constexpr uint32_t kThreadsMin = 128;  // rows are grouped into CTAs of at least this many threads
+
+// Shared-memory attributes of a kernel, set once per device: its dynamic size,
+// and the largest carveout, so that as many CTAs fit an SM as it is built for.
+template <auto K>
+void kernel_smem(size_t smem) {
+    static std::atomic<uint64_t> done{0};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    const uint64_t bit = 1ull << (dev & 63);
+    if (done.load(std::memory_order_acquire) & bit) return;
+    cudaFuncSetAttribute(K, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaFuncSetAttribute(K, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared);
+    done.fetch_or(bit, std::memory_order_release);
+}
 
 template <class K>
 int launch(K kernel, const char* name, dim3 grid, dim3 block, size_t smem, const Args& a, const void* limbs,
@@ -36,20 +52,20 @@ int launch(K kernel, const char* name, dim3 grid, dim3 block, size_t smem, const
     return launch_rc(cudaLaunchKernelExC(&cfg, reinterpret_cast<const void*>(kernel), params));
 }
 
-template <class A, class S, int LG, int LGE, bool INV>
+template <class A, class S, int LG, int LGE, int DIR>
 int launch_single(Args a, const LimbDev<A>* limbs, cudaStream_t s) {
     using E = typename A::elem;
     constexpr uint32_t NT = 1u << (LG - LGE);
     constexpr Lay<LG, 0, kBankBits<E>, kLanePos<E, LG, 0, LGE>> L;
-    auto k = radix_pass<A, S, S, LG, 0, LGE, INV, 0, 0, false, 1024>;
+    constexpr auto k = radix_pass<A, S, S, LG, 0, LGE, DIR, 0, 0, kStrided, 1024>;
     uint32_t rows = NT < kThreadsMin ? kThreadsMin / NT : 1u;
     while (rows > 1 && (a.units + rows - 1) / rows < 148) rows >>= 1;  // small calls spread over the SMs first
     const size_t smem = (size_t)rows * L.words * sizeof(E);
-    if (smem > 48 * 1024) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if constexpr ((size_t)L.words * sizeof(E) > 48 * 1024) kernel_smem<k>((size_t)L.words * sizeof(E));
     return launch(k, "scalar_pass_row", dim3((a.units + rows - 1) / rows), dim3(NT, rows), smem, a, limbs, s);
 }
 
-template <class A, class S, class D, int LG, int LGV, int LGE, bool INV, int S0, int LST, bool CONT>
+template <class A, class S, class D, int LG, int LGV, int LGE, int DIR, int S0, int LST, int MODE>
 int launch_pass(Args a, const LimbDev<A>* limbs, cudaStream_t s) {
     using E = typename A::elem;
     constexpr Lay<LG, LGV, kBankBits<E>, kLanePos<E, LG, LGV, LGE>> L;
@@ -67,10 +83,14 @@ int launch_pass(Args a, const LimbDev<A>* limbs, cudaStream_t s) {
     // and want twice the warps.  Forward of 24 x 2^16: 9.7 us against 11.9; of
     // 33 x 2^17: 26.5 against 22.8
     constexpr uint32_t threads = 1u << (LG + LGV - LGE);
-    auto k = ctas * threads <= 148u * 1024u ? radix_pass<A, S, D, LG, LGV, LGE, INV, S0, LST, CONT, 512>
-                                            : radix_pass<A, S, D, LG, LGV, LGE, INV, S0, LST, CONT, 1024>;
-    if (smem > 48 * 1024) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    return launch(k, CONT ? "scalar_pass_col" : "scalar_pass_col_b",
+    constexpr auto few = radix_pass<A, S, D, LG, LGV, LGE, DIR, S0, LST, MODE, 512>;
+    constexpr auto many = radix_pass<A, S, D, LG, LGV, LGE, DIR, S0, LST, MODE, 1024>;
+    const bool one_wave = ctas * threads <= 148u * 1024u;
+    if constexpr (smem > 48 * 1024) {
+        if (one_wave) kernel_smem<few>(smem);
+        else kernel_smem<many>(smem);
+    }
+    return launch(one_wave ? few : many, MODE == kContOut ? "scalar_pass_col" : DIR == kBoth ? "scalar_pass_mid" : "scalar_pass_col_b",
                   dim3(tiles, a.n_limbs, (a.polys + ppc - 1) / ppc), dim3(threads), smem, a, limbs, s);
 }
 
@@ -87,20 +107,34 @@ int launch_two(Args a, void* mid, const LimbDev<A>* limbs, bool inverse, cudaStr
     constexpr int LA = (L + 1) / 2, LB = L / 2, LGV = kLogCols<A, S, L>;
     void* dst = a.dst;
     a.dst = mid;
-    int rc = inverse ? launch_pass<A, S, M, LB, LGV, LGE, true, LA, LA, true>(a, limbs, s)
-                     : launch_pass<A, S, M, LA, LGV, LGE, false, 0, LB, true>(a, limbs, s);
+    int rc = inverse ? launch_pass<A, S, M, LB, LGV, LGE, kInv, LA, LA, kContOut>(a, limbs, s)
+                     : launch_pass<A, S, M, LA, LGV, LGE, kFwd, 0, LB, kContOut>(a, limbs, s);
     if (rc) return rc;
     a.src = mid;
     a.dst = dst;
-    return inverse ? launch_pass<A, M, S, LA, LGV, LGE, true, 0, LB, false>(a, limbs, s)
-                   : launch_pass<A, M, S, LB, LGV, LGE, false, LA, LA, false>(a, limbs, s);
+    return inverse ? launch_pass<A, M, S, LA, LGV, LGE, kInv, 0, LB, kStrided>(a, limbs, s)
+                   : launch_pass<A, M, S, LB, LGV, LGE, kFwd, LA, LA, kStrided>(a, limbs, s);
 }
 
-// Runs one transform of n_polys x n_limbs rows; `mid` (two-pass sizes) holds
-// the first pass in words of M.  Returns 1 when the size is not served.
-template <class A, class S, class M, int LGE>
-int transform(const LimbDev<A>* limbs, uint32_t log_n, uint32_t n_limbs, const void* src, void* dst, void* mid,
-              uint32_t n_polys, bool inverse, cudaStream_t s) {
+// Forward then inverse of one size, in place through `mid`: the first pass, the
+// rows' forward and inverse stages in one pass over `mid`, the last pass (which
+// reads contiguous columns): three passes over memory instead of four.
+template <class A, class S, int L, int LGE>
+int launch_round_trip(Args a, void* mid, const LimbDev<A>* limbs, cudaStream_t s) {
+    constexpr int LA = (L + 1) / 2, LB = L / 2, LGV = kLogCols<A, S, L>;
+    void* data = a.dst;
+    a.dst = mid;
+    int rc = launch_pass<A, S, S, LA, LGV, LGE, kFwd, 0, LB, kContOut>(a, limbs, s);
+    if (rc) return rc;
+    a.src = mid;
+    rc = launch_pass<A, S, S, LB, LGV, LGE, kBoth, LA, LA, kStrided>(a, limbs, s);
+    if (rc) return rc;
+    a.dst = data;
+    return launch_pass<A, S, S, LA, LGV, LGE, kInv, 0, LB, kContIn>(a, limbs, s);
+}
+
+template <class A>
+Args make_args(uint32_t log_n, uint32_t n_limbs, const void* src, void* dst, uint32_t n_polys) {
     Args a{};
     a.src = src;
     a.dst = dst;
@@ -109,8 +143,17 @@ int transform(const LimbDev<A>* limbs, uint32_t log_n, uint32_t n_limbs, const v
     a.polys = n_polys;
     a.n_limbs = n_limbs;
     a.units = n_polys * n_limbs;
+    return a;
+}
+
+// Runs one transform of n_polys x n_limbs rows; `mid` (two-pass sizes) holds
+// the first pass in words of M.  Returns 1 when the size is not served.
+template <class A, class S, class M, int LGE>
+int transform(const LimbDev<A>* limbs, uint32_t log_n, uint32_t n_limbs, const void* src, void* dst, void* mid,
+              uint32_t n_polys, bool inverse, cudaStream_t s) {
+    const Args a = make_args<A>(log_n, n_limbs, src, dst, n_polys);
 #define NTTB_SINGLE(l) \
-    case l: return inverse ? launch_single<A, S, l, LGE, true>(a, limbs, s) : launch_single<A, S, l, LGE, false>(a, limbs, s);
+    case l: return inverse ? launch_single<A, S, l, LGE, kInv>(a, limbs, s) : launch_single<A, S, l, LGE, kFwd>(a, limbs, s);
 #define NTTB_TWO(l) \
     case l: return launch_two<A, S, M, l, LGE>(a, mid, limbs, inverse, s);
     switch (log_n) {

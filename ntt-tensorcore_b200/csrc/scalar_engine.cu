@@ -375,21 +375,34 @@ static size_t staged_words(uint32_t log_n, uint32_t e_max, uint32_t n_limbs, uin
     return two ? ((size_t)n_polys * n_limbs) << log_n : 0;
 }
 
-int scalar_transform32(Plan32& p, const void* src, void* dst, bool src_u64, uint32_t n_polys, bool inverse,
-                       cudaStream_t s) {
-    const bool radix = radix_serves(p.log_n);
-    void* mid = dst;
-    if (const size_t words = staged_words(p.log_n, 8192, p.n_limbs, n_polys); words && (src == dst || (radix && src_u64))) {
-        mid = plan_workspace(&p.ws, &p.ws_bytes, words * (src_u64 && !radix ? 8 : 4));
-        if (!mid) return 2;
-    }
-    if (n_polys > 65535 || p.n_limbs > 65535) return 1;
-    if (radix) return (src_u64 ? radix_w64 : radix_u32)(p, src, dst, mid, n_polys, inverse, s);
+static int run32(Plan32& p, const void* src, void* dst, void* mid, bool src_u64, uint32_t n_polys, bool inverse,
+                 cudaStream_t s) {
+    if (radix_serves(p.log_n)) return (src_u64 ? radix_w64 : radix_u32)(p, src, dst, mid, n_polys, inverse, s);
     if (src_u64)
         return transform_generic<uint64_t, M32>(p.log_n, p.n_limbs, p.negacyclic, p.d_limbs, src, dst, mid, n_polys,
                                                 inverse, 8192, s);
     return transform_generic<uint32_t, M32>(p.log_n, p.n_limbs, p.negacyclic, p.d_limbs, src, dst, mid, n_polys,
                                             inverse, 8192, s);
+}
+
+int scalar_transform32(Plan32& p, const void* src, void* dst, bool src_u64, uint32_t n_polys, bool inverse,
+                       cudaStream_t s) {
+    if (n_polys > 65535 || p.n_limbs > 65535) return 1;
+    const bool radix = radix_serves(p.log_n);
+    const size_t words = staged_words(p.log_n, 8192, p.n_limbs, n_polys);
+    if (!words || (src != dst && !(radix && src_u64))) return run32(p, src, dst, dst, src_u64, n_polys, inverse, s);
+    StreamWorkspace ws(p.pool, &p.ws, &p.ws_bytes, words * (src_u64 && !radix ? 8 : 4), s);
+    if (!ws.ptr) return kNoWorkspace;
+    return run32(p, src, dst, ws.ptr, src_u64, n_polys, inverse, s);
+}
+
+int scalar_round_trip32(Plan32& p, uint32_t* data, uint32_t n_polys, cudaStream_t s) {
+    if (!radix_serves(p.log_n) || n_polys > 65535 || p.n_limbs > 65535) return 1;
+    const size_t words = staged_words(p.log_n, 8192, p.n_limbs, n_polys);
+    if (!words) return radix_round_trip_u32(p, data, nullptr, n_polys, s);
+    StreamWorkspace ws(p.pool, &p.ws, &p.ws_bytes, words * 4, s);
+    if (!ws.ptr) return kNoWorkspace;
+    return radix_round_trip_u32(p, data, ws.ptr, n_polys, s);
 }
 
 int scalar_transform32_ws(const Plan32& p, uint32_t* data, void* ws, uint32_t n_polys, bool inverse,
@@ -403,16 +416,19 @@ size_t scalar_transform32_ws_bytes(const Plan32& p, uint32_t n_polys) {
     return staged_words(p.log_n, 8192, p.n_limbs, n_polys) * sizeof(uint32_t);
 }
 
-int scalar_transform64(Plan64& p, const void* src, void* dst, uint32_t n_polys, bool inverse, cudaStream_t s) {
-    void* mid = dst;
-    if (const size_t words = staged_words(p.log_n, 4096, p.n_limbs, n_polys); words && src == dst) {
-        mid = plan_workspace(&p.ws, &p.ws_bytes, words * 8);
-        if (!mid) return 2;
-    }
-    if (n_polys > 65535 || p.n_limbs > 65535) return 1;
+static int run64(Plan64& p, const void* src, void* dst, void* mid, uint32_t n_polys, bool inverse, cudaStream_t s) {
     if (radix_serves(p.log_n)) return radix_q64(p, src, dst, mid, n_polys, inverse, s);
     return transform_generic<uint64_t, M64>(p.log_n, p.n_limbs, p.negacyclic, p.d_limbs, src, dst, mid, n_polys,
                                             inverse, 4096, s);
+}
+
+int scalar_transform64(Plan64& p, const void* src, void* dst, uint32_t n_polys, bool inverse, cudaStream_t s) {
+    if (n_polys > 65535 || p.n_limbs > 65535) return 1;
+    const size_t words = staged_words(p.log_n, 4096, p.n_limbs, n_polys);
+    if (!words || src != dst) return run64(p, src, dst, dst, n_polys, inverse, s);
+    StreamWorkspace ws(p.pool, &p.ws, &p.ws_bytes, words * 8, s);
+    if (!ws.ptr) return kNoWorkspace;
+    return run64(p, src, dst, ws.ptr, n_polys, inverse, s);
 }
 
 // The RowMaj pre-transposed layout pre[b*M + a] = x[a*M + b] for n = M^2
