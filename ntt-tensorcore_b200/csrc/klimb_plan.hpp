@@ -2,12 +2,14 @@
 // (csrc/klimb.cu), host-only so that it can be checked on the CPU.
 //
 // A transform of 2^log_n elements runs either as one tile in one launch (the
-// bit reversal fused into the loads), or as a tiled bit reversal followed by
-// passes of radix-2 DIT stages: pass i runs stages s0 .. s0 + r - 1 on tiles
-// of 2^(r + logC) elements (2^logC columns of 2^r-element groups, logC <= s0).
+// bit reversal in its loads), or as a first pass that swaps tile pairs (the bit
+// reversal and the first r stages, r bits at either end of the index), followed
+// by passes of radix-2 DIT stages: pass i runs stages s0 .. s0 + r - 1 on tiles of
+// 2^(r + logC) elements (2^logC columns of 2^r-element groups, logC <= s0), the
+// stages spread evenly over as few passes as 8 stages each allow.
 // Tiles hold at most 2^log_emax elements, 48 KB of shared memory at the
-// largest; log_emax shrinks while a pass would have fewer than 148 tiles
-// (small transforms are bound by the latency of their stage chains, so more,
+// largest; log_emax shrinks while a pass would have fewer than kKlimbTargetCtas
+// tiles (small transforms are bound by the latency of their stage chains, so more,
 // shorter tiles win), but not below 2^6.
 #pragma once
 
@@ -26,7 +28,8 @@ struct KlimbPlan {
     KlimbPass pass[24];
 };
 
-constexpr uint32_t kKlimbTargetCtas = 148;
+// 128 tiles of 128 threads are one warp per scheduler on most of the 148 SMs
+constexpr uint32_t kKlimbTargetCtas = 128;
 
 // K: limbs per element (2, 3 or 11); log_n <= 24
 inline KlimbPlan klimb_plan(uint32_t K, uint32_t log_n) {
@@ -38,16 +41,16 @@ inline KlimbPlan klimb_plan(uint32_t K, uint32_t log_n) {
     // measured: K <= 3 up to 2^10, K = 11 up to 2^8 are fastest as one tile
     P.single_tile = log_n <= (K <= 3 ? 10u : 8u);
     if (P.single_tile) return P;
-    uint32_t s0 = 0;
-    while (s0 < log_n) {
-        uint32_t r = log_n - s0, logC = 0;
-        if (s0 == 0) {
-            if (r > log_emax) r = log_emax;
-        } else {
-            if (r > 8) r = 8;
-            if (r > log_emax) r = log_emax;
-            logC = log_emax - r < s0 ? log_emax - r : s0;
-        }
+    // the swapping pass: pairs of 2^h x 2^h tiles, one butterfly per thread
+    const uint32_t h = 4;
+    P.pass[P.n_passes++] = {0, h, 0};
+    // a thread per butterfly: tiles of at most 2^10 (K <= 3) or 2^9 elements
+    const uint32_t log_tile = log_emax < (K <= 3 ? 10u : 9u) ? log_emax : (K <= 3 ? 10u : 9u);
+    const uint32_t most = log_tile < 8 ? log_tile : 8u;
+    uint32_t s0 = h;
+    for (uint32_t left = (log_n - h + most - 1) / most; left > 0; left--) {
+        const uint32_t r = (log_n - s0 + left - 1) / left;
+        const uint32_t logC = log_tile - r < s0 ? log_tile - r : s0;
         P.pass[P.n_passes++] = {s0, r, logC};
         s0 += r;
     }
