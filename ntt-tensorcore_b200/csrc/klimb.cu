@@ -438,7 +438,7 @@ template <class F, int WHERE>
 int launch(const F& f, const PassArgs& g, uint32_t blocks, uint32_t elements, cudaStream_t s) {
     constexpr auto k = klimb_pass<F, WHERE, F::K <= 3 ? 512 : 256>;
     constexpr size_t kAlone = 116 * 1024;
-    rdx::kernel_smem<k>(kAlone);
+    rdx::kernel_smem<k, true>(kAlone);
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(blocks);
     cfg.blockDim = dim3(elements / 2);

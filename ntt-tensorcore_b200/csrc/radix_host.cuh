@@ -18,9 +18,11 @@ namespace rdx {
 constexpr uint32_t kSingleMax = 13;
 constexpr uint32_t kThreadsMin = 128;  // rows are grouped into CTAs of at least this many threads
 
-// Shared-memory attributes of a kernel, set once per device: its dynamic size,
-// and the largest carveout, so that as many CTAs fit an SM as it is built for.
-template <auto K>
+// Shared-memory attributes of a kernel, set once per device: the dynamic size it
+// may ask for and, with `carveout`, the largest shared-memory share of the SM, so that
+// as many CTAs fit as it is built for (the roots that others read stay in L1, which
+// that would take away: 33 x 2^17 25.6 -> 30.1 us).
+template <auto K, bool carveout>
 void kernel_smem(size_t smem) {
     static std::atomic<uint64_t> done{0};
     int dev = 0;
@@ -28,9 +30,29 @@ void kernel_smem(size_t smem) {
     const uint64_t bit = 1ull << (dev & 63);
     if (done.load(std::memory_order_acquire) & bit) return;
     cudaFuncSetAttribute(K, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    cudaFuncSetAttribute(K, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared);
+    if (carveout)
+        cudaFuncSetAttribute(K, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared);
     done.fetch_or(bit, std::memory_order_release);
 }
+
+// Dynamic shared memory that keeps a grid of a few blocks an SM spread out.  With
+// programmatic launches the blocks that start while the grid before drains crowd
+// the SMs that happen to be free, and finish last.  Asking for a share of the SM's
+// 228 KB such that only ceil(grid / 148) blocks fit prevents it.  us: 52 x 2^14
+// round trip 14.2 -> 10.7, 33 x 2^15 forward 9.4 -> 7.5, 4 x 2^18 11.8 -> 9.3,
+// 8 x 2^17 9.3 -> 8.4, 64-bit 18 x 2^15 12.1 -> 11.7, 4 x 2^17 12.7 -> 12.0.  Not below two blocks an SM,
+// where the early start hides more than it costs (64-bit 1 x 2^18 8.5, spread 9.4);
+// up to 4 for 32-bit words (beyond, L1 for the roots is worth more: 96 x 2^14 round
+// trip 15.6, spread 16.1), 8 for 64-bit ones; from 3 for the round trip's middle
+// pass, which reads two tables (18 x 2^15: 9.9, spread 12.1).  Two passes only: one
+// launch by itself gains nothing.
+inline size_t spread_smem(uint64_t grid, size_t smem, uint32_t least, uint32_t most) {
+    const uint64_t per = (grid + 147) / 148;
+    if (per < least || per > most) return smem;
+    const size_t share = 228 * 1024 / (per + 1);
+    return smem > share ? smem : share;
+}
+constexpr size_t kSpreadMax = 228 * 1024 / 3;
 
 template <class K>
 int launch(K kernel, const char* name, dim3 grid, dim3 block, size_t smem, const Args& a, const void* limbs,
@@ -61,7 +83,7 @@ int launch_single(Args a, const LimbDev<A>* limbs, cudaStream_t s) {
     uint32_t rows = NT < kThreadsMin ? kThreadsMin / NT : 1u;
     while (rows > 1 && (a.units + rows - 1) / rows < 148) rows >>= 1;  // small calls spread over the SMs first
     const size_t smem = (size_t)rows * L.words * sizeof(E);
-    if constexpr ((size_t)L.words * sizeof(E) > 48 * 1024) kernel_smem<k>((size_t)L.words * sizeof(E));
+    if constexpr ((size_t)L.words * sizeof(E) > 48 * 1024) kernel_smem<k, true>((size_t)L.words * sizeof(E));
     return launch(k, "scalar_pass_row", dim3((a.units + rows - 1) / rows), dim3(NT, rows), smem, a, limbs, s);
 }
 
@@ -69,7 +91,7 @@ template <class A, class S, class D, int LG, int LGV, int LGE, int DIR, int S0, 
 int launch_pass(Args a, const LimbDev<A>* limbs, cudaStream_t s) {
     using E = typename A::elem;
     constexpr Lay<LG, LGV, kBankBits<E>, kLanePos<E, LG, LGV, LGE>> L;
-    constexpr size_t smem = (size_t)L.words * sizeof(E);
+    constexpr size_t tile_smem = (size_t)L.words * sizeof(E);
     constexpr uint32_t tiles = 1u << (LST - LGV);
     // a CTA keeps its columns' roots in L1 over several polynomials once the
     // launch has CTAs to spare
@@ -86,12 +108,13 @@ int launch_pass(Args a, const LimbDev<A>* limbs, cudaStream_t s) {
     constexpr auto few = radix_pass<A, S, D, LG, LGV, LGE, DIR, S0, LST, MODE, 512>;
     constexpr auto many = radix_pass<A, S, D, LG, LGV, LGE, DIR, S0, LST, MODE, 1024>;
     const bool one_wave = ctas * threads <= 148u * 1024u;
-    if constexpr (smem > 48 * 1024) {
-        if (one_wave) kernel_smem<few>(smem);
-        else kernel_smem<many>(smem);
-    }
+    const uint32_t chunks = (a.polys + ppc - 1) / ppc;
+    const size_t smem = spread_smem((uint64_t)tiles * a.n_limbs * chunks, tile_smem, DIR == kBoth ? 3 : 2, sizeof(E) == 8 ? 8 : 4);
+    constexpr size_t most = tile_smem > kSpreadMax ? tile_smem : kSpreadMax;
+    if (one_wave) kernel_smem<few, (tile_smem > 48 * 1024)>(most);
+    else kernel_smem<many, (tile_smem > 48 * 1024)>(most);
     return launch(one_wave ? few : many, MODE == kContOut ? "scalar_pass_col" : DIR == kBoth ? "scalar_pass_mid" : "scalar_pass_col_b",
-                  dim3(tiles, a.n_limbs, (a.polys + ppc - 1) / ppc), dim3(threads), smem, a, limbs, s);
+                  dim3(tiles, a.n_limbs, chunks), dim3(threads), smem, a, limbs, s);
 }
 
 // Columns per tile: a warp's loads touch 32 / V lines of 128 bytes, and at
