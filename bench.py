@@ -697,7 +697,7 @@ def run_uneven(args, world, rank, local):
     traffic, traffic_src = None, None
     try:
         with open(os.path.join(ROOT, "profiles", "traffic.json")) as f:
-            bpr = json.load(f).get("batch_queue_tc_bytes_per_residue")
+            bpr = json.load(f).get("batch_queue_radix_bytes_per_residue")
         if bpr and info["config"].get("tensor"):
             traffic = bpr * coeffs
             traffic_src = "ncu DRAM bytes per residue of a 150 M-residue capture, scaled to this launch's residues"
@@ -713,7 +713,7 @@ def run_uneven(args, world, rank, local):
                    "workspace_bytes": info["ws_bytes"], "tuned": tuned, "l2": "inputs 7.9 GB >> L2",
                    "parallelism": "replicas x%d" % world},
         "graph_replay": {"value": world * coeffs * args.steps / (g_ms / 1e3), "ms_per_step": g_ms / args.steps},
-        "roofline": {"bound": "hbm", "kernel": "batch_queue_tc" if info["config"].get("tensor") else "batch_queue",
+        "roofline": {"bound": "hbm", "kernel": "batch_queue_radix" if info["config"].get("tensor") else "batch_queue",
                      "achieved": alg_bytes / avg_s / 1e9, "peak": peak,
                      "unit": "GB/s", "frac": alg_bytes / avg_s / 1e9 / peak, "traffic": traffic,
                      "traffic_source": traffic_src,
@@ -1114,7 +1114,7 @@ def profile_case(name):
     int8 / dmma: forward+inverse of the 24-limb 2^16 negacyclic batch, four
     launches; batch: a ~600 MB uneven batch (log2 N 12..20, 1..8 limbs, mixed
     directions) launched twice; batch_tc: the same with log2 N 17..20 on
-    tensor-core tiles; q60: forward + inverse of one 2^20 polynomial mod the
+    register-radix tiles; q60: forward + inverse of one 2^20 polynomial mod the
     60-bit prime, four times; move: the TMA tile kernels on 4096 x 4096
     words (transpose, in-place transpose, bit reversal), one launch each;
     klimb: the K-limb forward NTT over the BN254 field (K = 11) at 2^14,
