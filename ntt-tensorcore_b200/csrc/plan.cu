@@ -243,6 +243,7 @@ static cudaMemPool_t plan_pool(PlanPool& pp) {  // pp.mu held
         pp.pool = nullptr;
         return nullptr;
     }
+    pp.device = props.location.id;
     uint64_t keep = ~0ull;  // what one call frees, the next takes; the pool goes with the plan
     int off = 0;            // streams never wait for one another for memory
     cudaMemPoolSetAttribute(pp.pool, cudaMemPoolAttrReleaseThreshold, &keep);
@@ -289,11 +290,22 @@ StreamWorkspace::~StreamWorkspace() {
 }
 
 static void free_pool(PlanPool& pp) {
-    for (PlanPool::Slot& t : pp.slot) {
-        if (t.ptr) cudaFree(t.ptr);
-        t = PlanPool::Slot{};
+    if (!pp.pool) return;  // no call has staged anything
+    // cudaFree of stream-ordered memory does not wait for the calls that still use
+    // it, as that of cudaMalloc's does: wait for them here.  Where the device cannot
+    // be waited for, the memory stays allocated.
+    int dev = pp.device;
+    cudaGetDevice(&dev);
+    if (dev != pp.device) cudaSetDevice(pp.device);
+    if (cudaDeviceSynchronize() == cudaSuccess) {
+        for (PlanPool::Slot& t : pp.slot)
+            if (t.ptr) cudaFree(t.ptr);
+        cudaMemPoolDestroy(pp.pool);  // its memory goes once the last free has been reached
+    } else {
+        cudaGetLastError();
     }
-    if (pp.pool) cudaMemPoolDestroy(pp.pool);  // its memory goes once the last free has been reached
+    if (dev != pp.device) cudaSetDevice(dev);
+    for (PlanPool::Slot& t : pp.slot) t = PlanPool::Slot{};
     pp.pool = nullptr;
     pp.tried = false;
 }

@@ -87,6 +87,7 @@ struct PlanPool {
         size_t bytes = 0;
     };
     cudaMemPool_t pool = nullptr;
+    int device = -1;
     bool tried = false;
     Slot slot[kSlots];
     std::mutex mu;
