@@ -40,16 +40,18 @@ enum {
 };
 
 /* Inner-DFT engines.  AUTO takes the CUDA-core engine for RNS plans and wide
- * plans.  Its in-place calls above 2^13 stage a pass in a workspace of the plan's
- * (one for each of the first four streams, then one per call, in stream order:
- * streams and threads may share a plan).  Where that memory cannot be had, while
- * the stream is captured, and for the drop-in's uint64 words and the host stream,
- * AUTO takes the INT8 tensor-core kernel at N = 2^16 from 8 (polynomial, limb)
- * units on, the batch queue at N = 2^17 .. 2^20 once a call holds 2^20 residues,
- * the CUDA-core engine otherwise (captured in place, it stages in the plan's own
- * buffer: order those calls).  The queue route keeps up to eight prepared queues
- * per plan (one per source, destination, count, direction), each with its own
- * workspace ring of up to 16 x N words. */
+ * plans.  Its in-place calls above 2^13 stage a pass in a workspace of the plan's:
+ * one for each of the first four streams, then one per call, in stream order;
+ * one of each graph's own where the stream is captured (held until the graph and
+ * its executables are destroyed).  Streams, threads and graphs may share a plan.
+ * Where that memory cannot be had, and for the drop-in's uint64 words and the host
+ * stream, AUTO takes the INT8 tensor-core kernel at N = 2^16 from 8 (polynomial,
+ * limb) units on, the batch queue at N = 2^17 .. 2^20 once a call holds 2^20
+ * residues, the CUDA-core engine otherwise.  The INT8 kernel's tables and the
+ * queues are built on first use: call once before a capture.  The queue route
+ * keeps up to eight prepared queues per plan (one per source, destination, count,
+ * direction), each with its own workspace ring of up to 16 x N words.  Destroying
+ * a plan waits for its calls. */
 enum {
     NTTB_ENGINE_AUTO = 0,
     NTTB_ENGINE_SCALAR = 1, /* CUDA-core radix-2 stages in registers and shared memory */

@@ -624,7 +624,7 @@ int nttb_rns_transform(const nttb_rns_plan* P, uint32_t* dst, const uint32_t* sr
     Plan32& p = const_cast<Plan32&>(P->p);
     cudaStream_t s = (cudaStream_t)stream;
     int rc = kNoWorkspace;
-    if (auto_radix32(p, (uint64_t)n_polys * p.n_limbs, engine, s))
+    if (auto_radix32(p, (uint64_t)n_polys * p.n_limbs, engine))
         rc = scalar_transform32(p, src, dst, false, n_polys, inverse != 0, s);
     if (rc == kNoWorkspace) rc = run_transform32(p, src, dst, false, n_polys, inverse != 0, engine, s);
     return engine_status(rc, "rns_transform");
@@ -638,7 +638,7 @@ int nttb_rns_forward_inverse(const nttb_rns_plan* P, uint32_t* d, uint32_t n_pol
     cudaStream_t s = (cudaStream_t)stream;
     const uint64_t units = (uint64_t)n_polys * p.n_limbs;
     int rc = kNoWorkspace;
-    if (auto_radix32(p, units, engine, s) || (engine == NTTB_ENGINE_SCALAR && radix_serves(p.log_n)))
+    if (auto_radix32(p, units, engine) || (engine == NTTB_ENGINE_SCALAR && radix_serves(p.log_n)))
         rc = scalar_round_trip32(p, d, n_polys, s);
     if (rc != kNoWorkspace) return engine_status(rc, "rns_forward_inverse");
     if ((engine == NTTB_ENGINE_AUTO ? auto_engine32(p, false, units, true) : engine) == NTTB_ENGINE_INT8) {

@@ -21,11 +21,11 @@ static int env_engine() {
 // every size (us, forward, this engine / the other): 8 x 2^16 6.6 / 16.6 (INT8),
 // 24 x 2^16 9.7 / 17.4 (INT8), 192 x 2^16 54 / 95 (INT8), 33 x 2^17 22.5 / 62
 // (tensor tiles), 1 x 2^20 10 / 25 (queue).  In place they stage their first pass
-// in a workspace; calls that must not need one (it could not be had, or the
-// stream is captured) and the drop-in's and the host stream's calls, whose
-// engines those entry points name, take the INT8 cluster kernel at 2^16 from
-// kInt8MinUnits (polynomial, limb) units on and the batch queue at 2^17 .. 2^20
-// once a call holds 2^20 residues (each prepared queue has a ring of its own).
+// in a workspace; calls for which it could not be had and the drop-in's and the
+// host stream's calls, whose engines those entry points name, take the INT8
+// cluster kernel at 2^16 from kInt8MinUnits (polynomial, limb) units on and the
+// batch queue at 2^17 .. 2^20 once a call holds 2^20 residues (each prepared queue
+// has a ring of its own).
 constexpr uint64_t kInt8MinUnits = 8;
 constexpr uint32_t kTilesMinLog = 17;
 constexpr uint64_t kTilesMinResidues = 1ull << 20;
@@ -37,9 +37,9 @@ int auto_engine32(const Plan32& p, bool src_u64, uint64_t units, bool in_place) 
     return NTTB_ENGINE_SCALAR;
 }
 
-bool auto_radix32(const Plan32& p, uint64_t units, int engine, cudaStream_t s) {
+bool auto_radix32(const Plan32& p, uint64_t units, int engine) {
     return engine == NTTB_ENGINE_AUTO && env_engine() == NTTB_ENGINE_AUTO && radix_serves(p.log_n) &&
-           scalar_serves(p, units) && (p.log_n <= kRadixSingleMax || !stream_capturing(s));
+           scalar_serves(p, units);
 }
 
 int run_transform32(Plan32& p, const void* src, void* dst, bool src_u64, uint32_t n_polys, bool inverse,

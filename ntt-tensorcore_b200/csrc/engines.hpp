@@ -19,7 +19,7 @@ int auto_engine32(const Plan32& p, bool src_u64, uint64_t units, bool in_place);
 
 // Whether an RNS call with this engine argument runs the register-radix passes,
 // in place too; if they then return kNoWorkspace, AUTO's other engines take it.
-bool auto_radix32(const Plan32& p, uint64_t units, int engine, cudaStream_t s);
+bool auto_radix32(const Plan32& p, uint64_t units, int engine);
 
 // Frees engine caches attached to a plan.
 void engines_release32(Plan32* p);

@@ -223,15 +223,6 @@ void* plan_workspace(void** ws, size_t* ws_bytes, size_t bytes) {
     return *ws;
 }
 
-bool stream_capturing(cudaStream_t s) {
-    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(s, &st) != cudaSuccess) {
-        cudaGetLastError();  // the legacy stream while another stream is captured
-        return true;
-    }
-    return st != cudaStreamCaptureStatusNone;
-}
-
 static cudaMemPool_t plan_pool(PlanPool& pp) {  // pp.mu held
     if (pp.tried) return pp.pool;
     pp.tried = true;
@@ -251,13 +242,82 @@ static cudaMemPool_t plan_pool(PlanPool& pp) {  // pp.mu held
     return pp.pool;
 }
 
-StreamWorkspace::StreamWorkspace(PlanPool& pp, void** ws, size_t* ws_bytes, size_t bytes, cudaStream_t s)
-    : lock_(pp.mu), stream_(s) {
-    unsigned long long id = 0;
-    if (stream_capturing(s) || !plan_pool(pp) || cudaStreamGetId(s, &id) != cudaSuccess) {
+namespace {
+struct GraphRef {
+    std::shared_ptr<GraphWorkspaces> all;
+    GraphWorkspaces::Buf* buf;
+};
+void CUDART_CB drop_graph_ref(void* p) {  // no CUDA calls here
+    GraphRef* r = static_cast<GraphRef*>(p);
+    {
+        std::lock_guard<std::mutex> lock(r->all->mu);
+        r->buf->held = false;
+    }
+    delete r;
+}
+}  // namespace
+
+// A workspace of the graph that `s` is being captured into: calls captured on one
+// stream of one capture run one after the other and share it.  The stream's handle
+// stands for it, which does not change hands during a capture (the per-thread
+// handle is one of several streams; cudaStreamGetId invalidates a capture).
+static void* graph_workspace(const std::shared_ptr<GraphWorkspaces>& all, size_t bytes, unsigned long long capture,
+                             cudaGraph_t graph, cudaStream_t stream) {
+    GraphWorkspaces::Buf* b = nullptr;
+    {
+        std::lock_guard<std::mutex> lock(all->mu);
+        for (GraphWorkspaces::Buf& t : all->bufs) {
+            if (t.bytes < bytes) continue;
+            if (t.held && t.capture == capture && t.stream == stream && stream != cudaStreamPerThread) return t.ptr;
+            if (!t.held && (!b || t.bytes < b->bytes)) b = &t;
+        }
+        if (b) b->held = true;
+    }
+    if (!b) {
+        // no capture depends on the allocation: it may be made in the middle of one
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        void* ptr = nullptr;
+        const cudaError_t e = cudaMalloc(&ptr, bytes);
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        if (e != cudaSuccess) return nullptr;
+        std::lock_guard<std::mutex> lock(all->mu);
+        all->bufs.emplace_back();
+        b = &all->bufs.back();
+        b->ptr = ptr;
+        b->bytes = bytes;
+        b->held = true;
+    }
+    b->capture = capture;
+    b->stream = stream;
+    GraphRef* ref = new GraphRef{all, b};
+    cudaUserObject_t obj = nullptr;
+    if (cudaUserObjectCreate(&obj, ref, drop_graph_ref, 1, cudaUserObjectNoDestructorSync) != cudaSuccess) {
+        drop_graph_ref(ref);
+        return nullptr;
+    }
+    if (cudaGraphRetainUserObject(graph, obj, 1, cudaGraphUserObjectMove) != cudaSuccess) {
+        cudaUserObjectRelease(obj, 1);
+        return nullptr;
+    }
+    return b->ptr;
+}
+
+StreamWorkspace::StreamWorkspace(PlanPool& pp, size_t bytes, cudaStream_t s) : lock_(pp.mu), stream_(s) {
+    unsigned long long id = 0, capture = 0;
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    cudaGraph_t graph = nullptr;
+    if (cudaStreamGetCaptureInfo(s, &status, &capture, &graph) != cudaSuccess) {
         cudaGetLastError();
-        ptr = plan_workspace(ws, ws_bytes, bytes);
+        return;
+    }
+    if (status != cudaStreamCaptureStatusNone) {
+        if (status == cudaStreamCaptureStatusActive) ptr = graph_workspace(pp.graphs, bytes, capture, graph, s);
         if (!ptr) cudaGetLastError();
+        return;
+    }
+    if (!plan_pool(pp) || cudaStreamGetId(s, &id) != cudaSuccess) {
+        cudaGetLastError();
         return;
     }
     PlanPool::Slot* slot = nullptr;
@@ -290,7 +350,15 @@ StreamWorkspace::~StreamWorkspace() {
 }
 
 static void free_pool(PlanPool& pp) {
-    if (!pp.pool) return;  // no call has staged anything
+    {
+        std::lock_guard<std::mutex> lock(pp.graphs->mu);
+        for (GraphWorkspaces::Buf& b : pp.graphs->bufs) {
+            if (b.ptr) cudaFree(b.ptr);
+            b.ptr = nullptr;
+            b.bytes = 0;
+        }
+    }
+    if (!pp.pool) return;  // no call has staged anything outside a capture
     // cudaFree of stream-ordered memory does not wait for the calls that still use
     // it, as that of cudaMalloc's does: wait for them here.  Where the device cannot
     // be waited for, the memory stays allocated.

@@ -3,6 +3,8 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <list>
+#include <memory>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -77,6 +79,21 @@ struct PassArgs {
     int inverse;
 };
 
+// Workspaces of captured calls.  A graph holds its own until it and what was
+// instantiated from it are gone; then the next capture may take them.  The plan
+// frees them, and the graphs' references may outlive it.
+struct GraphWorkspaces {
+    struct Buf {
+        void* ptr = nullptr;
+        size_t bytes = 0;
+        unsigned long long capture = 0;  // the calls that share it: one stream of one capture
+        cudaStream_t stream = nullptr;
+        bool held = false;
+    };
+    std::mutex mu;
+    std::list<Buf> bufs;
+};
+
 // The pool behind a plan's stream-ordered workspaces (StreamWorkspace), and the
 // workspaces that the first kSlots streams keep.
 struct PlanPool {
@@ -91,6 +108,7 @@ struct PlanPool {
     bool tried = false;
     Slot slot[kSlots];
     std::mutex mu;
+    std::shared_ptr<GraphWorkspaces> graphs = std::make_shared<GraphWorkspaces>();
 };
 
 // A u32-residue plan (q < 2^31 for every limb).
@@ -102,7 +120,7 @@ struct Plan32 {
     std::vector<void*> allocations;   // device memory owned by the plan
     void* engine_data[4] = {nullptr, nullptr, nullptr, nullptr};  // per-engine host-side caches
     std::mutex engine_mu;             // guards the lazy construction of engine_data
-    void* ws = nullptr;               // workspace for in-place multi-pass transforms
+    void* ws = nullptr;               // plan_workspace's buffer
     size_t ws_bytes = 0;
     PlanPool pool;                    // stream-ordered workspaces (StreamWorkspace)
     int device = -1;                  // the CUDA device holding d_limbs and the tables
@@ -140,12 +158,12 @@ int engine_status(int rc, const char* what);
 // so that threads on one stream enqueue one after the other.  Further streams
 // allocate per call.  So calls on several streams or threads never share one.
 // The pool keeps what its calls needed at once, until the plan is destroyed.
-// While the stream is being captured, and where there is no pool, it is the
-// plan's own buffer (plan_workspace), whose calls must be ordered.  ptr: null on
-// failure.
+// While the stream is being captured it is a buffer that the graph holds
+// (GraphWorkspaces), so that a captured call needs no earlier one and replays race
+// neither with other graphs nor with calls outside.  ptr: null on failure.
 class StreamWorkspace {
 public:
-    StreamWorkspace(PlanPool& pool, void** ws, size_t* ws_bytes, size_t bytes, cudaStream_t s);
+    StreamWorkspace(PlanPool& pool, size_t bytes, cudaStream_t s);
     ~StreamWorkspace();
     StreamWorkspace(const StreamWorkspace&) = delete;
     void* ptr = nullptr;
@@ -155,12 +173,11 @@ private:
     cudaStream_t stream_;
     bool per_call_ = false;
 };
-bool stream_capturing(cudaStream_t s);
 // scalar_transform32's and scalar_transform64's status when the workspace could not be had.
 constexpr int kNoWorkspace = 3;
 
 // Returns a device workspace of at least `bytes`, growing the plan's buffer
-// (an in-place multi-pass transform stages its first pass there).  Calls
+// (the DMMA and the INT8 wide engine stage their first pass there).  Calls
 // that share a plan must be ordered on one stream while they use it.
 void* plan_workspace(void** ws, size_t* ws_bytes, size_t bytes);
 

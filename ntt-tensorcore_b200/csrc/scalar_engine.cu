@@ -391,7 +391,7 @@ int scalar_transform32(Plan32& p, const void* src, void* dst, bool src_u64, uint
     const bool radix = radix_serves(p.log_n);
     const size_t words = staged_words(p.log_n, 8192, p.n_limbs, n_polys);
     if (!words || (src != dst && !(radix && src_u64))) return run32(p, src, dst, dst, src_u64, n_polys, inverse, s);
-    StreamWorkspace ws(p.pool, &p.ws, &p.ws_bytes, words * (src_u64 && !radix ? 8 : 4), s);
+    StreamWorkspace ws(p.pool, words * (src_u64 && !radix ? 8 : 4), s);
     if (!ws.ptr) return kNoWorkspace;
     return run32(p, src, dst, ws.ptr, src_u64, n_polys, inverse, s);
 }
@@ -400,7 +400,7 @@ int scalar_round_trip32(Plan32& p, uint32_t* data, uint32_t n_polys, cudaStream_
     if (!radix_serves(p.log_n) || n_polys > 65535 || p.n_limbs > 65535) return 1;
     const size_t words = staged_words(p.log_n, 8192, p.n_limbs, n_polys);
     if (!words) return radix_round_trip_u32(p, data, nullptr, n_polys, s);
-    StreamWorkspace ws(p.pool, &p.ws, &p.ws_bytes, words * 4, s);
+    StreamWorkspace ws(p.pool, words * 4, s);
     if (!ws.ptr) return kNoWorkspace;
     return radix_round_trip_u32(p, data, ws.ptr, n_polys, s);
 }
@@ -426,7 +426,7 @@ int scalar_transform64(Plan64& p, const void* src, void* dst, uint32_t n_polys, 
     if (n_polys > 65535 || p.n_limbs > 65535) return 1;
     const size_t words = staged_words(p.log_n, 4096, p.n_limbs, n_polys);
     if (!words || src != dst) return run64(p, src, dst, dst, n_polys, inverse, s);
-    StreamWorkspace ws(p.pool, &p.ws, &p.ws_bytes, words * 8, s);
+    StreamWorkspace ws(p.pool, words * 8, s);
     if (!ws.ptr) return kNoWorkspace;
     return run64(p, src, dst, ws.ptr, n_polys, inverse, s);
 }
