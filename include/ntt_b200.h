@@ -43,7 +43,8 @@ enum {
  * plans.  Its in-place calls above 2^13 stage a pass in a workspace of the plan's:
  * one for each of the first four streams, then one per call, in stream order;
  * one of each graph's own where the stream is captured (held until the graph and
- * its executables are destroyed).  Streams, threads and graphs may share a plan.
+ * its executables are destroyed).  Each is at most 2^25 words (or one row): longer
+ * calls run in groups of rows.  Streams, threads and graphs may share a plan.
  * Where that memory cannot be had, and for the drop-in's uint64 words and the host
  * stream, AUTO takes the INT8 tensor-core kernel at N = 2^16 from 8 (polynomial,
  * limb) units on, the batch queue at N = 2^17 .. 2^20 once a call holds 2^20

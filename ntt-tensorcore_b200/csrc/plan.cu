@@ -235,7 +235,8 @@ static cudaMemPool_t plan_pool(PlanPool& pp) {  // pp.mu held
         return nullptr;
     }
     pp.device = props.location.id;
-    uint64_t keep = ~0ull;  // what one call frees, the next takes; the pool goes with the plan
+    // what one call frees, the next takes; the pool goes with the plan
+    uint64_t keep = 2 * PlanPool::kSlots * kStagedWordsMax * 8;
     int off = 0;            // streams never wait for one another for memory
     cudaMemPoolSetAttribute(pp.pool, cudaMemPoolAttrReleaseThreshold, &keep);
     cudaMemPoolSetAttribute(pp.pool, cudaMemPoolReuseAllowInternalDependencies, &off);

@@ -157,7 +157,8 @@ int engine_status(int rc, const char* what);
 // call 2 us on the host: in place 1 x 2^16 6.3 -> 8.7 us); it is locked meanwhile,
 // so that threads on one stream enqueue one after the other.  Further streams
 // allocate per call.  So calls on several streams or threads never share one.
-// The pool keeps what its calls needed at once, until the plan is destroyed.
+// The pool keeps what kSlots streams and as many calls beyond them need
+// (kStagedWordsMax each) until the plan is destroyed, and gives back the rest.
 // While the stream is being captured it is a buffer that the graph holds
 // (GraphWorkspaces), so that a captured call needs no earlier one and replays race
 // neither with other graphs nor with calls outside.  ptr: null on failure.
@@ -205,16 +206,42 @@ int scalar_transform32_ws(const Plan32& p, uint32_t* data, void* ws, uint32_t n_
 // (0 when the shape runs as one pass and stages nothing).
 size_t scalar_transform32_ws_bytes(const Plan32& p, uint32_t n_polys);
 
-// Register-radix passes on CUDA cores (radix.cuh): sizes 2^5 .. 2^20.  Sizes
-// above 2^13 run two passes through `mid`, n_polys * n_limbs * n words (uint32
-// for the 31-bit plans, uint64 for the wide ones): the destination, if the
-// source is another buffer and the words have its size, or a workspace.
+// Register-radix passes on CUDA cores (radix.cuh): sizes 2^5 .. 2^20, n_polys x
+// n_limbs rows under the moduli `limbs`.  Sizes above 2^13 run two passes through
+// `mid`, n_polys * n_limbs * n words (uint32 for the 31-bit moduli, uint64 for the
+// wide ones): the destination, if the source is another buffer and the words have
+// its size, or a workspace.
 constexpr uint32_t kRadixMinLog = 5, kRadixMaxLog = 20, kRadixSingleMax = 13;
 inline bool radix_serves(uint32_t log_n) { return log_n >= kRadixMinLog && log_n <= kRadixMaxLog; }
-int radix_u32(const Plan32& p, const void* src, void* dst, void* mid, uint32_t n_polys, bool inverse, cudaStream_t s);
-int radix_round_trip_u32(const Plan32& p, uint32_t* data, void* mid, uint32_t n_polys, cudaStream_t s);
-int radix_w64(const Plan32& p, const void* src, void* dst, void* mid, uint32_t n_polys, bool inverse, cudaStream_t s);
-int radix_q64(const Plan64& p, const void* src, void* dst, void* mid, uint32_t n_polys, bool inverse, cudaStream_t s);
+int radix_u32(const LimbDev<M32>* limbs, uint32_t log_n, uint32_t n_limbs, const void* src, void* dst, void* mid,
+              uint32_t n_polys, bool inverse, cudaStream_t s);
+int radix_round_trip_u32(const LimbDev<M32>* limbs, uint32_t log_n, uint32_t n_limbs, uint32_t* data, void* mid,
+                         uint32_t n_polys, cudaStream_t s);
+int radix_w64(const LimbDev<M32>* limbs, uint32_t log_n, uint32_t n_limbs, const void* src, void* dst, void* mid,
+              uint32_t n_polys, bool inverse, cudaStream_t s);
+int radix_q64(const LimbDev<M64>* limbs, uint32_t log_n, uint32_t n_limbs, const void* src, void* dst, void* mid,
+              uint32_t n_polys, bool inverse, cudaStream_t s);
+
+// Rows that a call stages at a time: 2^25 words, or one row where that is larger.
+// Longer calls run their rows in groups of that, one after the other, so that what a
+// plan holds for a stream does not grow with the call.  A group pays for its last
+// waves and shares roots among fewer polynomials; us in place at 2^24 / 2^25 words /
+// one group: 64 x 24 x 2^16 448 / 425 / 385, 8 x 30 x 2^18 347 / 328 / 304, round
+// trip 16 x 24 x 2^16 198 / 187 / 187, 64-bit 20 x 2^20 378 / 362 / 364.
+constexpr uint64_t kStagedWordsMax = 1ull << 25;
+struct RowGroups {
+    uint32_t polys, limbs;  // per group; limbs < the plan's: groups lie within one polynomial
+};
+inline RowGroups row_groups(uint32_t log_n, uint32_t n_limbs, uint32_t n_polys) {
+    const uint64_t most = kStagedWordsMax >> log_n > 0 ? kStagedWordsMax >> log_n : 1;
+    // groups of even size: the last one is not a remainder of a few rows
+    auto even = [](uint64_t total, uint64_t per) {
+        const uint64_t k = (total + per - 1) / per;
+        return (uint32_t)((total + k - 1) / k);
+    };
+    if (n_limbs <= most) return {even(n_polys, most / n_limbs), n_limbs};
+    return {1, even(n_limbs, most)};
+}
 
 // INT8 tensor-core engine for the wide plans (tc_wide.cu): n = 2^20, cyclic,
 // moduli below 2^62 on byte planes of uint64 words.  Returns 1 when the plan

@@ -3,8 +3,9 @@
 
 namespace nttb {
 
-int radix_q64(const Plan64& p, const void* src, void* dst, void* mid, uint32_t n_polys, bool inverse, cudaStream_t s) {
-    return rdx::transform<M64, uint64_t, uint64_t, 3>(p.d_limbs, p.log_n, p.n_limbs, src, dst, mid, n_polys, inverse, s);
+int radix_q64(const LimbDev<M64>* limbs, uint32_t log_n, uint32_t n_limbs, const void* src, void* dst, void* mid,
+              uint32_t n_polys, bool inverse, cudaStream_t s) {
+    return rdx::transform<M64, uint64_t, uint64_t, 3>(limbs, log_n, n_limbs, src, dst, mid, n_polys, inverse, s);
 }
 
 }  // namespace nttb

@@ -4,8 +4,9 @@
 
 namespace nttb {
 
-int radix_w64(const Plan32& p, const void* src, void* dst, void* mid, uint32_t n_polys, bool inverse, cudaStream_t s) {
-    return rdx::transform<M32, uint64_t, uint32_t, 4>(p.d_limbs, p.log_n, p.n_limbs, src, dst, mid, n_polys, inverse, s);
+int radix_w64(const LimbDev<M32>* limbs, uint32_t log_n, uint32_t n_limbs, const void* src, void* dst, void* mid,
+              uint32_t n_polys, bool inverse, cudaStream_t s) {
+    return rdx::transform<M32, uint64_t, uint32_t, 4>(limbs, log_n, n_limbs, src, dst, mid, n_polys, inverse, s);
 }
 
 }  // namespace nttb

@@ -375,14 +375,31 @@ static size_t staged_words(uint32_t log_n, uint32_t e_max, uint32_t n_limbs, uin
     return two ? ((size_t)n_polys * n_limbs) << log_n : 0;
 }
 
-static int run32(Plan32& p, const void* src, void* dst, void* mid, bool src_u64, uint32_t n_polys, bool inverse,
-                 cudaStream_t s) {
-    if (radix_serves(p.log_n)) return (src_u64 ? radix_w64 : radix_u32)(p, src, dst, mid, n_polys, inverse, s);
+static int run32(const LimbDev<M32>* limbs, uint32_t log_n, uint32_t n_limbs, bool negacyclic, const void* src,
+                 void* dst, void* mid, bool src_u64, uint32_t n_polys, bool inverse, cudaStream_t s) {
+    if (radix_serves(log_n))
+        return (src_u64 ? radix_w64 : radix_u32)(limbs, log_n, n_limbs, src, dst, mid, n_polys, inverse, s);
     if (src_u64)
-        return transform_generic<uint64_t, M32>(p.log_n, p.n_limbs, p.negacyclic, p.d_limbs, src, dst, mid, n_polys,
-                                                inverse, 8192, s);
-    return transform_generic<uint32_t, M32>(p.log_n, p.n_limbs, p.negacyclic, p.d_limbs, src, dst, mid, n_polys,
-                                            inverse, 8192, s);
+        return transform_generic<uint64_t, M32>(log_n, n_limbs, negacyclic, limbs, src, dst, mid, n_polys, inverse,
+                                                8192, s);
+    return transform_generic<uint32_t, M32>(log_n, n_limbs, negacyclic, limbs, src, dst, mid, n_polys, inverse, 8192,
+                                            s);
+}
+
+// Runs run(limbs, n_limbs, word offset, n_polys, workspace) over the call's groups
+// of rows, with one workspace of `word` bytes per staged word for all of them.
+template <class PlanT, class Run>
+static int staged_groups(PlanT& p, uint32_t n_polys, size_t word, cudaStream_t s, Run run) {
+    const RowGroups g = row_groups(p.log_n, p.n_limbs, n_polys);
+    StreamWorkspace ws(p.pool, (((size_t)g.polys * g.limbs) << p.log_n) * word, s);
+    if (!ws.ptr) return kNoWorkspace;
+    for (uint32_t poly = 0; poly < n_polys; poly += g.polys)
+        for (uint32_t limb = 0; limb < p.n_limbs; limb += g.limbs) {
+            const uint32_t nl = p.n_limbs - limb < g.limbs ? p.n_limbs - limb : g.limbs;
+            const uint32_t np = n_polys - poly < g.polys ? n_polys - poly : g.polys;
+            if (int rc = run(p.d_limbs + limb, nl, (((size_t)poly * p.n_limbs) + limb) << p.log_n, np, ws.ptr)) return rc;
+        }
+    return 0;
 }
 
 int scalar_transform32(Plan32& p, const void* src, void* dst, bool src_u64, uint32_t n_polys, bool inverse,
@@ -390,24 +407,30 @@ int scalar_transform32(Plan32& p, const void* src, void* dst, bool src_u64, uint
     if (n_polys > 65535 || p.n_limbs > 65535) return 1;
     const bool radix = radix_serves(p.log_n);
     const size_t words = staged_words(p.log_n, 8192, p.n_limbs, n_polys);
-    if (!words || (src != dst && !(radix && src_u64))) return run32(p, src, dst, dst, src_u64, n_polys, inverse, s);
-    StreamWorkspace ws(p.pool, words * (src_u64 && !radix ? 8 : 4), s);
-    if (!ws.ptr) return kNoWorkspace;
-    return run32(p, src, dst, ws.ptr, src_u64, n_polys, inverse, s);
+    if (!words || (src != dst && !(radix && src_u64)))
+        return run32(p.d_limbs, p.log_n, p.n_limbs, p.negacyclic, src, dst, dst, src_u64, n_polys, inverse, s);
+    const size_t es = src_u64 ? 8 : 4;
+    return staged_groups(p, n_polys, radix ? 4 : es, s,
+                         [&](const LimbDev<M32>* limbs, uint32_t n_limbs, size_t off, uint32_t polys, void* mid) {
+                             return run32(limbs, p.log_n, n_limbs, p.negacyclic, static_cast<const char*>(src) + off * es,
+                                          static_cast<char*>(dst) + off * es, mid, src_u64, polys, inverse, s);
+                         });
 }
 
 int scalar_round_trip32(Plan32& p, uint32_t* data, uint32_t n_polys, cudaStream_t s) {
     if (!radix_serves(p.log_n) || n_polys > 65535 || p.n_limbs > 65535) return 1;
-    const size_t words = staged_words(p.log_n, 8192, p.n_limbs, n_polys);
-    if (!words) return radix_round_trip_u32(p, data, nullptr, n_polys, s);
-    StreamWorkspace ws(p.pool, words * 4, s);
-    if (!ws.ptr) return kNoWorkspace;
-    return radix_round_trip_u32(p, data, ws.ptr, n_polys, s);
+    if (!staged_words(p.log_n, 8192, p.n_limbs, n_polys))
+        return radix_round_trip_u32(p.d_limbs, p.log_n, p.n_limbs, data, nullptr, n_polys, s);
+    return staged_groups(p, n_polys, 4, s,
+                         [&](const LimbDev<M32>* limbs, uint32_t n_limbs, size_t off, uint32_t polys, void* mid) {
+                             return radix_round_trip_u32(limbs, p.log_n, n_limbs, data + off, mid, polys, s);
+                         });
 }
 
 int scalar_transform32_ws(const Plan32& p, uint32_t* data, void* ws, uint32_t n_polys, bool inverse,
                           cudaStream_t s) {
-    if (radix_serves(p.log_n)) return p.n_limbs > 65535 ? 1 : radix_u32(p, data, data, ws, n_polys, inverse, s);
+    if (radix_serves(p.log_n))
+        return p.n_limbs > 65535 ? 1 : radix_u32(p.d_limbs, p.log_n, p.n_limbs, data, data, ws, n_polys, inverse, s);
     return transform_generic<uint32_t, M32>(p.log_n, p.n_limbs, p.negacyclic, p.d_limbs, data, data, ws, n_polys,
                                             inverse, 8192, s);
 }
@@ -416,19 +439,24 @@ size_t scalar_transform32_ws_bytes(const Plan32& p, uint32_t n_polys) {
     return staged_words(p.log_n, 8192, p.n_limbs, n_polys) * sizeof(uint32_t);
 }
 
-static int run64(Plan64& p, const void* src, void* dst, void* mid, uint32_t n_polys, bool inverse, cudaStream_t s) {
-    if (radix_serves(p.log_n)) return radix_q64(p, src, dst, mid, n_polys, inverse, s);
-    return transform_generic<uint64_t, M64>(p.log_n, p.n_limbs, p.negacyclic, p.d_limbs, src, dst, mid, n_polys,
-                                            inverse, 4096, s);
+static int run64(const LimbDev<M64>* limbs, uint32_t log_n, uint32_t n_limbs, bool negacyclic, const uint64_t* src,
+                 uint64_t* dst, void* mid, uint32_t n_polys, bool inverse, cudaStream_t s) {
+    if (radix_serves(log_n)) return radix_q64(limbs, log_n, n_limbs, src, dst, mid, n_polys, inverse, s);
+    return transform_generic<uint64_t, M64>(log_n, n_limbs, negacyclic, limbs, src, dst, mid, n_polys, inverse, 4096,
+                                            s);
 }
 
-int scalar_transform64(Plan64& p, const void* src, void* dst, uint32_t n_polys, bool inverse, cudaStream_t s) {
+int scalar_transform64(Plan64& p, const void* src_, void* dst_, uint32_t n_polys, bool inverse, cudaStream_t s) {
     if (n_polys > 65535 || p.n_limbs > 65535) return 1;
-    const size_t words = staged_words(p.log_n, 4096, p.n_limbs, n_polys);
-    if (!words || src != dst) return run64(p, src, dst, dst, n_polys, inverse, s);
-    StreamWorkspace ws(p.pool, words * 8, s);
-    if (!ws.ptr) return kNoWorkspace;
-    return run64(p, src, dst, ws.ptr, n_polys, inverse, s);
+    const uint64_t* src = static_cast<const uint64_t*>(src_);
+    uint64_t* dst = static_cast<uint64_t*>(dst_);
+    if (!staged_words(p.log_n, 4096, p.n_limbs, n_polys) || src != dst)
+        return run64(p.d_limbs, p.log_n, p.n_limbs, p.negacyclic, src, dst, dst, n_polys, inverse, s);
+    return staged_groups(p, n_polys, 8, s,
+                         [&](const LimbDev<M64>* limbs, uint32_t n_limbs, size_t off, uint32_t polys, void* mid) {
+                             return run64(limbs, p.log_n, n_limbs, p.negacyclic, src + off, dst + off, mid, polys,
+                                          inverse, s);
+                         });
 }
 
 // The RowMaj pre-transposed layout pre[b*M + a] = x[a*M + b] for n = M^2
