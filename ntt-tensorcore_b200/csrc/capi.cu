@@ -641,11 +641,13 @@ int nttb_rns_forward_inverse(const nttb_rns_plan* P, uint32_t* d, uint32_t n_pol
     if (auto_radix32(p, units, engine) || (engine == NTTB_ENGINE_SCALAR && radix_serves(p.log_n)))
         rc = scalar_round_trip32(p, d, n_polys, s);
     if (rc != kNoWorkspace) return engine_status(rc, "rns_forward_inverse");
-    if ((engine == NTTB_ENGINE_AUTO ? auto_engine32(p, false, units, true) : engine) == NTTB_ENGINE_INT8) {
+    const bool named = engine != NTTB_ENGINE_AUTO;
+    if (!named) engine = auto_engine32(p, false, units, true);
+    if (engine == NTTB_ENGINE_INT8) {
         rc = int8_forward_inverse32(p, d, n_polys, s);
     } else {
-        rc = run_transform32(p, d, d, false, n_polys, false, engine, s);
-        if (!rc) rc = run_transform32(p, d, d, false, n_polys, true, engine, s);
+        rc = run_engine32(p, d, d, false, n_polys, false, engine, named, s);
+        if (!rc) rc = run_engine32(p, d, d, false, n_polys, true, engine, named, s);
     }
     return engine_status(rc, "rns_forward_inverse");
 }
@@ -658,7 +660,8 @@ int nttb_rns_stream_host(nttb_rns_plan* P, const uint32_t* h_src, uint32_t* h_ds
     Plan32& p = P->p;
     cudaStream_t s = (cudaStream_t)stream;
     const size_t bw = (size_t)n_polys * p.n_limbs * p.n;
-    const int eng = engine == NTTB_ENGINE_AUTO ? auto_engine32(p, false, (uint64_t)n_polys * p.n_limbs, true) : engine;
+    const bool named = engine != NTTB_ENGINE_AUTO;
+    const int eng = named ? engine : auto_engine32(p, false, (uint64_t)n_polys * p.n_limbs, true);
     nttb::HostStream*& H = P->hs;
     if (!H || H->words < bw) {  // (re)build the buffers, streams and events
         nttb::host_stream_free(H);
@@ -709,11 +712,11 @@ int nttb_rns_stream_host(nttb_rns_plan* P, const uint32_t* h_src, uint32_t* h_ds
         int rc = 0;
         if (mode == 2) {
             rc = eng == NTTB_ENGINE_INT8 ? int8_forward_inverse32(p, H->dbuf[k], n_polys, s)
-                                         : run_transform32(p, H->dbuf[k], H->dbuf[k], false, n_polys, false, engine, s);
+                                         : run_engine32(p, H->dbuf[k], H->dbuf[k], false, n_polys, false, eng, named, s);
             if (!rc && eng != NTTB_ENGINE_INT8)
-                rc = run_transform32(p, H->dbuf[k], H->dbuf[k], false, n_polys, true, engine, s);
+                rc = run_engine32(p, H->dbuf[k], H->dbuf[k], false, n_polys, true, eng, named, s);
         } else {
-            rc = run_transform32(p, H->dbuf[k], H->dbuf[k], false, n_polys, mode == 1, engine, s);
+            rc = run_engine32(p, H->dbuf[k], H->dbuf[k], false, n_polys, mode == 1, eng, named, s);
         }
         if (rc) return engine_status(rc, "rns_stream_host");
         cudaEventRecord(H->ev_c[k], s);

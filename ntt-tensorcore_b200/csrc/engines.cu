@@ -47,6 +47,11 @@ int run_transform32(Plan32& p, const void* src, void* dst, bool src_u64, uint32_
     if (engine == NTTB_ENGINE_AUTO) engine = env_engine();
     const bool named = engine != NTTB_ENGINE_AUTO;
     if (!named) engine = auto_engine32(p, src_u64, (uint64_t)n_polys * p.n_limbs, src == dst);
+    return run_engine32(p, src, dst, src_u64, n_polys, inverse, engine, named, s);
+}
+
+int run_engine32(Plan32& p, const void* src, void* dst, bool src_u64, uint32_t n_polys, bool inverse, int engine,
+                 bool named, cudaStream_t s) {
     switch (engine) {
         case NTTB_ENGINE_SCALAR:
             return scalar_transform32(p, src, dst, src_u64, n_polys, inverse, s);

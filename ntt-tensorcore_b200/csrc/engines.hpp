@@ -14,6 +14,11 @@ namespace nttb {
 int run_transform32(Plan32& p, const void* src, void* dst, bool src_u64, uint32_t n_polys, bool inverse,
                     int engine, cudaStream_t s);
 
+// The same on `engine` (not AUTO); `named`: the caller asked for it, else AUTO
+// resolved to it.
+int run_engine32(Plan32& p, const void* src, void* dst, bool src_u64, uint32_t n_polys, bool inverse, int engine,
+                 bool named, cudaStream_t s);
+
 // Which engine AUTO resolves to for this plan (NTTB_ENGINE_*).
 int auto_engine32(const Plan32& p, bool src_u64, uint64_t units, bool in_place);
 
