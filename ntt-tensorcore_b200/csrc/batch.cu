@@ -1505,6 +1505,14 @@ bool ensure_images(BatchPlan& P) {
     return true;
 }
 
+// Sizes of the register-radix tiles' root tables, per kind of root: quotients of
+// the roots up to 2^log_r and pairs of those up to 2^log_p for each modulus.
+uint32_t root_log_r(const BatchPlan& P) { return std::min(P.max_log, kRxMaxLog); }
+uint32_t root_log_p(const BatchPlan& P) { return std::min(P.max_log, kRxMaxLog / 2); }
+size_t root_bytes(const BatchPlan& P, size_t nm) {
+    return (nm << root_log_p(P)) * sizeof(uint2) + (nm << root_log_r(P)) * sizeof(uint32_t);
+}
+
 // Device tables of the register-radix tiles for one kind of root (bit 0
 // inverse, bit 1 negacyclic), made on first use: per modulus 4 bytes per root
 // up to 2^min(max_log, 20) and 8 per root up to 2^10 (the uniform passes').
@@ -1536,11 +1544,11 @@ bool ensure_roots(BatchPlan& P, uint32_t kind) {
         }
     }
     if (M.rx_host[0].quot[kind]) return true;
-    const uint32_t log_r = std::min(P.max_log, kRxMaxLog), log_p = std::min(P.max_log, kRxMaxLog / 2);
+    const uint32_t log_r = root_log_r(P), log_p = root_log_p(P);
     uint2* pairs = nullptr;
     uint32_t* quot = nullptr;
-    const size_t pair_bytes = (nm << log_p) * sizeof(uint2), quot_bytes = (nm << log_r) * sizeof(uint32_t);
-    bool ok = cudaMalloc(&pairs, pair_bytes) == cudaSuccess && cudaMalloc(&quot, quot_bytes) == cudaSuccess;
+    bool ok = cudaMalloc(&pairs, (nm << log_p) * sizeof(uint2)) == cudaSuccess &&
+              cudaMalloc(&quot, (nm << log_r) * sizeof(uint32_t)) == cudaSuccess;
     ok = ok && (M.rx || cudaMalloc(&M.rx, nm * sizeof(RxModulus)) == cudaSuccess);
     if (ok) {
         const dim3 grid(std::max(1u, std::min(64u, (1u << log_r) / 256u)), (unsigned)nm);
@@ -1564,7 +1572,7 @@ bool ensure_roots(BatchPlan& P, uint32_t kind) {
     }
     P.allocations.push_back(pairs);
     P.allocations.push_back(quot);
-    P.table_bytes += pair_bytes + quot_bytes;
+    P.table_bytes += root_bytes(P, nm);
     return true;
 }
 
@@ -1700,6 +1708,11 @@ void runner_free_queue(BatchRunner* r) {
     r->h_tiles = nullptr;
     r->cap_units = r->cap_tiles = 0;
 }
+// A new runner's queue: 30 KB of units and 48 KB of tiles; it grows with the job lists.
+constexpr size_t kRunnerUnits = 176, kRunnerTiles = 4096;
+size_t queue_bytes(size_t units = kRunnerUnits, size_t tiles = kRunnerTiles) {
+    return units * (sizeof(BUnit) + 8) + tiles * (sizeof(BTile) + 4);
+}
 int runner_reserve(BatchRunner* r, size_t units, size_t tiles) {
     if (units <= r->cap_units && tiles <= r->cap_tiles) return 0;
     const size_t cu = std::max(units, r->cap_units * 2), ct = std::max(tiles, r->cap_tiles * 2);
@@ -1720,25 +1733,46 @@ int runner_reserve(BatchRunner* r, size_t units, size_t tiles) {
 }  // namespace
 
 // A runner's tiles: its job lists are all of the plan's twist, in both directions.
-static Tiles runner_tiles(BatchPlan* P, const nttb_batch_config& cfg) {
+static Tiles runner_tiles(BatchPlan* P, const nttb_batch_config& cfg, bool radix) {
     if (!tensor_tiles(cfg)) return Tiles::kCore;
-    if (P->max_log >= kRxMinLog && ensure_roots(*P, P->negacyclic ? 2 : 0) && ensure_roots(*P, P->negacyclic ? 3 : 1))
+    if (radix && P->max_log >= kRxMinLog && ensure_roots(*P, P->negacyclic ? 2 : 0) &&
+        ensure_roots(*P, P->negacyclic ? 3 : 1))
         return Tiles::kRadix;
     return ensure_images(*P) ? Tiles::kTensor : Tiles::kCore;
 }
-void batch_plan_prepare(BatchPlan* P, const nttb_batch_config& cfg) { runner_tiles(P, cfg); }
 
-int runner_create(BatchPlan* P, const nttb_batch_config& cfg, BatchRunner** out) {
+bool batch_plan_prepare(BatchPlan* P, const nttb_batch_config& cfg, uint32_t runners, size_t budget) {
+    if (check_config(cfg)) return false;  // runner_create refuses it
+    const size_t nm = P->limbs.size();
+    // what requests would be left on either kind of tiles
+    auto left = [&](Tiles kind) {
+        size_t bytes = batch_plan_device_bytes(P) + runners * (ws_layout(*P, cfg, kind, nullptr).words * 4 + queue_bytes());
+        if (kind == Tiles::kRadix) bytes += 2 * root_bytes(*P, nm) + nm * sizeof(RxModulus);
+        if (kind == Tiles::kTensor) bytes += nm * (size_t)kImgPerMod;
+        return budget > bytes ? budget - bytes : 0;
+    };
+    bool radix = false;
+    if (tensor_tiles(cfg) && P->max_log >= kRxMinLog) {
+        // a budget that the root tables (4 bytes per root up to the largest size,
+        // modulus and direction) would overrun, and the tensor tiles' images do not,
+        // is served on tensor tiles
+        const size_t with = left(Tiles::kRadix);
+        radix = with > kServerMinRegion || with >= left(P->max_log >= 13 ? Tiles::kTensor : Tiles::kCore);
+    }
+    return runner_tiles(P, cfg, radix) == Tiles::kRadix;
+}
+
+int runner_create(BatchPlan* P, const nttb_batch_config& cfg, bool radix, BatchRunner** out) {
     if (int rc = check_config(cfg)) return rc;
     auto* r = new BatchRunner();
     r->plan = P;
     r->cfg = cfg;
-    r->kind = runner_tiles(P, cfg);
+    r->kind = runner_tiles(P, cfg, radix);
     r->var = r->kind == Tiles::kRadix ? &kRadixVariant
                                       : find_variant(cfg.tile_elems, cfg.threads, cfg.group, r->kind == Tiles::kTensor);
     r->layout = ws_layout(*P, cfg, r->kind, nullptr);  // rings for every size class the plan allows
     r->ws_bytes = (size_t)r->layout.words * 4;
-    if ((r->ws_bytes && cudaMalloc(&r->d_ws, r->ws_bytes) != cudaSuccess) || runner_reserve(r, 256, 4096)) {
+    if ((r->ws_bytes && cudaMalloc(&r->d_ws, r->ws_bytes) != cudaSuccess) || runner_reserve(r, kRunnerUnits, kRunnerTiles)) {
         runner_destroy(r);
         return fail(NTTB_ERR_NO_MEMORY, "batch runner: allocation failed");
     }
@@ -1754,9 +1788,7 @@ void runner_destroy(BatchRunner* r) {
     delete r;
 }
 
-size_t runner_device_bytes(const BatchRunner* r) {
-    return r->ws_bytes + r->cap_units * (sizeof(BUnit) + 8) + r->cap_tiles * (sizeof(BTile) + 4);
-}
+size_t runner_device_bytes(const BatchRunner* r) { return r->ws_bytes + queue_bytes(r->cap_units, r->cap_tiles); }
 
 // Plans the jobs, uploads the queue from pinned staging and launches, all on
 // `s`.  One run per runner may be in flight: the staging is reused.

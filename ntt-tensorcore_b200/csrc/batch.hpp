@@ -30,12 +30,15 @@ struct BatchPlan {
 // persistent launch all go on the caller's stream, with no allocation unless
 // a job list outgrows every earlier one.  One run per runner in flight.
 struct BatchRunner;
-int runner_create(BatchPlan* plan, const nttb_batch_config& cfg, BatchRunner** out);
+int runner_create(BatchPlan* plan, const nttb_batch_config& cfg, bool radix, BatchRunner** out);
 int runner_run(BatchRunner* r, const nttb_batch_job* jobs, uint32_t n_jobs, cudaStream_t s);
 void runner_destroy(BatchRunner* r);
 size_t runner_device_bytes(const BatchRunner* r);
-// Makes the tables that a runner of this configuration needs.
-void batch_plan_prepare(BatchPlan* plan, const nttb_batch_config& cfg);
+// Makes the tables that `runners` runners of this configuration need, chosen by
+// what they leave of `budget` bytes for requests: true: runners run the register-radix tiles.
+bool batch_plan_prepare(BatchPlan* plan, const nttb_batch_config& cfg, uint32_t runners, size_t budget);
+// A server keeps more than this for requests, or is refused.
+constexpr size_t kServerMinRegion = 1u << 20;
 size_t batch_plan_device_bytes(const BatchPlan* plan);
 
 }  // namespace nttb

@@ -235,13 +235,13 @@ NTTB_API int nttb_server_create(const uint64_t* moduli, uint32_t n_moduli, const
         delete s;
         return rc;
     }
-    nttb::batch_plan_prepare(&s->plan->p, cfg->batch);
+    const bool radix = nttb::batch_plan_prepare(&s->plan->p, cfg->batch, cfg->slots, cfg->hbm_budget_bytes);
     s->resident = nttb::batch_plan_device_bytes(&s->plan->p);
     s->slots.resize(cfg->slots);
     for (nttb::Slot& sl : s->slots) {
         sl.srv = s;
         if (cudaStreamCreateWithFlags(&sl.stream, cudaStreamNonBlocking) != cudaSuccess ||
-            nttb::runner_create(&s->plan->p, cfg->batch, &sl.runner)) {
+            nttb::runner_create(&s->plan->p, cfg->batch, radix, &sl.runner)) {
             for (nttb::Slot& t : s->slots) {
                 if (t.runner) nttb::runner_destroy(t.runner);
                 if (t.stream) cudaStreamDestroy(t.stream);
@@ -252,7 +252,7 @@ NTTB_API int nttb_server_create(const uint64_t* moduli, uint32_t n_moduli, const
         }
         s->resident += nttb::runner_device_bytes(sl.runner);
     }
-    if (cfg->hbm_budget_bytes <= s->resident + (1u << 20)) {
+    if (cfg->hbm_budget_bytes <= s->resident + nttb::kServerMinRegion) {
         for (nttb::Slot& t : s->slots) {
             nttb::runner_destroy(t.runner);
             cudaStreamDestroy(t.stream);
