@@ -218,6 +218,8 @@ __device__ __forceinline__ void rx_rows(const BArgs& a, const BUnit& u, uint32_t
         make_uint2(0, 0), c0, c1, 0, tid, sm, active, nullptr);
 }
 
+// What the tile threads do with a slot.
+enum : uint32_t { kRxRun = 0, kRxStop = 1, kRxSkip = 2 };
 struct RxSlot {
     BUnit u;
     uint32_t unit, pass, tile, stop;
@@ -352,11 +354,18 @@ __global__ void __launch_bounds__(kRxThreads + 32, kRxCtas) batch_queue_radix(co
             uint32_t ticket = 0;
             if (lane == 0) ticket = atomicAdd(a.ctr, 1u);
             ticket = __shfl_sync(~0u, ticket, 0);
-            bool stop = ticket >= a.n_tiles, rx = false;
+            uint32_t stop = ticket >= a.n_tiles ? kRxStop : kRxRun;
+            bool rx = false;
             if (!stop) {
                 const BTile tl = a.tiles[ticket];
 #if NTTB_DEBUG_BOUNDS
-                if (!tile_in_range(a, tl)) stop = true;  // recorded; this CTA takes no more tiles
+                if (!tile_in_range(a, tl)) {  // recorded; the tile is passed over, and counted as done
+                    stop = kRxSkip;
+                    if (lane == 0) {
+                        slot[s].unit = tl.unit;
+                        slot[s].pass = tl.pass_tile >> 31;
+                    }
+                }
 #endif
                 if (!stop) {
                     if (lane < sizeof(BUnit) / 16)
@@ -385,7 +394,7 @@ __global__ void __launch_bounds__(kRxThreads + 32, kRxCtas) batch_queue_radix(co
             if (lane == 0) slot[s].stop = stop;
             __syncwarp();
             asm volatile("bar.arrive %0, %1;" ::"r"(2u + s), "n"(kRxThreads + 32) : "memory");
-            if (stop) return;
+            if (stop == kRxStop) return;
             if (rx) {  // the roots of the running tile's last round are in use until then
                 if (roots_used) asm volatile("bar.sync 7, %0;" ::"n"(kRxThreads + 32) : "memory");
                 roots_used = true;
@@ -398,10 +407,15 @@ __global__ void __launch_bounds__(kRxThreads + 32, kRxCtas) batch_queue_radix(co
     for (uint32_t k = 0;; k++) {
         const uint32_t s = k & 1u;
         asm volatile("bar.sync %0, %1;" ::"r"(2u + s), "n"(kRxThreads + 32) : "memory");
-        if (slot[s].stop) return;
-        rx_dispatch<W64>(a, slot[s], work, inbox, few + s * kRxFew, s_ar);
+        if (slot[s].stop == kRxStop) return;
+        bool signal = true;
+#if NTTB_DEBUG_BOUNDS
+        if (slot[s].stop == kRxSkip) signal = slot[s].unit < a.n_units;
+        else
+#endif
+            rx_dispatch<W64>(a, slot[s], work, inbox, few + s * kRxFew, s_ar);
         rx_sync();
-        if (threadIdx.x == 0) signal_done(a.ctr + 1 + 2 * slot[s].unit + slot[s].pass);
+        if (threadIdx.x == 0 && signal) signal_done(a.ctr + 1 + 2 * slot[s].unit + slot[s].pass);
         asm volatile("bar.arrive %0, %1;" ::"r"(4u + s), "n"(kRxThreads + 32) : "memory");
     }
 }
