@@ -79,11 +79,12 @@ NTTB_API int nttb_device_errors(uint32_t* flags, int clear);
  * `python ntt-tensorcore_b200/build.py --debug-bounds`), the stand-in for a
  * memory checker: bits 0-7 the INT8 cluster kernel, 8-15 the DMMA passes,
  * 16-23 the uneven-batch queue kernels, 24-31 the 64-bit byte-plane engine
- * (nttb_wide_transform_engine); within each byte the kind of check
- * that failed (bit 0 global-memory index, 1 shared-memory offset, 2
- * distributed-shared-memory piece copy, 3 queue ticket / unit / tile index,
- * 4 workspace slot, 5 output residue not reduced).  A failed check skips
- * the access it guards.  *enabled = 1 in that build; the release build
+ * (nttb_wide_transform_engine), the register-radix passes and the K-limb
+ * passes; within each byte the kind of check that failed (bit 0 global-memory
+ * index, 1 shared-memory offset, 2 distributed-shared-memory piece copy, 3
+ * queue ticket / unit / tile index, 4 workspace slot, 5 output residue not
+ * reduced, 6 input residue outside the contract, in the register-radix kernels).
+ * A failed check skips the access it guards.  *enabled = 1 in that build; the release build
  * compiles the checks away (enabled 0, flags 0).  Reads after a device
  * synchronize; clear != 0 resets them.  No reference counterpart (the
  * reference's debug build is nvcc -G -g, CMakeLists.txt:10). */

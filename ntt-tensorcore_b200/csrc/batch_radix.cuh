@@ -88,16 +88,19 @@ constexpr int kRxNP = LGV == 0 ? 5 : kRxTL<LG, LB> < 5 ? kRxTL<LG, LB> : 5;
 // column v at (i << LGV) + v (uint64 words are read from `src` instead), and
 // the roots: pairs, or (kQuot) quotients, root i of column v at (i << LGV) + v;
 // `box` those of the last round (in the forward order), `few` the others.
+// lim_in, lim_out: words from src (and pre) and from dst (range checks).
 template <int LG, int LGV, bool INV, int S0, bool kQuot, int LSI, int LSO, int LB, int LBP, class S, class D>
 __device__ __forceinline__ void rx_tile(const M32& ar, const uint32_t* in, const uint32_t* few,
                                         const uint32_t* box, const S* src, D* dst,
                                         const uint32_t* pre, uint2 one, uint2 c0, uint2 c1, uint32_t col0, uint32_t tid,
-                                        uint32_t* sm, bool active, const uint32_t* drop) {
+                                        uint32_t* sm, bool active, const uint32_t* drop, uint32_t lim_in,
+                                        uint32_t lim_out) {
     using P = typename std::conditional<kQuot, uint32_t, uint2>::type;
     constexpr uint32_t NE = 1u << kRxE, V = 1u << LGV, NT = 1u << (LG - kRxE);
     constexpr rdx::Rounds<LG, kRxE> R;
     constexpr int NR = R.n;
     constexpr bool kBlock = LB >= 0;
+    constexpr bool kInput = kBlock || LGV == 0;  // the pass that reads the caller's residues
     // the blocked store: positions below the block, then columns, then positions
     constexpr int TL = kRxTL<LG, LBP>;
     const uint32_t v_v = tid & (V - 1u), t_v = tid >> LGV;
@@ -109,9 +112,13 @@ __device__ __forceinline__ void rx_tile(const M32& ar, const uint32_t* in, const
         constexpr bool blk = kBlock && K == NR - 1;
         using Pl = rdx::Place<uint32_t, LG, LGV, kRxE, I, kRxNP<LG, LGV, LBP>>;
         const uint32_t t = blk ? t_b : t_v, v = blk ? v_b : v_v;
-        uint32_t* base = sm + Pl::base(t) + v;
-        const P* roots = reinterpret_cast<const P*>(I == NR - 1 ? box : few) +
-                         (kQuot ? (Pl::natural(t) << LGV) + v : Pl::natural(t));
+        uint32_t at0 = Pl::base(t) + v, block = Pl::natural(t);
+        constexpr rdx::Lay<LG, LGV, 5, kRxNP<LG, LGV, LBP>> Y;
+        if (!NTTB_CHECK(g_batch_bounds, kBoundsShared, at0 + Pl::reg(NE - 1u) < Y.words)) at0 = 0;
+        // a block of the round's first stage: then every root's index is below 2^LG (box) or 2^LG / 16 (few)
+        if (!NTTB_CHECK(g_batch_bounds, kBoundsShared, block < (1u << R.s0[I]) && v < V)) block = 0;
+        uint32_t* base = sm + at0;
+        const P* roots = reinterpret_cast<const P*>(I == NR - 1 ? box : few) + (kQuot ? (block << LGV) + v : block);
         if constexpr (K == 0) {
             // position t + rev(e) NT (inverse) or t + e NT: the parts share no bit, so
             // every address is a thread's base plus a constant
@@ -121,19 +128,26 @@ __device__ __forceinline__ void rx_tile(const M32& ar, const uint32_t* in, const
             for (uint32_t e = 0; e < NE; e++) {
                 const uint32_t ie = (INV ? rdx::brv(e, kRxE) : e) * NT;
                 if constexpr (sizeof(S) == 8) {  // any word below 2^32: its residue
-                    const uint32_t y = (uint32_t)__ldcs(gsrc + ((size_t)ie << LSI));
+                    uint64_t w = 0;
+                    if (NTTB_CHECK(g_batch_bounds, kBoundsGlobal, ((size_t)(t + ie) << LSI) + v < lim_in))
+                        w = __ldcs(gsrc + ((size_t)ie << LSI));
+                    (void)NTTB_CHECK(g_batch_bounds, kBoundsInput, w >> 32 == 0);
+                    const uint32_t y = (uint32_t)w;
                     x[e] = rdx::sub_if(y - __umulhi(y, one.y) * ar.q, ar.q);
                 } else {
-                    x[e] = isrc[ie << LGV];
+                    x[e] = NTTB_CHECK(g_batch_bounds, kBoundsShared, ((t + ie) << LGV) + v < kRxTile) ? isrc[ie << LGV] : 0u;
+                    if constexpr (kInput) (void)NTTB_CHECK(g_batch_bounds, kBoundsInput, !active || x[e] < ar.q);
                 }
             }
             if constexpr (sizeof(S) != 8) rx_inbox_free();
             if (INV && pre) {  // a product's spectra; the scale carries the factor 2^32
                 const uint32_t* p = pre + (((size_t)t << LSI) + v);
 #pragma unroll
-                for (uint32_t e = 0; e < NE; e++)
-                    x[e] = rdx::sub_if(tca::mont_lazy(x[e], __ldcg(p + ((size_t)(rdx::brv(e, kRxE) * NT) << LSI)), ar.q, ar.qinv),
-                                       ar.q);
+                for (uint32_t e = 0; e < NE; e++) {
+                    const size_t i = (size_t)(rdx::brv(e, kRxE) * NT) << LSI;
+                    if (!NTTB_CHECK(g_batch_bounds, kBoundsGlobal, ((size_t)t << LSI) + v + i < lim_in)) continue;
+                    x[e] = rdx::sub_if(tca::mont_lazy(x[e], __ldcg(p + i), ar.q, ar.qinv), ar.q);
+                }
             }
         } else {
             rdx::exchange<Pl, false>(base, x);
@@ -153,14 +167,23 @@ __device__ __forceinline__ void rx_tile(const M32& ar, const uint32_t* in, const
             if constexpr (kBlock) {
                 const uint64_t keep = tc::l2_policy_evict_last();
                 auto at = [](uint32_t i) { return ((size_t)(i >> LB) << (LSI + LB)) + (i & ((1u << LB) - 1u)); };
-                D* p = dst + (at(t) + ((size_t)(col0 + v) << LB));
+                const size_t p0 = at(t) + ((size_t)(col0 + v) << LB);
+                D* p = dst + p0;
 #pragma unroll
-                for (uint32_t e = 0; e < NE; e++) st_keep(p + at((INV ? e : rdx::brv(e, kRxE)) * NT), x[e], keep);
+                for (uint32_t e = 0; e < NE; e++) {
+                    const size_t i = at((INV ? e : rdx::brv(e, kRxE)) * NT);
+                    if (NTTB_CHECK(g_batch_bounds, kBoundsWorkspace, p0 + i < lim_out)) st_keep(p + i, x[e], keep);
+                }
             } else if (active) {
-                D* p = dst + (((size_t)t << LSO) + v);
+                const size_t p0 = ((size_t)t << LSO) + v;
+                D* p = dst + p0;
 #pragma unroll
-                for (uint32_t e = 0; e < NE; e++)
-                    __stcs(p + ((size_t)((INV ? e : rdx::brv(e, kRxE)) * NT) << LSO), (D)rdx::canon_out<INV>(ar, x[e]));
+                for (uint32_t e = 0; e < NE; e++) {
+                    const size_t i = (size_t)((INV ? e : rdx::brv(e, kRxE)) * NT) << LSO;
+                    const uint32_t y = rdx::canon_out<INV>(ar, x[e]);
+                    (void)NTTB_CHECK(g_batch_bounds, kBoundsResidue, y < ar.q);
+                    if (NTTB_CHECK(g_batch_bounds, kBoundsGlobal, p0 + i < lim_out)) __stcs(p + i, (D)y);
+                }
             }
         }
     };
@@ -184,12 +207,12 @@ __device__ __forceinline__ void rx_pass(const BUnit& u, uint32_t tile, uint32_t*
         const W* src = static_cast<const W*>(u.in ? u.in : u.data) + col0;
         rx_tile<LG, LGV, INV, S0, kRow, LC, 0, LB, LB, W, uint32_t>(
             ar, in, few, box, src, u.ws, INV && u.pre_mul ? u.pre_mul + col0 : nullptr, u.one, u.scale[0], u.scale[1], col0,
-            threadIdx.x, sm, true, nullptr);
+            threadIdx.x, sm, true, nullptr, (1u << L) - col0, 1u << L);
     } else {
         const uint32_t* src = u.ws + (size_t)tile * kRxTile;
         rx_tile<LG, LGV, INV, S0, kRow, LGV, LC, -1, LB, uint32_t, W>(
             ar, in, few, box, src, reinterpret_cast<W*>(u.data) + col0, nullptr, u.one, u.scale[0], u.scale[1], col0, threadIdx.x,
-            sm, true, src);
+            sm, true, src, 0, (1u << L) - col0);
     }
 }
 
@@ -215,7 +238,7 @@ __device__ __forceinline__ void rx_rows(const BArgs& a, const BUnit& u, uint32_t
     uint32_t* x = u.data + ((size_t)row << L);
     rx_tile<L, 0, INV, 0, true, 0, 0, -1, 0, uint32_t, uint32_t>(
         ar, in + (row << L), few + (row << (L - kRxE)), in + kRxTile + (row << L), x, x, INV && u.pre_mul ? u.pre_mul + ((size_t)row << L) : nullptr,
-        make_uint2(0, 0), c0, c1, 0, tid, sm, active, nullptr);
+        make_uint2(0, 0), c0, c1, 0, tid, sm, active, nullptr, 1u << L, 1u << L);
 }
 
 // What the tile threads do with a slot.
@@ -268,6 +291,12 @@ __device__ __forceinline__ void rx_fetch(const BUnit& u, uint32_t pass, uint32_t
         pitch = (size_t)1 << (L - lg);
         src = static_cast<const uint32_t*>(u.in ? u.in : u.data) + ((size_t)tile << (kRxLogTile - lg));
     }
+    // the last piece ends within the unit's words (or its slot) and the inbox
+    const uint32_t* all = static_cast<const uint32_t*>(pass ? u.ws : u.in ? u.in : u.data);
+    if (!NTTB_CHECK(g_batch_bounds, kBoundsGlobal,
+                    (size_t)(src - all) + ((chunks >> lgc) - 1) * pitch + ((size_t)4 << lgc) <= ((size_t)u.rows << L)) ||
+        !NTTB_CHECK(g_batch_bounds, kBoundsShared, chunks <= kRxTile / 4))
+        return;
     rx_copy(src, lgc, pitch, chunks, inbox, lane);
 }
 

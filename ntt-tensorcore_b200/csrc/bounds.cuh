@@ -4,7 +4,8 @@
 // so the kernels whose addressing is computed by hand (the INT8 cluster
 // kernel's swizzled shared-memory staging and distributed-shared-memory
 // piece copies, the DMMA passes' tile coordinates, the batch queue's
-// tickets, units and workspace slots) can be built with their own checks:
+// tickets, units and workspace slots, the register-radix and K-limb passes'
+// operands, roots and exchanges) can be built with their own checks:
 // `python ntt-tensorcore_b200/build.py --debug-bounds` compiles every source
 // with -DNTT_DEBUG_BOUNDS into ntt_b200/libntt_b200_dbg.so.  There, each
 // checked index or residue that falls outside its range sets one bit of a

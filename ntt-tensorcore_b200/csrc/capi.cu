@@ -285,7 +285,10 @@ int nttb_bounds_errors(uint32_t* flags, int* enabled, int clear) {
     *enabled = 0;
 #endif
     *flags = int8_bounds_errors(clear != 0) | (dmma_bounds_errors(clear != 0) << 8) |
-             (batch_bounds_errors(clear != 0) << 16) | (wide_bounds_errors(clear != 0) << 24);
+             (batch_bounds_errors(clear != 0) << 16) |
+             ((wide_bounds_errors(clear != 0) | radix_u32_bounds_errors(clear != 0) | radix_w64_bounds_errors(clear != 0) |
+               radix_q64_bounds_errors(clear != 0) | klimb_bounds_errors(clear != 0))
+              << 24);
     return cuda_status("bounds_errors");
 }
 

@@ -37,6 +37,7 @@
 
 #include "../../include/ntt_b200.h"
 #include "../../include/ntt_limb_arith.cuh"
+#include "bounds.cuh"
 #include "engines.hpp"
 #include "klimb_plan.hpp"
 #include "profiler.hpp"
@@ -44,6 +45,17 @@
 
 namespace nttb {
 namespace {
+
+#if NTTB_DEBUG_BOUNDS
+__device__ uint32_t g_klimb_bounds;
+// w < p, words from the lowest up
+template <int W>
+__device__ __forceinline__ bool below(const uint32_t* w, const uint32_t* p) {
+    bool lt = false;
+    for (int i = 0; i < W; i++) lt = w[i] != p[i] ? w[i] < p[i] : lt;
+    return lt;
+}
+#endif
 
 // ------------------------------------------------------------ residue forms
 // Each form: W words per element in shared memory, load / store between them
@@ -68,7 +80,9 @@ struct LimbForm {
         nttb_limb::add_mod<K>(u, u, x, p);
         unpack(v, d);
     }
-    __device__ __forceinline__ void finish(uint32_t*) const {}
+    __device__ __forceinline__ void finish(uint32_t* w) const {
+        (void)NTTB_CHECK(g_klimb_bounds, kBoundsResidue, below<W>(w, p));
+    }
 };
 
 // 24-bit limbs <-> 32-bit words (W words hold the value: its limbs above are 0)
@@ -221,6 +235,7 @@ struct Form256 : Words<11, 8> {
     __device__ __forceinline__ void finish(uint32_t* w) const {
         reduce(w, w, p2);
         reduce(w, w, p);
+        (void)NTTB_CHECK(g_klimb_bounds, kBoundsResidue, below<W>(w, p));
     }
 };
 
@@ -248,7 +263,9 @@ struct Form64 : Words<3, 2> {
         put(u, (s < c || s >= p) ? s - p : s);
         put(v, c < x ? c - x + p : c - x);
     }
-    __device__ __forceinline__ void finish(uint32_t*) const {}
+    __device__ __forceinline__ void finish(uint32_t* w) const {
+        (void)NTTB_CHECK(g_klimb_bounds, kBoundsResidue, val(w) < p);
+    }
 };
 
 // ------------------------------------------------------------------- kernel
@@ -297,6 +314,13 @@ __global__ void __launch_bounds__(MAXT) klimb_pass(const __grid_constant__ PassA
     const uint32_t P = E + (E >> 5);
     uint32_t* const roots = sm + E * K;
     uint32_t* const tile = roots + E * W;
+#if NTTB_DEBUG_BOUNDS
+    // every shared-memory index below is an element below E of one of the three arrays
+    uint32_t dyn;
+    asm("mov.u32 %0, %%dynamic_smem_size;" : "=r"(dyn));
+    if (!NTTB_CHECK(g_klimb_bounds, kBoundsShared, (E * (K + W) + P * W) * 4 <= dyn && E <= 2 * blockDim.x)) return;
+#endif
+    const size_t words = (size_t)K << log_n;  // of the data and of the table
     auto at = [](uint32_t e) { return e + (e >> 5); };
     auto sync = [] {
         if (blockDim.x <= 32) __syncwarp();
@@ -330,8 +354,11 @@ __global__ void __launch_bounds__(MAXT) klimb_pass(const __grid_constant__ PassA
             const uint32_t i = tid + q * blockDim.x, j1 = (i >> logC) + 1, t = 31 - __clz(j1);
             if (i >= n_roots) break;
             const uint32_t k = ((j1 - (1u << t)) << s0) + low0 + (i & (C - 1)), sh = log_n - s0 - t - 1;
-            const uint32_t* w = g.tw + ((size_t)k << sh) * K;
-            if (K > 2 && g.vec_tw && sh >= 2) {
+            const size_t off = ((size_t)k << sh) * K;
+            const bool wide = K > 2 && g.vec_tw && sh >= 2;
+            if (!NTTB_CHECK(g_klimb_bounds, kBoundsGlobal, off + (wide ? RAW : K) <= words)) continue;
+            const uint32_t* w = g.tw + off;
+            if (wide) {
 #pragma unroll
                 for (int m = 0; m + 4 <= RAW; m += 4) {
                     const uint4 x = __ldg(reinterpret_cast<const uint4*>(w + m));
@@ -353,11 +380,15 @@ __global__ void __launch_bounds__(MAXT) klimb_pass(const __grid_constant__ PassA
     // 32 elements touch K lines each), by way of shared memory, where a stride of
     // K words is free of conflicts.
     if (g.vec_data) {
-        for (uint32_t v = 4 * tid; v < E * K; v += 4 * blockDim.x)
-            cp_async<16>(sm + v, g.data + place(v / K, true) * K + v % K);
+        for (uint32_t v = 4 * tid; v < E * K; v += 4 * blockDim.x) {
+            const size_t i = place(v / K, true) * K + v % K;
+            if (NTTB_CHECK(g_klimb_bounds, kBoundsGlobal, i + 4 <= words)) cp_async<16>(sm + v, g.data + i);
+        }
     } else {
-        for (uint32_t v = tid; v < E * K; v += blockDim.x)
-            cp_async<4>(sm + v, g.data + place(v / K, true) * K + v % K);
+        for (uint32_t v = tid; v < E * K; v += blockDim.x) {
+            const size_t i = place(v / K, true) * K + v % K;
+            if (NTTB_CHECK(g_klimb_bounds, kBoundsGlobal, i < words)) cp_async<4>(sm + v, g.data + i);
+        }
     }
 #pragma unroll
     for (int q = 0; q < 2; q++) {
@@ -399,7 +430,9 @@ __global__ void __launch_bounds__(MAXT) klimb_pass(const __grid_constant__ PassA
                     v[k] = tile[k * P + at(ehi)];
                 }
             }
+            if (!NTTB_CHECK(g_klimb_bounds, kBoundsShared, elo < E && ehi < E)) elo = ehi = 0;
             const uint32_t* rt = roots + (((half - 1) + (pi & (half - 1))) << logC) + c;
+            if (!NTTB_CHECK(g_klimb_bounds, kBoundsShared, rt < roots + E)) rt = roots;
 #pragma unroll
             for (int k = 0; k < W; k++) w[k] = rt[k * E];
             f.butterfly(u, v, w);
@@ -423,10 +456,16 @@ __global__ void __launch_bounds__(MAXT) klimb_pass(const __grid_constant__ PassA
         sync();
     }
     if (g.vec_data) {
-        for (uint32_t v = 4 * tid; v < E * K; v += 4 * blockDim.x)
-            *reinterpret_cast<uint4*>(g.data + place(v / K, false) * K + v % K) = *reinterpret_cast<const uint4*>(sm + v);
+        for (uint32_t v = 4 * tid; v < E * K; v += 4 * blockDim.x) {
+            const size_t i = place(v / K, false) * K + v % K;
+            if (NTTB_CHECK(g_klimb_bounds, kBoundsGlobal, i + 4 <= words))
+                *reinterpret_cast<uint4*>(g.data + i) = *reinterpret_cast<const uint4*>(sm + v);
+        }
     } else {
-        for (uint32_t v = tid; v < E * K; v += blockDim.x) g.data[place(v / K, false) * K + v % K] = sm[v];
+        for (uint32_t v = tid; v < E * K; v += blockDim.x) {
+            const size_t i = place(v / K, false) * K + v % K;
+            if (NTTB_CHECK(g_klimb_bounds, kBoundsGlobal, i < words)) g.data[i] = sm[v];
+        }
     }
 }
 
@@ -509,6 +548,19 @@ int klimb11(uint32_t* d_data, const uint32_t* d_tw, uint32_t log_n, const uint32
 }
 
 }  // namespace
+
+uint32_t klimb_bounds_errors(bool clear) {
+    uint32_t v = 0;
+#if NTTB_DEBUG_BOUNDS
+    const uint32_t z = 0;
+    cudaMemcpyFromSymbol(&v, g_klimb_bounds, sizeof v);
+    if (clear) cudaMemcpyToSymbol(g_klimb_bounds, &z, sizeof z);
+#else
+    (void)clear;
+#endif
+    return v;
+}
+
 }  // namespace nttb
 
 extern "C" {

@@ -265,6 +265,10 @@ uint32_t int8_bounds_errors(bool clear);
 void int8_phase_profile(uint64_t* out16, bool clear);
 uint32_t dmma_bounds_errors(bool clear);
 uint32_t batch_bounds_errors(bool clear);
+uint32_t radix_u32_bounds_errors(bool clear);
+uint32_t radix_w64_bounds_errors(bool clear);
+uint32_t radix_q64_bounds_errors(bool clear);
+uint32_t klimb_bounds_errors(bool clear);
 // Forward then inverse, in place, in one persistent launch.
 int int8_forward_inverse32(Plan32& p, uint32_t* data, uint32_t n_polys, cudaStream_t s);
 

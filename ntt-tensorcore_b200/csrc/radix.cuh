@@ -33,10 +33,15 @@
 #include <cstdint>
 
 #include "arith.cuh"
+#include "bounds.cuh"
 #include "plan.hpp"
 
 namespace nttb {
 namespace rdx {
+
+#if NTTB_DEBUG_BOUNDS
+static __device__ uint32_t g_radix_bounds;  // one per file that includes this
+#endif
 
 struct Args {
     const void* src;
@@ -286,12 +291,20 @@ struct Pass {
 
     template <int K>
     __device__ __forceinline__ static void roots(P (&w)[NE - 1], const P* tab, uint32_t col0) {
-        round_roots<LG, LGE, kI<K>, S0, INV>(w, tab + (S0 > 0 ? col0 + v<K>() : 0u) + ((size_t)Pl<K>::natural(t<K>()) << S0));
+        uint32_t block = (S0 > 0 ? col0 + v<K>() : 0u) + (Pl<K>::natural(t<K>()) << S0);
+        // below the blocks of the round's first stage: then every index is below 2^(S0 + LG)
+        if (!NTTB_CHECK(g_radix_bounds, kBoundsGlobal, block < (1u << (S0 + Pl<K>::s0)))) block = 0;
+        round_roots<LG, LGE, kI<K>, S0, INV>(w, tab + block);
     }
     template <int K = 0>
     __device__ __forceinline__ static void run(const A& ar, E (&x)[NE], P (&w)[NE - 1], E* sm, const P* tab, uint32_t col0,
                                                P c0, P c1) {
-        E* base = sm + (NR > 1 ? Pl<K>::base(t<K>()) + v<K>() : 0u);
+        uint32_t at = NR > 1 ? Pl<K>::base(t<K>()) + v<K>() : 0u;
+        if constexpr (NR > 1) {
+            constexpr Lay<LG, LGV, kBankBits<E>, kLanePos<E, LG, LGV, LGE>> L;
+            if (!NTTB_CHECK(g_radix_bounds, kBoundsShared, at + Pl<K>::reg(NE - 1u) < L.words)) at = 0;
+        }
+        E* base = sm + at;
         if constexpr (K > 0) exchange<Pl<K>, false>(base, x);
         round_stages<A, LG, LGE, kI<K>, S0, INV>(ar, x, w, c0, c1);
         if constexpr (K < NR - 1) {
@@ -324,6 +337,8 @@ __global__ void __launch_bounds__(kThreads<LG, LGV, LGE>, TSM / kThreads<LG, LGV
     constexpr bool kSingle = LGV == 0;
     // the pass that leaves canonical residues
     constexpr bool kLast = DIR == kFwd ? MODE != kContOut : S0 == 0;
+    // the pass that reads the caller's residues
+    constexpr bool kFirst = kSingle || MODE == kContOut;
     constexpr bool kReduce = sizeof(S) == 8 && sizeof(E) == 4;
     extern __shared__ __align__(16) unsigned char rdx_smem[];
     constexpr Lay<LG, LGV, kBankBits<E>, kLanePos<E, LG, LGV, LGE>> L;
@@ -360,6 +375,8 @@ __global__ void __launch_bounds__(kThreads<LG, LGV, LGE>, TSM / kThreads<LG, LGV
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
+    // words of either operand: no index reaches them (range checks)
+    const uint64_t words = (uint64_t)a.polys * a.poly_stride;
     // register e's position is a thread's base plus a constant: the parts share no bit
     constexpr int LI = MODE == kContIn ? 0 : LST, LO = MODE == kContOut ? 0 : LST, NR = First::NR;
     for (uint32_t k = 0; k < n_poly; k++) {
@@ -373,7 +390,12 @@ __global__ void __launch_bounds__(kThreads<LG, LGV, LGE>, TSM / kThreads<LG, LGV
             const S* p = src + (MODE == kContIn ? ((size_t)col << LG) + t : ((size_t)t << LST) + col);
 #pragma unroll
             for (uint32_t e = 0; e < NE; e++) {
-                const S y = __ldcg(p + ((size_t)First::in(e) << LI));
+                const S* at = p + ((size_t)First::in(e) << LI);
+                const bool ok = NTTB_CHECK(g_radix_bounds, kBoundsGlobal,
+                                           (uint64_t)(at - reinterpret_cast<const S*>(a.src)) < words);
+                const S y = ok ? __ldcg(at) : S(0);
+                if constexpr (kFirst)
+                    (void)NTTB_CHECK(g_radix_bounds, kBoundsInput, kReduce ? (uint64_t)y >> 32 == 0 : y < (S)ar.q);
                 if constexpr (kReduce) {  // any word below 2^32: its residue
                     x[e] = sub_if((uint32_t)y - __umulhi((uint32_t)y, one.y) * ar.q, ar.q);
                 } else {
@@ -396,7 +418,11 @@ __global__ void __launch_bounds__(kThreads<LG, LGV, LGE>, TSM / kThreads<LG, LGV
 #pragma unroll
             for (uint32_t e = 0; e < NE; e++) {
                 const E y = kLast ? canon_out<(DIR != kFwd)>(ar, x[e]) : x[e];
-                if (active) p[(size_t)Last::out(e) << LO] = (D)y;
+                D* at = p + ((size_t)Last::out(e) << LO);
+                if constexpr (kLast) (void)NTTB_CHECK(g_radix_bounds, kBoundsResidue, y < ar.q);
+                if (active && NTTB_CHECK(g_radix_bounds, kBoundsGlobal,
+                                         (uint64_t)(at - reinterpret_cast<D*>(a.dst)) < words))
+                    *at = (D)y;
             }
         }
         src += a.poly_stride;

@@ -18,6 +18,19 @@ namespace rdx {
 constexpr uint32_t kSingleMax = 13;
 constexpr uint32_t kThreadsMin = 128;  // rows are grouped into CTAs of at least this many threads
 
+// Failed range checks of this file's passes (0 in the release build).
+static inline uint32_t bounds_errors(bool clear) {
+    uint32_t v = 0;
+#if NTTB_DEBUG_BOUNDS
+    const uint32_t z = 0;
+    cudaMemcpyFromSymbol(&v, g_radix_bounds, sizeof v);
+    if (clear) cudaMemcpyToSymbol(g_radix_bounds, &z, sizeof z);
+#else
+    (void)clear;
+#endif
+    return v;
+}
+
 // Shared-memory attributes of a kernel, set once per device: the dynamic size it
 // may ask for and, with `carveout`, the largest shared-memory share of the SM, so that
 // as many CTAs fit as it is built for (the roots that others read stay in L1, which

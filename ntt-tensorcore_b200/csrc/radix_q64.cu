@@ -8,4 +8,6 @@ int radix_q64(const LimbDev<M64>* limbs, uint32_t log_n, uint32_t n_limbs, const
     return rdx::transform<M64, uint64_t, uint64_t, 3>(limbs, log_n, n_limbs, src, dst, mid, n_polys, inverse, s);
 }
 
+uint32_t radix_q64_bounds_errors(bool clear) { return rdx::bounds_errors(clear); }
+
 }  // namespace nttb

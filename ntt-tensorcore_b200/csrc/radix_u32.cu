@@ -27,4 +27,6 @@ int radix_round_trip_u32(const LimbDev<M32>* limbs, uint32_t log_n, uint32_t n_l
 #undef NTTB_TWO
 }
 
+uint32_t radix_u32_bounds_errors(bool clear) { return rdx::bounds_errors(clear); }
+
 }  // namespace nttb

@@ -9,4 +9,6 @@ int radix_w64(const LimbDev<M32>* limbs, uint32_t log_n, uint32_t n_limbs, const
     return rdx::transform<M32, uint64_t, uint32_t, 4>(limbs, log_n, n_limbs, src, dst, mid, n_polys, inverse, s);
 }
 
+uint32_t radix_w64_bounds_errors(bool clear) { return rdx::bounds_errors(clear); }
+
 }  // namespace nttb
