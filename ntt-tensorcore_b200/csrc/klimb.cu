@@ -475,14 +475,13 @@ __global__ void __launch_bounds__(MAXT) klimb_pass(const __grid_constant__ PassA
 // K = 11 at 2^15 24.1 -> 18.4 us, K = 3 at 2^17 19.8 -> 15.3.
 template <class F, int WHERE>
 int launch(const F& f, const PassArgs& g, uint32_t blocks, uint32_t elements, cudaStream_t s) {
-    constexpr auto k = klimb_pass<F, WHERE, F::K <= 3 ? 512 : 256>;
-    constexpr size_t kAlone = 116 * 1024;
-    rdx::kernel_smem<k, true>(kAlone);
+    constexpr auto k = klimb_pass<F, WHERE, klimb_max_threads(F::K)>;
+    rdx::kernel_smem<k, true>(kKlimbSmemAlone);
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(blocks);
     cfg.blockDim = dim3(elements / 2);
-    cfg.dynamicSmemBytes = ((size_t)elements * (F::K + F::W) + (size_t)(elements + elements / 32) * F::W) * 4;
-    if (blocks > 1 && blocks <= 148 && cfg.dynamicSmemBytes < kAlone) cfg.dynamicSmemBytes = kAlone;
+    cfg.dynamicSmemBytes = klimb_smem_bytes(F::K, F::W, elements);
+    if (blocks > 1 && blocks <= 148 && cfg.dynamicSmemBytes < kKlimbSmemAlone) cfg.dynamicSmemBytes = kKlimbSmemAlone;
     cfg.stream = s;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -504,8 +503,9 @@ int klimb_forward(const F& f, uint32_t* d_data, const uint32_t* d_tw, uint32_t l
     for (uint32_t i = 0; i < P.n_passes; i++) {
         const KlimbPass& ps = P.pass[i];
         const PassArgs g{d_data, d_tw, log_n, ps.s0, ps.r, ps.logC, va && (i == 0 || ps.logC >= 2), vt};
-        const int rc = i == 0 ? launch<F, kSwap>(f, g, n >> (2 * ps.r), 2u << (2 * ps.r), s)
-                              : launch<F, kStages>(f, g, n >> (ps.r + ps.logC), 1u << (ps.r + ps.logC), s);
+        const uint32_t elements = klimb_pass_elements(ps, i == 0);
+        const int rc = i == 0 ? launch<F, kSwap>(f, g, n >> (2 * ps.r), elements, s)
+                              : launch<F, kStages>(f, g, n / elements, elements, s);
         if (rc) return rc;
     }
     return 0;

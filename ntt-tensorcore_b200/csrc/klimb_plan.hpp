@@ -7,10 +7,11 @@
 // by passes of radix-2 DIT stages: pass i runs stages s0 .. s0 + r - 1 on tiles of
 // 2^(r + logC) elements (2^logC columns of 2^r-element groups, logC <= s0), the
 // stages spread evenly over as few passes as 8 stages each allow.
-// Tiles hold at most 2^log_emax elements, 48 KB of shared memory at the
-// largest; log_emax shrinks while a pass would have fewer than kKlimbTargetCtas
+// The stage passes' tiles hold at most 2^log_emax elements and at most a thread per
+// butterfly; log_emax shrinks while a pass would have fewer than kKlimbTargetCtas
 // tiles (small transforms are bound by the latency of their stage chains, so more,
-// shorter tiles win), but not below 2^6.
+// shorter tiles win), but not below 2^6.  The swapping pass's blocks hold a pair of
+// 2^r x 2^r tiles whatever log_emax is.
 #pragma once
 
 #include <cstdint>
@@ -20,6 +21,19 @@ namespace nttb {
 struct KlimbPass {
     uint32_t s0, r, logC;
 };
+
+// Elements of a block, of which it has a thread for every two.
+inline uint32_t klimb_pass_elements(const KlimbPass& p, bool first) { return first ? 2u << (2 * p.r) : 1u << (p.r + p.logC); }
+// Threads that the kernel is built for.
+constexpr uint32_t klimb_max_threads(uint32_t K) { return K <= 3 ? 512u : 256u; }
+// Shared memory of a block whose elements have W words between stages: the limbs as
+// in memory, the tile's roots, and the tile (a spare word after every 32).
+constexpr uint64_t klimb_smem_bytes(uint32_t K, uint32_t W, uint64_t elements) {
+    return (elements * (K + W) + (elements + elements / 32) * W) * 4;
+}
+// More than half of an SM's shared memory: a block that asks for it has the SM to
+// itself.  No block needs more.
+constexpr uint64_t kKlimbSmemAlone = 116 * 1024;
 
 struct KlimbPlan {
     bool single_tile = false;  // one launch, bit reversal fused
