@@ -73,11 +73,20 @@ struct LimbForm {
     }
     __device__ __forceinline__ static void pack(uint32_t* l, const uint32_t* w) { unpack(l, w); }
     __device__ __forceinline__ void root(uint32_t* w, const uint32_t* l) const { unpack(w, l); }
+    // ONE: the block is the whole launch.  Its one warp or so waits for each of the
+    // modulus's limbs read from the parameters (K = 11 at 2^6 18.1 us a call), so they
+    // are kept in registers (15.5); more warps hide that and lose 1 - 3 % by it.
+    template <bool ONE>
     __device__ __forceinline__ void butterfly(uint32_t* u, uint32_t* v, const uint32_t* w) const {
-        uint32_t x[W], d[W];
-        nttb_limb::mont_mul<K>(x, v, w, p, np);
-        nttb_limb::sub_mod<K>(d, u, x, p);
-        nttb_limb::add_mod<K>(u, u, x, p);
+        uint32_t x[W], d[W], q[W];
+#pragma unroll
+        for (int k = 0; k < K; k++) {
+            if constexpr (ONE) asm("mov.u32 %0, %1;" : "=r"(q[k]) : "r"(p[k]));
+            else q[k] = p[k];
+        }
+        nttb_limb::mont_mul<K>(x, v, w, q, np);
+        nttb_limb::sub_mod<K>(d, u, x, q);
+        nttb_limb::add_mod<K>(u, u, x, q);
         unpack(v, d);
     }
     __device__ __forceinline__ void finish(uint32_t* w) const {
@@ -224,6 +233,7 @@ struct Form256 : Words<11, 8> {
         for (int i = 0; i < 8; i++) x[i] = borrow ? t[i] : d[i];
     }
     // Values between stages stay in [0, 4p): after the product one carry chain each.
+    template <bool>
     __device__ __forceinline__ void butterfly(uint32_t* u, uint32_t* v, const uint32_t* w) const {
         uint32_t x[8], c[8], c2[8];
         reduce(c, u, p2);
@@ -255,6 +265,7 @@ struct Form64 : Words<3, 2> {
         const uint64_t hi = __umul64hi(m, p) + (lo < v);
         put(w, (lo >> 8) | (hi << 56));
     }
+    template <bool>
     __device__ __forceinline__ void butterfly(uint32_t* u, uint32_t* v, const uint32_t* w) const {
         const uint64_t a = val(v), b = val(w), c = val(u);
         const uint64_t hi = __umul64hi(a, b), q = __umul64hi(a * b * pinv, p);
@@ -435,7 +446,7 @@ __global__ void __launch_bounds__(MAXT) klimb_pass(const __grid_constant__ PassA
             if (!NTTB_CHECK(g_klimb_bounds, kBoundsShared, rt < roots + E)) rt = roots;
 #pragma unroll
             for (int k = 0; k < W; k++) w[k] = rt[k * E];
-            f.butterfly(u, v, w);
+            f.template butterfly<WHERE == kWhole>(u, v, w);
             if (t + 1 < r) {
 #pragma unroll
                 for (int k = 0; k < W; k++) {
@@ -469,19 +480,21 @@ __global__ void __launch_bounds__(MAXT) klimb_pass(const __grid_constant__ PassA
     }
 }
 
-// One butterfly per thread: `elements` / 2 threads.  A launch of at most one block
-// per SM asks for more than half of an SM's shared memory, so that blocks started
-// early (behind a pass that is still draining) don't share an SM while others idle:
-// K = 11 at 2^15 24.1 -> 18.4 us, K = 3 at 2^17 19.8 -> 15.3.
+// One butterfly per thread: `elements` / 2 threads.  A launch of up to four blocks an
+// SM asks for the share of shared memory at which no more fit, so that blocks
+// started early (behind a pass that is still draining) don't crowd some SMs.  us:
+// K = 11 at 2^15 24.1 -> 18.4, K = 3 at 2^17 19.8 -> 15.3 (one block an SM); K = 11 at
+// 2^17 67.8 -> 46.8, from 2^254 on 171 -> 133, K = 3 at 2^18 from 2^64 on 53.0 -> 40.0,
+// K = 2 38.2 -> 26.7 (two to four).
 template <class F, int WHERE>
 int launch(const F& f, const PassArgs& g, uint32_t blocks, uint32_t elements, cudaStream_t s) {
     constexpr auto k = klimb_pass<F, WHERE, klimb_max_threads(F::K)>;
-    rdx::kernel_smem<k, true>(kKlimbSmemAlone);
+    rdx::kernel_smem<k, true>(kKlimbSmemMax);
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(blocks);
     cfg.blockDim = dim3(elements / 2);
     cfg.dynamicSmemBytes = klimb_smem_bytes(F::K, F::W, elements);
-    if (blocks > 1 && blocks <= 148 && cfg.dynamicSmemBytes < kKlimbSmemAlone) cfg.dynamicSmemBytes = kKlimbSmemAlone;
+    if (blocks > 1) cfg.dynamicSmemBytes = rdx::spread_smem(blocks, cfg.dynamicSmemBytes, 1, 4);
     cfg.stream = s;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;

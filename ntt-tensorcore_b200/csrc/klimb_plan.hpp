@@ -31,9 +31,9 @@ constexpr uint32_t klimb_max_threads(uint32_t K) { return K <= 3 ? 512u : 256u; 
 constexpr uint64_t klimb_smem_bytes(uint32_t K, uint32_t W, uint64_t elements) {
     return (elements * (K + W) + (elements + elements / 32) * W) * 4;
 }
-// More than half of an SM's shared memory: a block that asks for it has the SM to
-// itself.  No block needs more.
-constexpr uint64_t kKlimbSmemAlone = 116 * 1024;
+// Shared memory that a block may ask for: more than the half of an SM's at which it
+// has the SM to itself.  No block needs more.
+constexpr uint64_t kKlimbSmemMax = 116 * 1024;
 
 struct KlimbPlan {
     bool single_tile = false;  // one launch, bit reversal fused

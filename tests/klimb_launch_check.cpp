@@ -28,7 +28,7 @@ int main() {
             const unsigned long n = 1ul << lg;
             auto block = [&](unsigned long elements) {
                 expect(elements >= 2 && elements / 2 <= nttb::klimb_max_threads(f.K), "threads", f.K, f.W, lg);
-                expect(nttb::klimb_smem_bytes(f.K, f.W, elements) <= nttb::kKlimbSmemAlone, "shared memory", f.K, f.W, lg);
+                expect(nttb::klimb_smem_bytes(f.K, f.W, elements) <= nttb::kKlimbSmemMax, "shared memory", f.K, f.W, lg);
             };
             if (P.single_tile) {
                 block(n);
