@@ -291,9 +291,9 @@ typedef struct {
     uint32_t ctas_per_sm; /* 0: as many as fit */
     uint32_t group;       /* radix-2 stages per register group inside a tile: 1, 3 or 4 */
     uint32_t tensor;      /* 1 (threads 256 and tile_elems 4096 or 8192; otherwise ignored): a batch with
-                             units of 2^10 .. 2^20 residues runs the queue's register-radix tiles, which
-                             take the lag alone; where a job is off a 16-byte boundary or their root
-                             tables do not fit in memory, tensor-core tiles (INT8 DFT-64 + radix-2 DFT of
+                             units of 2^13 .. 2^20 residues, or with enough of its work at 2^10 .. 2^12,
+                             runs the queue's register-radix tiles, which take the lag alone; where a
+                             job is off a 16-byte boundary or their root tables do not fit in memory, tensor-core tiles (INT8 DFT-64 + radix-2 DFT of
                              up to 16 points) for the two-pass units of 2^13 .. 2^20 above the tile */
 } nttb_batch_config;
 

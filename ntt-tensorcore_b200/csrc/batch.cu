@@ -1576,12 +1576,35 @@ bool ensure_roots(BatchPlan& P, uint32_t kind) {
     return true;
 }
 
+// Whether the register-radix queue is the faster one for a job list, by its work
+// (residues times stages).  Its CUDA-core tiles, which take the sizes outside 2^10 ..
+// 2^20, are slower than the CUDA-core kernel's: 4096 residues on 512 threads.  So
+// below 2^10 they cost as much as the radix tiles gain on the same work, above 2^20
+// an eighth.  us, CUDA-core / radix queue, work in range 12 / 25 / 50 %: 2^8 and 2^12
+// 41 / 46, 38.6 / 41.4, 35.1 / 33.0; 2^9 and 2^10 33.4 / 35.1, 29.6 / 34.9, 29.3 / 29.1;
+// 2^21 and 2^12 at 4 / 15 %: 250 / 262, 279 / 270.  Two-pass sizes that the tensor
+// tiles would take make the other units slower there than here (2^8 and 5 % 2^14:
+// 58 / 50).
+bool radix_pays(const nttb_batch_job* jobs, uint32_t n_jobs) {
+    uint64_t below = 0, within = 0, above = 0;
+    for (uint32_t j = 0; j < n_jobs; j++) {
+        const uint32_t L = jobs[j].log_n;
+        if (L > 12 && L <= kRxMaxLog) return true;
+        if (L > 24) continue;  // refused later
+        const uint64_t work = ((uint64_t)jobs[j].n_limbs << L) * L * (jobs[j].flags & NTTB_BATCH_POLYMUL ? 3 : 1);
+        (L < kRxMinLog ? below : L <= kRxMaxLog ? within : above) += work;
+    }
+    return within && within >= below + above / 8;
+}
+
 // The tiles a job list runs: with tensor set (and a 256-thread configuration)
-// the register-radix tiles if any unit is in their range and the tables fit in
-// memory, else the tensor tiles; the configured CUDA-core tiles otherwise.
+// the register-radix tiles where they pay and the tables fit in memory, else the
+// tensor tiles; the configured CUDA-core tiles otherwise.
 Tiles pick_tiles(BatchPlan& P, const nttb_batch_job* jobs, uint32_t n_jobs, const nttb_batch_config& cfg) {
     if (!tensor_tiles(cfg)) return Tiles::kCore;
     uint32_t kinds = 0;
+    bool tensor = false;  // sizes that tensor tiles would take
+    for (uint32_t j = 0; j < n_jobs; j++) tensor = tensor || (jobs[j].log_n > 12 && jobs[j].log_n <= 20);
     for (uint32_t j = 0; j < n_jobs; j++) {
         if (jobs[j].log_n < kRxMinLog || jobs[j].log_n > kRxMaxLog || jobs[j].log_n > P.max_log) continue;
         if ((reinterpret_cast<uintptr_t>(jobs[j].data) | reinterpret_cast<uintptr_t>(jobs[j].pointwise)) & 15u) {
@@ -1592,11 +1615,11 @@ Tiles pick_tiles(BatchPlan& P, const nttb_batch_job* jobs, uint32_t n_jobs, cons
         if (jobs[j].flags & NTTB_BATCH_POLYMUL) kinds |= 3u << nega;
         else kinds |= 1u << (nega + (jobs[j].flags & NTTB_BATCH_INVERSE ? 1u : 0u));
     }
-    bool ok = kinds != 0;
+    bool ok = kinds != 0 && radix_pays(jobs, n_jobs);
     for (uint32_t k = 0; k < 4 && ok; k++)
         if (kinds >> k & 1u) ok = ensure_roots(P, k);
     if (ok) return Tiles::kRadix;
-    return ensure_images(P) ? Tiles::kTensor : Tiles::kCore;
+    return tensor && ensure_images(P) ? Tiles::kTensor : Tiles::kCore;
 }
 
 int create_batch(BatchPlan* P, const nttb_batch_job* jobs, uint32_t n_jobs, const nttb_batch_config& cfg, Batch** out,
@@ -1681,6 +1704,8 @@ struct BatchRunner {
     nttb_batch_config cfg{};
     Tiles kind = Tiles::kCore;
     const Variant* var = nullptr;
+    const Variant* core = nullptr;  // plans up to 2^12 (no workspace): for lists that radix does not pay for
+    int core_grid = 0;
     BUnit* d_units = nullptr;
     BTile* d_tiles = nullptr;
     uint32_t* d_ctr = nullptr;
@@ -1777,6 +1802,10 @@ int runner_create(BatchPlan* P, const nttb_batch_config& cfg, bool radix, BatchR
         return fail(NTTB_ERR_NO_MEMORY, "batch runner: allocation failed");
     }
     r->grid = resident_ctas(r->var, cfg.ctas_per_sm);
+    if (r->kind == Tiles::kRadix && P->max_log <= 12) {
+        r->core = find_variant(cfg.tile_elems, cfg.threads, cfg.group, 0);
+        r->core_grid = resident_ctas(r->core, cfg.ctas_per_sm);
+    }
     *out = r;
     return 0;
 }
@@ -1793,7 +1822,10 @@ size_t runner_device_bytes(const BatchRunner* r) { return r->ws_bytes + queue_by
 // Plans the jobs, uploads the queue from pinned staging and launches, all on
 // `s`.  One run per runner may be in flight: the staging is reused.
 int runner_run(BatchRunner* r, const nttb_batch_job* jobs, uint32_t n_jobs, cudaStream_t s) {
-    if (int rc = plan_batch(*r->plan, jobs, n_jobs, r->cfg, r->kind, r->units, r->tiles, &r->layout, nullptr)) return rc;
+    const bool core = r->core && !radix_pays(jobs, n_jobs);
+    const Variant* var = core ? r->core : r->var;
+    const Tiles kind = core ? Tiles::kCore : r->kind;
+    if (int rc = plan_batch(*r->plan, jobs, n_jobs, r->cfg, kind, r->units, r->tiles, &r->layout, nullptr)) return rc;
     if (r->tiles.empty()) return 0;
     if (r->units.size() > r->cap_units || r->tiles.size() > r->cap_tiles) {
         cudaStreamSynchronize(s);  // the previous run may still read the queue
@@ -1824,9 +1856,9 @@ int runner_run(BatchRunner* r, const nttb_batch_job* jobs, uint32_t n_jobs, cuda
                    cudaSuccess;
     ok = ok && cudaMemsetAsync(r->d_ctr, 0, (1 + 2 * r->units.size() + a.n_dis) * 4, s) == cudaSuccess;
     if (!ok) return fail(NTTB_ERR_CUDA, "batch runner: queue upload failed");
-    const int grid = (int)std::min<size_t>((size_t)r->grid, r->tiles.size());
+    const int grid = (int)std::min<size_t>((size_t)(core ? r->core_grid : r->grid), r->tiles.size());
     ProfScope prof("batch_queue", s);
-    r->var->fn<<<grid, cta_threads(r->var), smem_bytes(r->var), s>>>(a);
+    var->fn<<<grid, cta_threads(var), smem_bytes(var), s>>>(a);
     return cudaGetLastError() == cudaSuccess ? 0 : fail(NTTB_ERR_CUDA, "batch runner: launch failed");
 }
 
