@@ -207,11 +207,15 @@ int scalar_transform32_ws(const Plan32& p, uint32_t* data, void* ws, uint32_t n_
 size_t scalar_transform32_ws_bytes(const Plan32& p, uint32_t n_polys);
 
 // Register-radix passes on CUDA cores (radix.cuh): sizes 2^5 .. 2^20, n_polys x
-// n_limbs rows under the moduli `limbs`.  Sizes above 2^13 run two passes through
+// n_limbs rows under the moduli `limbs`.  Sizes above 2^13 (2^12: 64-bit) run two passes through
 // `mid`, n_polys * n_limbs * n words (uint32 for the 31-bit moduli, uint64 for the
 // wide ones): the destination, if the source is another buffer and the words have
 // its size, or a workspace.
-constexpr uint32_t kRadixMinLog = 5, kRadixMaxLog = 20, kRadixSingleMax = 13;
+constexpr uint32_t kRadixMinLog = 5, kRadixMaxLog = 20;
+// Largest size of one launch.  64-bit rows of 2^13 fill an SM with one block of 1024
+// threads and five rounds of barriers: two passes take 9.5 us for up to 40 rows and
+// 114 for 1200, one launch 14.5 and 133 (at 148 rows, one wave, 16.4 and 15.1).
+constexpr uint32_t kRadixSingleMax = 13, kRadixSingleMax64 = 12;
 inline bool radix_serves(uint32_t log_n) { return log_n >= kRadixMinLog && log_n <= kRadixMaxLog; }
 int radix_u32(const LimbDev<M32>* limbs, uint32_t log_n, uint32_t n_limbs, const void* src, void* dst, void* mid,
               uint32_t n_polys, bool inverse, cudaStream_t s);

@@ -13,9 +13,8 @@
 namespace nttb {
 namespace rdx {
 
-// Sizes served: one pass up to 2^kSingleMax (a tile holds the whole row), two
+// Sizes served: one pass up to 2^kRadixSingleMax (a tile holds the whole row), two
 // passes of 2^ceil(L/2) and 2^floor(L/2) points above.
-constexpr uint32_t kSingleMax = 13;
 constexpr uint32_t kThreadsMin = 128;  // rows are grouped into CTAs of at least this many threads
 
 // Failed range checks of this file's passes (0 in the release build).
@@ -194,7 +193,11 @@ int transform(const LimbDev<A>* limbs, uint32_t log_n, uint32_t n_limbs, const v
     case l: return launch_two<A, S, M, l, LGE>(a, mid, limbs, inverse, s);
     switch (log_n) {
         NTTB_SINGLE(5) NTTB_SINGLE(6) NTTB_SINGLE(7) NTTB_SINGLE(8) NTTB_SINGLE(9)
-        NTTB_SINGLE(10) NTTB_SINGLE(11) NTTB_SINGLE(12) NTTB_SINGLE(13)
+        NTTB_SINGLE(10) NTTB_SINGLE(11) NTTB_SINGLE(12)
+        case 13:
+            if constexpr (sizeof(typename A::elem) == 8) return launch_two<A, S, M, 13, LGE>(a, mid, limbs, inverse, s);
+            else if (inverse) return launch_single<A, S, 13, LGE, kInv>(a, limbs, s);
+            else return launch_single<A, S, 13, LGE, kFwd>(a, limbs, s);
         NTTB_TWO(14) NTTB_TWO(15) NTTB_TWO(16) NTTB_TWO(17) NTTB_TWO(18) NTTB_TWO(19) NTTB_TWO(20)
         default: return 1;
     }

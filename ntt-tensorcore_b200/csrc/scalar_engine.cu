@@ -370,8 +370,9 @@ int transform_generic(uint32_t log_n, uint32_t n_limbs, bool negacyclic, const L
 
 // Words that a transform stages outside source and destination: the two-pass
 // sizes' first pass, unless it can go to the destination.
-static size_t staged_words(uint32_t log_n, uint32_t e_max, uint32_t n_limbs, uint32_t n_polys) {
-    const bool two = radix_serves(log_n) ? log_n > kRadixSingleMax : (1u << log_n) > e_max;
+// `single`: log2 of the largest size that the register-radix passes run as one.
+static size_t staged_words(uint32_t log_n, uint32_t single, uint32_t e_max, uint32_t n_limbs, uint32_t n_polys) {
+    const bool two = radix_serves(log_n) ? log_n > single : (1u << log_n) > e_max;
     return two ? ((size_t)n_polys * n_limbs) << log_n : 0;
 }
 
@@ -406,7 +407,7 @@ int scalar_transform32(Plan32& p, const void* src, void* dst, bool src_u64, uint
                        cudaStream_t s) {
     if (n_polys > 65535 || p.n_limbs > 65535) return 1;
     const bool radix = radix_serves(p.log_n);
-    const size_t words = staged_words(p.log_n, 8192, p.n_limbs, n_polys);
+    const size_t words = staged_words(p.log_n, kRadixSingleMax, 8192, p.n_limbs, n_polys);
     if (!words || (src != dst && !(radix && src_u64)))
         return run32(p.d_limbs, p.log_n, p.n_limbs, p.negacyclic, src, dst, dst, src_u64, n_polys, inverse, s);
     const size_t es = src_u64 ? 8 : 4;
@@ -419,7 +420,7 @@ int scalar_transform32(Plan32& p, const void* src, void* dst, bool src_u64, uint
 
 int scalar_round_trip32(Plan32& p, uint32_t* data, uint32_t n_polys, cudaStream_t s) {
     if (!radix_serves(p.log_n) || n_polys > 65535 || p.n_limbs > 65535) return 1;
-    if (!staged_words(p.log_n, 8192, p.n_limbs, n_polys))
+    if (!staged_words(p.log_n, kRadixSingleMax, 8192, p.n_limbs, n_polys))
         return radix_round_trip_u32(p.d_limbs, p.log_n, p.n_limbs, data, nullptr, n_polys, s);
     return staged_groups(p, n_polys, 4, s,
                          [&](const LimbDev<M32>* limbs, uint32_t n_limbs, size_t off, uint32_t polys, void* mid) {
@@ -436,7 +437,7 @@ int scalar_transform32_ws(const Plan32& p, uint32_t* data, void* ws, uint32_t n_
 }
 
 size_t scalar_transform32_ws_bytes(const Plan32& p, uint32_t n_polys) {
-    return staged_words(p.log_n, 8192, p.n_limbs, n_polys) * sizeof(uint32_t);
+    return staged_words(p.log_n, kRadixSingleMax, 8192, p.n_limbs, n_polys) * sizeof(uint32_t);
 }
 
 static int run64(const LimbDev<M64>* limbs, uint32_t log_n, uint32_t n_limbs, bool negacyclic, const uint64_t* src,
@@ -450,7 +451,7 @@ int scalar_transform64(Plan64& p, const void* src_, void* dst_, uint32_t n_polys
     if (n_polys > 65535 || p.n_limbs > 65535) return 1;
     const uint64_t* src = static_cast<const uint64_t*>(src_);
     uint64_t* dst = static_cast<uint64_t*>(dst_);
-    if (!staged_words(p.log_n, 4096, p.n_limbs, n_polys) || src != dst)
+    if (!staged_words(p.log_n, kRadixSingleMax64, 4096, p.n_limbs, n_polys) || src != dst)
         return run64(p.d_limbs, p.log_n, p.n_limbs, p.negacyclic, src, dst, dst, n_polys, inverse, s);
     return staged_groups(p, n_polys, 8, s,
                          [&](const LimbDev<M64>* limbs, uint32_t n_limbs, size_t off, uint32_t polys, void* mid) {
