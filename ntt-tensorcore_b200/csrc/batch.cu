@@ -110,8 +110,8 @@ __device__ __forceinline__ uint32_t pw(const BModulus& M, const M32& ar, uint32_
 }
 
 // Register-radix tiles (batch_radix.cuh): per-modulus roots by kind (bit 0
-// inverse, bit 1 negacyclic; null until a batch needs the kind) and the
-// inverse's scale [negacyclic][product][log2 n]: Shoup pairs of c and c W, c =
+// inverse, bit 1 negacyclic; null until a batch needs the kind), the pairs up to 2^10
+// and the quotients up to 2^13 (those of larger sizes: Mods::large), and the inverse's scale [negacyclic][product][log2 n]: Shoup pairs of c and c W, c =
 // n^-1 (times 2^32 for a product), W the inverse's root of its last stage.
 struct RxModulus {
     M32 ar;
@@ -1010,14 +1010,14 @@ __global__ void __launch_bounds__(T, (G == 1 ? 1536u : G == 3 ? 768u : 512u) / T
 
 // Roots of one kind for every modulus (blockIdx.y): quotients floor(w 2^32 / q)
 // of the entries 2^s + i, s < log_r, and the Shoup pairs (w, quotient) of the
-// first 2^log_p.  The quotient is (w 2^32 mod q) (-q^-1) mod 2^32.
+// first 2^log_p (pairs null: none).  The quotient is (w 2^32 mod q) (-q^-1) mod 2^32.
 __global__ void rx_roots_kernel(const BModulus* mods, uint32_t max_log, uint32_t log_r, uint32_t log_p, uint32_t kind,
                                 uint2* pairs, uint32_t* quot) {
     const BModulus& M = mods[blockIdx.y];
     const M32 ar = M.ar;
     const bool nega = kind & 2u;
     const uint32_t base = nega ? (kind & 1u ? PW_PSI_INV : PW_PSI) : (kind & 1u ? PW_OMEGA_INV : PW_OMEGA);
-    pairs += (size_t)blockIdx.y << log_p;
+    if (pairs) pairs += (size_t)blockIdx.y << log_p;
     quot += (size_t)blockIdx.y << log_r;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < (1u << log_r); i += gridDim.x * blockDim.x) {
         uint32_t r = 0;
@@ -1026,7 +1026,7 @@ __global__ void rx_roots_kernel(const BModulus* mods, uint32_t max_log, uint32_t
             r = pw(M, ar, base, (nega ? 1u + 2u * k : k) << (max_log - s - 1));
         }
         quot[i] = r * ar.qinv;
-        if (i < (1u << log_p)) pairs[i] = make_uint2(ar.mul(r, 1u), r * ar.qinv);
+        if (pairs && i < (1u << log_p)) pairs[i] = make_uint2(ar.mul(r, 1u), r * ar.qinv);
     }
 }
 
@@ -1126,6 +1126,8 @@ struct BatchPlan::Mods {
     BModulus* d = nullptr;
     RxModulus* rx = nullptr;         // device copy of rx_host
     std::vector<RxModulus> rx_host;
+    uint32_t* large[4][25] = {};     // [kind][L]: quotients of the roots up to 2^L, L > kRxLogTile, null until a
+                                     // batch needs a size that no larger table serves
     std::mutex mu;                   // guards the lazy tables (rx, images)
 };
 
@@ -1189,6 +1191,14 @@ bool tensor_tiles(const nttb_batch_config& cfg) {
 // Which tiles a batch runs: the configured CUDA-core ones alone, with tensor
 // tiles for the two-pass units, or the register-radix ones.
 enum class Tiles { kCore, kTensor, kRadix };
+
+// log2 of the size whose root table serves units of 2^L (L > kRxLogTile): the
+// smallest one made that is large enough; 0: none.
+uint32_t root_log(const BatchPlan::Mods& M, uint32_t kind, uint32_t L) {
+    for (uint32_t l = L; l <= kRxMaxLog; l++)
+        if (M.large[kind][l]) return l;
+    return 0;
+}
 
 // Pass geometry of a unit of 2^L residues (rows: limbs per single-pass tile).
 struct UnitShape {
@@ -1308,7 +1318,9 @@ int plan_batch(BatchPlan& P, const nttb_batch_job* jobs, uint32_t n_jobs, const 
                 const uint32_t nega = uf & UF_NEGA ? 1u : 0u, k = 2 * nega + (uf & UF_INV ? 1u : 0u);
                 u.ar = M.ar;
                 u.pairs = M.pairs[k];
-                u.quot = M.quot[k];
+                std::lock_guard<std::mutex> lock(P.mods->mu);  // another batch may be making a table
+                const uint32_t l = root_log(*P.mods, k, L);
+                u.quot = P.mods->large[k][l] + ((size_t)u.mod0 << l);
                 u.one = make_uint2(1u, (uint32_t)((1ull << 32) / M.ar.q));
                 u.scale[0] = M.scale[nega][pre_mul ? 1 : 0][L][0];
                 u.scale[1] = M.scale[nega][pre_mul ? 1 : 0][L][1];
@@ -1505,18 +1517,20 @@ bool ensure_images(BatchPlan& P) {
     return true;
 }
 
-// Sizes of the register-radix tiles' root tables, per kind of root: quotients of
-// the roots up to 2^log_r and pairs of those up to 2^log_p for each modulus.
-uint32_t root_log_r(const BatchPlan& P) { return std::min(P.max_log, kRxMaxLog); }
+// Sizes of the register-radix tiles' root tables, per kind of root: for each modulus
+// pairs up to 2^root_log_p, quotients up to 2^root_log_r and, for sizes L above
+// that, quotients up to 2^L.
+uint32_t root_log_r(const BatchPlan& P) { return std::min(P.max_log, kRxLogTile); }
 uint32_t root_log_p(const BatchPlan& P) { return std::min(P.max_log, kRxMaxLog / 2); }
-size_t root_bytes(const BatchPlan& P, size_t nm) {
-    return (nm << root_log_p(P)) * sizeof(uint2) + (nm << root_log_r(P)) * sizeof(uint32_t);
+size_t root_bytes(const BatchPlan& P, uint32_t L) {
+    const size_t nm = P.limbs.size();
+    return (nm << root_log_p(P)) * sizeof(uint2) + (nm << root_log_r(P)) * 4 + (L > kRxLogTile ? (nm << L) * 4 : 0);
 }
 
-// Device tables of the register-radix tiles for one kind of root (bit 0
-// inverse, bit 1 negacyclic), made on first use: per modulus 4 bytes per root
-// up to 2^min(max_log, 20) and 8 per root up to 2^10 (the uniform passes').
-bool ensure_roots(BatchPlan& P, uint32_t kind) {
+// Device tables of the register-radix tiles for one kind of root (bit 0 inverse,
+// bit 1 negacyclic) and sizes up to 2^L, made on first use: what a plan holds goes
+// by the sizes that its batches have, not by its largest.
+bool ensure_roots(BatchPlan& P, uint32_t kind, uint32_t L) {
     BatchPlan::Mods& M = *P.mods;
     std::lock_guard<std::mutex> lock(M.mu);
     const size_t nm = P.limbs.size();
@@ -1543,36 +1557,55 @@ bool ensure_roots(BatchPlan& P, uint32_t kind) {
                 }
         }
     }
-    if (M.rx_host[0].quot[kind]) return true;
-    const uint32_t log_r = root_log_r(P), log_p = root_log_p(P);
-    uint2* pairs = nullptr;
-    uint32_t* quot = nullptr;
-    bool ok = cudaMalloc(&pairs, (nm << log_p) * sizeof(uint2)) == cudaSuccess &&
-              cudaMalloc(&quot, (nm << log_r) * sizeof(uint32_t)) == cudaSuccess;
-    ok = ok && (M.rx || cudaMalloc(&M.rx, nm * sizeof(RxModulus)) == cudaSuccess);
-    if (ok) {
+    auto fill = [&](uint32_t log_r, uint32_t log_p, uint2* pairs, uint32_t* quot) {
         const dim3 grid(std::max(1u, std::min(64u, (1u << log_r) / 256u)), (unsigned)nm);
         rx_roots_kernel<<<grid, 256>>>(M.d, P.max_log, log_r, log_p, kind, pairs, quot);
-        for (size_t l = 0; l < nm; l++) {
-            M.rx_host[l].pairs[kind] = pairs + (l << log_p);
-            M.rx_host[l].quot[kind] = quot + (l << log_r);
+    };
+    if (!M.rx_host[0].quot[kind]) {
+        const uint32_t log_r = root_log_r(P), log_p = root_log_p(P);
+        uint2* pairs = nullptr;
+        uint32_t* quot = nullptr;
+        bool ok = cudaMalloc(&pairs, (nm << log_p) * sizeof(uint2)) == cudaSuccess &&
+                  cudaMalloc(&quot, (nm << log_r) * sizeof(uint32_t)) == cudaSuccess;
+        ok = ok && (M.rx || cudaMalloc(&M.rx, nm * sizeof(RxModulus)) == cudaSuccess);
+        if (ok) {
+            fill(log_r, log_p, pairs, quot);
+            for (size_t l = 0; l < nm; l++) {
+                M.rx_host[l].pairs[kind] = pairs + (l << log_p);
+                M.rx_host[l].quot[kind] = quot + (l << log_r);
+            }
+            ok = cudaMemcpy(M.rx, M.rx_host.data(), nm * sizeof(RxModulus), cudaMemcpyHostToDevice) == cudaSuccess &&
+                 cudaStreamSynchronize(0) == cudaSuccess;
         }
-        ok = cudaMemcpy(M.rx, M.rx_host.data(), nm * sizeof(RxModulus), cudaMemcpyHostToDevice) == cudaSuccess &&
-             cudaStreamSynchronize(0) == cudaSuccess;
+        if (!ok) {
+            cudaGetLastError();
+            for (RxModulus& R : M.rx_host) {
+                R.pairs[kind] = nullptr;
+                R.quot[kind] = nullptr;
+            }
+            cudaFree(pairs);
+            cudaFree(quot);
+            return false;
+        }
+        P.allocations.push_back(pairs);
+        P.allocations.push_back(quot);
+        P.table_bytes += root_bytes(P, 0);
+    }
+    if (L <= kRxLogTile || root_log(M, kind, L)) return true;
+    uint32_t* quot = nullptr;
+    bool ok = cudaMalloc(&quot, (nm << L) * sizeof(uint32_t)) == cudaSuccess;
+    if (ok) {
+        fill(L, 0, nullptr, quot);
+        ok = cudaGetLastError() == cudaSuccess && cudaStreamSynchronize(0) == cudaSuccess;
     }
     if (!ok) {
         cudaGetLastError();
-        for (RxModulus& R : M.rx_host) {
-            R.pairs[kind] = nullptr;
-            R.quot[kind] = nullptr;
-        }
-        cudaFree(pairs);
         cudaFree(quot);
         return false;
     }
-    P.allocations.push_back(pairs);
+    M.large[kind][L] = quot;
     P.allocations.push_back(quot);
-    P.table_bytes += root_bytes(P, nm);
+    P.table_bytes += (nm << L) * sizeof(uint32_t);
     return true;
 }
 
@@ -1602,22 +1635,25 @@ bool radix_pays(const nttb_batch_job* jobs, uint32_t n_jobs) {
 // tensor tiles; the configured CUDA-core tiles otherwise.
 Tiles pick_tiles(BatchPlan& P, const nttb_batch_job* jobs, uint32_t n_jobs, const nttb_batch_config& cfg) {
     if (!tensor_tiles(cfg)) return Tiles::kCore;
-    uint32_t kinds = 0;
+    uint32_t largest[4] = {};  // by kind of root; 0: not in use
+    bool any = false;
     bool tensor = false;  // sizes that tensor tiles would take
     for (uint32_t j = 0; j < n_jobs; j++) tensor = tensor || (jobs[j].log_n > 12 && jobs[j].log_n <= 20);
     for (uint32_t j = 0; j < n_jobs; j++) {
         if (jobs[j].log_n < kRxMinLog || jobs[j].log_n > kRxMaxLog || jobs[j].log_n > P.max_log) continue;
         if ((reinterpret_cast<uintptr_t>(jobs[j].data) | reinterpret_cast<uintptr_t>(jobs[j].pointwise)) & 15u) {
-            kinds = 0;  // the tiles copy 16 bytes at a time
+            any = false;  // the tiles copy 16 bytes at a time
             break;
         }
+        any = true;
         const uint32_t nega = (jobs[j].flags & NTTB_NEGACYCLIC) && P.negacyclic ? 2u : 0u;
-        if (jobs[j].flags & NTTB_BATCH_POLYMUL) kinds |= 3u << nega;
-        else kinds |= 1u << (nega + (jobs[j].flags & NTTB_BATCH_INVERSE ? 1u : 0u));
+        for (uint32_t inv = 0; inv < 2; inv++)
+            if (jobs[j].flags & NTTB_BATCH_POLYMUL || (jobs[j].flags & NTTB_BATCH_INVERSE ? 1u : 0u) == inv)
+                largest[nega + inv] = std::max(largest[nega + inv], jobs[j].log_n);
     }
-    bool ok = kinds != 0 && radix_pays(jobs, n_jobs);
+    bool ok = any && radix_pays(jobs, n_jobs);
     for (uint32_t k = 0; k < 4 && ok; k++)
-        if (kinds >> k & 1u) ok = ensure_roots(P, k);
+        if (largest[k]) ok = ensure_roots(P, k, largest[k]);
     if (ok) return Tiles::kRadix;
     return tensor && ensure_images(P) ? Tiles::kTensor : Tiles::kCore;
 }
@@ -1760,8 +1796,8 @@ int runner_reserve(BatchRunner* r, size_t units, size_t tiles) {
 // A runner's tiles: its job lists are all of the plan's twist, in both directions.
 static Tiles runner_tiles(BatchPlan* P, const nttb_batch_config& cfg, bool radix) {
     if (!tensor_tiles(cfg)) return Tiles::kCore;
-    if (radix && P->max_log >= kRxMinLog && ensure_roots(*P, P->negacyclic ? 2 : 0) &&
-        ensure_roots(*P, P->negacyclic ? 3 : 1))
+    const uint32_t L = std::min(P->max_log, kRxMaxLog);
+    if (radix && L >= kRxMinLog && ensure_roots(*P, P->negacyclic ? 2 : 0, L) && ensure_roots(*P, P->negacyclic ? 3 : 1, L))
         return Tiles::kRadix;
     return ensure_images(*P) ? Tiles::kTensor : Tiles::kCore;
 }
@@ -1772,7 +1808,7 @@ bool batch_plan_prepare(BatchPlan* P, const nttb_batch_config& cfg, uint32_t run
     // what requests would be left on either kind of tiles
     auto left = [&](Tiles kind) {
         size_t bytes = batch_plan_device_bytes(P) + runners * (ws_layout(*P, cfg, kind, nullptr).words * 4 + queue_bytes());
-        if (kind == Tiles::kRadix) bytes += 2 * root_bytes(*P, nm) + nm * sizeof(RxModulus);
+        if (kind == Tiles::kRadix) bytes += 2 * root_bytes(*P, std::min(P->max_log, kRxMaxLog)) + nm * sizeof(RxModulus);
         if (kind == Tiles::kTensor) bytes += nm * (size_t)kImgPerMod;
         return budget > bytes ? budget - bytes : 0;
     };
