@@ -41,7 +41,8 @@ enum {
 
 /* Inner-DFT engines.  AUTO takes the CUDA-core engine for RNS plans and wide
  * plans.  Its in-place calls above 2^13 stage a pass in a workspace of the plan's:
- * one for each of the first four streams, then one per call, in stream order;
+ * one for each of the first 32 streams (512 MB in all), else one per call, in
+ * stream order;
  * one of each graph's own where the stream is captured (held until the graph and
  * its executables are destroyed).  Each is at most 2^25 words (or one row): longer
  * calls run in groups of rows.  Streams, threads and graphs may share a plan.

@@ -236,7 +236,7 @@ static cudaMemPool_t plan_pool(PlanPool& pp) {  // pp.mu held
     }
     pp.device = props.location.id;
     // what one call frees, the next takes; the pool goes with the plan
-    uint64_t keep = 2 * PlanPool::kSlots * kStagedWordsMax * 8;
+    uint64_t keep = 2 * PlanPool::kHeldMax;
     int off = 0;            // streams never wait for one another for memory
     cudaMemPoolSetAttribute(pp.pool, cudaMemPoolAttrReleaseThreshold, &keep);
     cudaMemPoolSetAttribute(pp.pool, cudaMemPoolReuseAllowInternalDependencies, &off);
@@ -262,17 +262,21 @@ void CUDART_CB drop_graph_ref(void* p) {  // no CUDA calls here
 // stream of one capture run one after the other and share it.  The stream's handle
 // stands for it, which does not change hands during a capture (the per-thread
 // handle is one of several streams; cudaStreamGetId invalidates a capture).
-static void* graph_workspace(const std::shared_ptr<GraphWorkspaces>& all, size_t bytes, unsigned long long capture,
-                             cudaGraph_t graph, cudaStream_t stream) {
+static GraphWorkspaces::Buf* graph_workspace(const std::shared_ptr<GraphWorkspaces>& all, size_t bytes,
+                                             unsigned long long capture, cudaGraph_t graph, cudaStream_t stream) {
     GraphWorkspaces::Buf* b = nullptr;
     {
         std::lock_guard<std::mutex> lock(all->mu);
         for (GraphWorkspaces::Buf& t : all->bufs) {
             if (t.bytes < bytes) continue;
-            if (t.held && t.capture == capture && t.stream == stream && stream != cudaStreamPerThread) return t.ptr;
+            if (t.held && t.capture == capture && t.stream == stream && stream != cudaStreamPerThread) return &t;
             if (!t.held && (!b || t.bytes < b->bytes)) b = &t;
         }
-        if (b) b->held = true;
+        if (b) {
+            b->held = true;
+            b->capture = capture;
+            b->stream = stream;
+        }
     }
     if (!b) {
         // no capture depends on the allocation: it may be made in the middle of one
@@ -288,9 +292,9 @@ static void* graph_workspace(const std::shared_ptr<GraphWorkspaces>& all, size_t
         b->ptr = ptr;
         b->bytes = bytes;
         b->held = true;
+        b->capture = capture;
+        b->stream = stream;
     }
-    b->capture = capture;
-    b->stream = stream;
     GraphRef* ref = new GraphRef{all, b};
     cudaUserObject_t obj = nullptr;
     if (cudaUserObjectCreate(&obj, ref, drop_graph_ref, 1, cudaUserObjectNoDestructorSync) != cudaSuccess) {
@@ -301,10 +305,10 @@ static void* graph_workspace(const std::shared_ptr<GraphWorkspaces>& all, size_t
         cudaUserObjectRelease(obj, 1);
         return nullptr;
     }
-    return b->ptr;
+    return b;
 }
 
-StreamWorkspace::StreamWorkspace(PlanPool& pp, size_t bytes, cudaStream_t s) : lock_(pp.mu), stream_(s) {
+StreamWorkspace::StreamWorkspace(PlanPool& pp, size_t bytes, cudaStream_t s) : stream_(s) {
     unsigned long long id = 0, capture = 0;
     cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
     cudaGraph_t graph = nullptr;
@@ -313,36 +317,68 @@ StreamWorkspace::StreamWorkspace(PlanPool& pp, size_t bytes, cudaStream_t s) : l
         return;
     }
     if (status != cudaStreamCaptureStatusNone) {
-        if (status == cudaStreamCaptureStatusActive) ptr = graph_workspace(pp.graphs, bytes, capture, graph, s);
-        if (!ptr) cudaGetLastError();
+        GraphWorkspaces::Buf* b = nullptr;
+        if (status == cudaStreamCaptureStatusActive) {
+            std::lock_guard<std::mutex> lock(pp.mu);
+            b = graph_workspace(pp.graphs, bytes, capture, graph, s);
+        }
+        if (b) {
+            lock_ = std::unique_lock<std::mutex>(b->mu);
+            ptr = b->ptr;
+        } else {
+            cudaGetLastError();
+        }
         return;
     }
-    if (!plan_pool(pp) || cudaStreamGetId(s, &id) != cudaSuccess) {
+    if (cudaStreamGetId(s, &id) != cudaSuccess) {
         cudaGetLastError();
         return;
     }
     PlanPool::Slot* slot = nullptr;
-    for (PlanPool::Slot& t : pp.slot)
-        if (t.ptr && t.stream == id) slot = &t;
-    if (!slot)
-        for (PlanPool::Slot& t : pp.slot)
-            if (!t.ptr && !slot) slot = &t;
-    if (slot && slot->bytes >= bytes) {
-        ptr = slot->ptr;
-        return;
+    {
+        std::lock_guard<std::mutex> lock(pp.mu);
+        if (!plan_pool(pp)) return;
+        for (int i = 0; i < pp.used && !slot; i++)
+            if (pp.slot[i].stream == id) slot = &pp.slot[i];
+        if (!slot && pp.used < PlanPool::kSlots && pp.held + bytes <= PlanPool::kHeldMax) {
+            slot = &pp.slot[pp.used++];
+            slot->stream = id;
+        }
     }
-    if (slot && slot->ptr) {  // grown: freed behind the stream's earlier calls
-        cudaFreeAsync(slot->ptr, s);
-        *slot = PlanPool::Slot{};
+    if (slot) {
+        lock_ = std::unique_lock<std::mutex>(slot->mu);
+        if (slot->bytes >= bytes) {
+            ptr = slot->ptr;
+            return;
+        }
+        bool fits;
+        {
+            std::lock_guard<std::mutex> lock(pp.mu);
+            fits = pp.held - slot->bytes + bytes <= PlanPool::kHeldMax;
+            if (fits) pp.held += bytes - slot->bytes;
+        }
+        if (fits) {
+            if (slot->ptr) cudaFreeAsync(slot->ptr, s);  // behind the stream's earlier calls
+            slot->ptr = nullptr;
+            slot->bytes = 0;
+            if (cudaMallocFromPoolAsync(&slot->ptr, bytes, pp.pool, s) == cudaSuccess) {
+                ptr = slot->ptr;
+                slot->bytes = bytes;
+            } else {
+                cudaGetLastError();
+                slot->ptr = nullptr;
+                std::lock_guard<std::mutex> lock(pp.mu);
+                pp.held -= bytes;
+            }
+            return;
+        }
+        lock_.unlock();
     }
-    if (cudaMallocFromPoolAsync(&ptr, bytes, pp.pool, s) != cudaSuccess) {
+    if (cudaMallocFromPoolAsync(&ptr, bytes, pp.pool, s) == cudaSuccess) {
+        per_call_ = true;
+    } else {
         cudaGetLastError();
         ptr = nullptr;
-    } else if (slot) {
-        *slot = {id, ptr, bytes};
-    } else {
-        per_call_ = true;
-        lock_.unlock();
     }
 }
 
@@ -374,7 +410,13 @@ static void free_pool(PlanPool& pp) {
         cudaGetLastError();
     }
     if (dev != pp.device) cudaSetDevice(dev);
-    for (PlanPool::Slot& t : pp.slot) t = PlanPool::Slot{};
+    for (PlanPool::Slot& t : pp.slot) {
+        t.stream = 0;
+        t.ptr = nullptr;
+        t.bytes = 0;
+    }
+    pp.used = 0;
+    pp.held = 0;
     pp.pool = nullptr;
     pp.tried = false;
 }

@@ -89,25 +89,30 @@ struct GraphWorkspaces {
         unsigned long long capture = 0;  // the calls that share it: one stream of one capture
         cudaStream_t stream = nullptr;
         bool held = false;
+        std::mutex mu;  // held by the call that is being captured
     };
     std::mutex mu;
     std::list<Buf> bufs;
 };
 
 // The pool behind a plan's stream-ordered workspaces (StreamWorkspace), and the
-// workspaces that the first kSlots streams keep.
+// workspaces that its first kSlots streams keep, kHeldMax bytes in all.
 struct PlanPool {
-    static constexpr int kSlots = 4;
+    static constexpr int kSlots = 32;
+    static constexpr size_t kHeldMax = 512u << 20;
     struct Slot {
         unsigned long long stream = 0;  // cudaStreamGetId: never reused
         void* ptr = nullptr;
         size_t bytes = 0;
+        std::mutex mu;  // guards ptr and bytes; held by the call that uses them
     };
     cudaMemPool_t pool = nullptr;
     int device = -1;
     bool tried = false;
     Slot slot[kSlots];
-    std::mutex mu;
+    int used = 0;     // slots that have a stream
+    size_t held = 0;  // bytes of all slots
+    std::mutex mu;    // guards what is above but the slots' own memory
     std::shared_ptr<GraphWorkspaces> graphs = std::make_shared<GraphWorkspaces>();
 };
 
@@ -153,12 +158,12 @@ int engine_status(int rc, const char* what);
 
 // A workspace for the call that constructs it, until the call has enqueued its
 // launches: stream-ordered memory from a pool that the plan owns.  The first
-// kSlots streams that use a plan keep theirs (an allocation and a free cost a
-// call 2 us on the host: in place 1 x 2^16 6.3 -> 8.7 us); it is locked meanwhile,
-// so that threads on one stream enqueue one after the other.  Further streams
-// allocate per call.  So calls on several streams or threads never share one.
-// The pool keeps what kSlots streams and as many calls beyond them need
-// (kStagedWordsMax each) until the plan is destroyed, and gives back the rest.
+// kSlots streams that use a plan keep theirs, as far as kHeldMax goes (an allocation
+// and a free cost a call 2 us on the host, 10 where streams take turns: in place
+// 8 x 2^16 on ten streams 6 -> 17 us a call); it is locked meanwhile, so that threads
+// on one stream enqueue one after the other.  Further calls allocate their own.  So
+// calls on several streams or threads never share one.  The pool keeps twice
+// kHeldMax until the plan is destroyed, and gives back the rest.
 // While the stream is being captured it is a buffer that the graph holds
 // (GraphWorkspaces), so that a captured call needs no earlier one and replays race
 // neither with other graphs nor with calls outside.  ptr: null on failure.
