@@ -372,17 +372,20 @@ __global__ void __launch_bounds__(MAXT) klimb_pass(const __grid_constant__ PassA
             if (wide) {
 #pragma unroll
                 for (int m = 0; m + 4 <= RAW; m += 4) {
-                    const uint4 x = __ldg(reinterpret_cast<const uint4*>(w + m));
+                    const uint4* at = reinterpret_cast<const uint4*>(w + m);
+                    const uint4 x = WHERE == kStages ? __ldg(at) : __ldcg(at);
                     raw[q][m] = x.x, raw[q][m + 1] = x.y, raw[q][m + 2] = x.z, raw[q][m + 3] = x.w;
                 }
             } else {
 #pragma unroll
-                for (int m = 0; m < K; m++) raw[q][m] = __ldg(w + m);
+                for (int m = 0; m < K; m++) raw[q][m] = WHERE == kStages ? __ldg(w + m) : __ldcg(w + m);
             }
         }
     };
     // The table is older than the pass before this one, which waited for it; the
-    // first pass of a transform has no such pass.
+    // first pass of a transform has no such pass.  Its blocks may be older than the
+    // table, so it reads past the read-only path, which asks for memory that does not
+    // change while a grid is on the GPU.
     if constexpr (WHERE == kStages) fetch_roots();
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
