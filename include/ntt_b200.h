@@ -42,10 +42,10 @@ enum {
 /* Inner-DFT engines.  AUTO takes the CUDA-core engine for RNS plans and wide
  * plans.  Its in-place calls above 2^13 stage a pass in a workspace of the plan's:
  * one for each of the first 32 streams (512 MB in all), else one per call, in
- * stream order;
- * one of each graph's own where the stream is captured (held until the graph and
- * its executables are destroyed).  Each is at most 2^25 words (or one row): longer
- * calls run in groups of rows.  Streams, threads and graphs may share a plan.
+ * stream order; one of each graph's own where the stream is captured (held until
+ * the graph and its executables are destroyed).  Each is at most 2^25 words (or one
+ * row): longer calls run in groups of rows.  Streams, threads and graphs may share
+ * a plan.  (64-bit plans: above 2^12.)
  * Where that memory cannot be had, and for the drop-in's uint64 words and the host
  * stream, AUTO takes the INT8 tensor-core kernel at N = 2^16 from 8 (polynomial,
  * limb) units on, the batch queue at N = 2^17 .. 2^20 once a call holds 2^20
@@ -53,7 +53,7 @@ enum {
  * queues are built on first use: call once before a capture.  The queue route
  * keeps up to eight prepared queues per plan (one per source, destination, count,
  * direction), each with its own workspace ring of up to 16 x N words.  Destroying
- * a plan waits for its calls. */
+ * a plan waits for its calls; graphs that hold some are not replayed afterwards. */
 enum {
     NTTB_ENGINE_AUTO = 0,
     NTTB_ENGINE_SCALAR = 1, /* CUDA-core radix-2 stages in registers and shared memory */

@@ -38,8 +38,8 @@
 // barrier and one shared-memory round trip per group.  Twiddles and twists
 // come from two-level power tables (8 KB per base and modulus, L2-resident).
 //
-// Batches with units of 2^10 .. 2^20 residues run register-radix tiles instead
-// (batch_radix.cuh, the default configuration): 145 - 260 G residues/s by size,
+// Batches whose work lies at 2^10 .. 2^20 (radix_pays) run register-radix tiles
+// instead (batch_radix.cuh, the default configuration): 145 - 260 G residues/s by size,
 // against 80 - 100 on the tensor tiles below and less on the CUDA-core tiles.
 // 96 mixed polynomials (283 M residues): 3.01 -> 1.53 ms; twelve products of
 // 12 x 2^14: 107 -> 49 us.  The tensor tiles serve the named tiles engine and

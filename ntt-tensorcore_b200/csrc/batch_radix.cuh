@@ -16,7 +16,7 @@
 // whole rows, which use one root per residue, read the pair's quotient ws =
 // floor(w 2^32 / q) alone, 4 bytes, and make w = floor(ws q / 2^32) + 1 (ws q =
 // w 2^32 - r with 0 < r < q).  Tables are per modulus, direction and twist, and
-// one table serves every size: root 2^s + i is zeta^(1 + 2 i), zeta of order
+// one table serves its size and those below: root 2^s + i is zeta^(1 + 2 i), zeta of order
 // 2^(s+2) (negacyclic), or zeta^i, zeta of order 2^(s+1) (cyclic).
 //
 // A seventeenth warp feeds the tiles: while the 512 threads run one, it claims

@@ -18,9 +18,11 @@ static int env_engine() {
 }
 
 // The CUDA-core engine's register-radix passes (radix.cuh) are the fastest at
-// every size (us, forward, this engine / the other): 8 x 2^16 6.6 / 16.6 (INT8),
-// 24 x 2^16 9.7 / 17.4 (INT8), 192 x 2^16 54 / 95 (INT8), 33 x 2^17 22.5 / 62
-// (tensor tiles), 1 x 2^20 10 / 25 (queue).  In place they stage their first pass
+// every size (us, forward, the same buffers again and again, this engine / the
+// other): 4 x 2^16 6.7 / 16.7 (INT8), 33 x 2^16 12.5 / 18.0 (INT8), 256 x 2^16 73 / 129
+// (INT8), 33 x 2^17 22.8 / 61.9 (tensor tiles), 1 x 2^20 10.1 / 26.0 (queue).  Calls of
+// 8 rows that take turns on four or more streams are bound by the host, where two
+// launches cost 7 - 10 us and the INT8 kernel's one 4 - 6.  In place they stage their first pass
 // in a workspace; calls for which it could not be had and the drop-in's and the
 // host stream's calls, whose engines those entry points name, take the INT8
 // cluster kernel at 2^16 from kInt8MinUnits (polynomial, limb) units on and the

@@ -28,8 +28,8 @@
 // against 2^64); a root is divided by 2^8 mod p as it is loaded.  Other moduli
 // stay on the 24-bit limbs.
 // Measured: one product, a warp alone on its scheduler, 832 cycles (544 of them the
-// multiplier's); K = 11 at 2^15 63.6 -> 18.4 us, at 2^18 305 -> 75; K = 3 at 2^15
-// 26 -> 10 (the host), at 2^20 175 -> 68 (24-bit limbs, radix-2 sweeps of gathered
+// multiplier's); K = 11 at 2^15 63.6 -> 18.2 us, at 2^17 156 -> 47, at 2^18 305 -> 75;
+// K = 3 at 2^15 26 -> 10 (the host), at 2^20 175 -> 68 (24-bit limbs, radix-2 sweeps of gathered
 // roots behind a bit reversal of its own before).
 #include <cuda_runtime.h>
 
@@ -171,7 +171,9 @@ struct Form256 : Words<11, 8> {
             : "r"(x1), "r"(x3), "r"(x5), "r"(x7), "r"(y));
     }
 
-    // x = a b 2^-256 mod p in [0, 2p) for a < p, b < 2^256.  The running sum is kept
+    // x = a b 2^-256 mod p in [0, 2p) for a < p, b < 2^256, by coarsely integrated
+    // operand scanning (Koc, Acar, Kaliski, "Analyzing and comparing Montgomery
+    // multiplication algorithms", IEEE Micro 1996).  The running sum is kept
     // as two columns of word pairs, e at word 0 and o at word 1: each product row is
     // two independent carry chains of four wide multiply-adds.  Per round
     // t += a b_i + m p, t / 2^32: the columns change roles and e[1] moves down to the

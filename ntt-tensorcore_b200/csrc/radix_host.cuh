@@ -112,10 +112,17 @@ int launch_pass(Args a, const LimbDev<A>* limbs, cudaStream_t s) {
     if (ppc < 1) ppc = 1;
     if (ppc > a.polys) ppc = a.polys;
     a.polys_per_cta = ppc;
-    // a grid of one wave is bound by each thread's own latency and runs faster
-    // with up to 128 registers a thread; larger ones are bound by L1 and issue
-    // and want twice the warps.  Forward of 24 x 2^16: 9.7 us against 11.9; of
-    // 33 x 2^17: 26.5 against 22.8
+    // A grid that leaves an SM few warps is bound by each thread's own latency and
+    // runs faster with up to 128 registers a thread; larger ones are bound by L1 and
+    // issue and want twice the warps.  The line lies at 1024 threads an SM, where the
+    // larger variant is one full wave (the other one then runs up to two).  us
+    // forward, 128 / 64 registers, by threads in units of the line: 0.35 52 x 2^14
+    // 6.8 / 6.6; 0.54 80 x 2^14 9.1 / 9.8; 0.65 24 x 2^16 10.1 / 10.4; 1.3 24 x 2^17
+    // 19.7 / 18.0; 2.0 36 x 2^17 27.8 / 23.4.  64-bit: 0.70 52 x 2^14 13.5 / 16.8; 0.97
+    // 36 x 2^15 17.7 / 18.8; 2.6 3 x 2^20 73 / 62; nineteen of its 80 kernels, all
+    // built for 1024 threads, spill 8 - 88 bytes.  Blocks of 512 threads, of which the 128 registers fit one
+    // an SM, would rather change over at 0.5: 12 x 2^17 13.0 / 11.8, 2 x 2^20
+    // 18.4 / 16.3, 64-bit 1 x 2^20 25.8 / 23.7.
     constexpr uint32_t threads = 1u << (LG + LGV - LGE);
     constexpr auto few = radix_pass<A, S, D, LG, LGV, LGE, DIR, S0, LST, MODE, 512>;
     constexpr auto many = radix_pass<A, S, D, LG, LGV, LGE, DIR, S0, LST, MODE, 1024>;

@@ -4,8 +4,9 @@
 // traffic conflict-free for the pass's global access order), with the
 // four-step twiddles and the negacyclic twists fused into the load/store.
 //
-// It serves every size and modulus width and is the engine of the 60-bit
-// path; the tensor-core engines replace it for the hot 31-bit sizes.
+// It serves the sizes that the register-radix passes (radix.cuh) do not, below
+// 2^5 and above 2^20, for either modulus width, and the pre-transposed and the
+// four-step layout at every size.
 //
 // Two-pass decomposition for n = N1 * N2 (input index a*N2 + b):
 //   pass A (MODE_COL):     U[d][b] = DFT_N1(x[.][b])[d] * root^(d*b)

@@ -550,7 +550,8 @@ class RnsPlan:
         _check(lib().nttb_rns_pointwise_mul(self._h, _ptr(out), _ptr(a), _ptr(b), n_polys, _stream(stream)))
 
     def forward_inverse(self, data, n_polys, engine="auto", stream=None):
-        """Forward then inverse in place (one persistent launch on the INT8 engine)."""
+        """Forward then inverse in place (one launch up to 2^13, three above; one
+        persistent launch on the INT8 engine)."""
         _check(lib().nttb_rns_forward_inverse(self._h, _ptr(data), n_polys, _engine(engine), _stream(stream)))
 
     def stream_host(self, h_src, h_dst, n_polys, n_batches, mode="forward_inverse", engine="auto", stream=None):
@@ -592,8 +593,8 @@ class WidePlan:
         self.log_n, self.n, self.moduli = log_n, 1 << log_n, [int(x) for x in m]
 
     def transform(self, dst, src, n_polys, inverse=False, engine="auto", stream=None):
-        """engine "auto" (the INT8 byte-plane engine where it serves the plan),
-        "int8" or "scalar" (nttb_wide_transform_engine)."""
+        """engine "auto" (the CUDA-core engine), "scalar" (the same) or "int8" (the
+        byte-plane engine, 2^20) (nttb_wide_transform_engine)."""
         _check(lib().nttb_wide_transform_engine(self._h, _ptr(dst), _ptr(src), n_polys, int(inverse), _engine(engine),
                                                 _stream(stream)))
 
