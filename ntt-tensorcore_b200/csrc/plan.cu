@@ -387,14 +387,16 @@ StreamWorkspace::~StreamWorkspace() {
 }
 
 static void free_pool(PlanPool& pp) {
+    std::vector<void*> captured;  // freed without the lock, which graphs' callbacks take
     {
         std::lock_guard<std::mutex> lock(pp.graphs->mu);
         for (GraphWorkspaces::Buf& b : pp.graphs->bufs) {
-            if (b.ptr) cudaFree(b.ptr);
+            captured.push_back(b.ptr);
             b.ptr = nullptr;
             b.bytes = 0;
         }
     }
+    for (void* p : captured) cudaFree(p);
     if (!pp.pool) return;  // no call has staged anything outside a capture
     // cudaFree of stream-ordered memory does not wait for the calls that still use
     // it, as that of cudaMalloc's does: wait for them here.  Where the device cannot
